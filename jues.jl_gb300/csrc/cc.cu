@@ -284,7 +284,7 @@ double ccd_sweep(CCState *s, int prec) {
     // their packs here (the integrals keep theirs).
     for (const double *p : {s->T.p, s->Tn.p, s->Wp.p, s->WJ.p, s->WK.p, s->W12.p, s->Fae.p, s->Fmi.p})
         pack_cache_drop(ctx, p);
-    s->cache_operands = is_split(prec);
+    s->cache_operands = true;
     const double *W = s->oovv.p;
 
     // In split precision the ladders and the ring contractions run on K-stacked packs (two planes).

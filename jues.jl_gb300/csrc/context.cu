@@ -42,6 +42,7 @@ Ctx::~Ctx() {
 
 void *Ctx::alloc(size_t bytes) {
     if (bytes == 0) return nullptr;
+    if (mem_limit && mem_used + bytes > mem_limit) pack_cache_reclaim(this);
     if (mem_limit && mem_used + bytes > mem_limit)
         throw Error(JUES_ENOMEM, "device allocation of " + std::to_string(bytes) +
                                      " bytes exceeds the context memory limit (" +
@@ -67,6 +68,7 @@ void *Ctx::alloc(size_t bytes) {
     if (e != cudaSuccess) {
         // give the pool's idle blocks back and try once more (fragmentation)
         cudaGetLastError();
+        pack_cache_reclaim(this);
         cudaStreamSynchronize(stream);
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);

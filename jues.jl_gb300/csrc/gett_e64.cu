@@ -1,0 +1,942 @@
+// FP64 tensor contraction on the sm_103a tensor cores, at FP64 accuracy.
+//
+// GB300 issues about two FP64 operations per clock per SM (1.25 TFLOP/s in all) and has no FP64
+// tensor kind, but kind::f16 multiplies small integers exactly.  Every operand row (a row of A or a
+// column of B, running over the whole K) gets one power-of-two scale 2^e with max |x| < 2^e, and an
+// element becomes a 63-bit fixed-point number q = rint(x 2^(62-e)) cut into seven balanced 9-bit
+// digits, q = sum_p d_p 2^(9 (6-p)), d_p in [-256, 256], each exact in FP16.  Then
+//     sum_k a_k b_k = 2^(ea + eb - 70) sum_j S_j 2^(9 (6-j)),   S_j = sum_k sum_{p+q=j} d_p(a_k) d_q(b_k)
+// with the products of j >= 7 left out (2^-63 of max|a| max|b| each).  One tcgen05.mma with plane p
+// of A against the stacked planes 0..6-p of B adds to the accumulators j = p..6, so 28 products run
+// as seven instructions per K = 16 step.  Over a chunk of 64 K values |S_j| <= (j+1) 64 2^16 <= 2^24
+// for j <= 3, so the FP32 accumulators hold these sums exactly whatever the data; S_4, S_5 and S_6
+// (2^-36 to 2^-54 of the product) could pass 2^24 only for a chunk of equal-signed maximal digits and
+// then lose one unit in 2^24.  After each chunk the sums are added into 64-bit integers (S_0..S_2 and
+// S_3..S_6 combined), so the accumulation over K is exact: the whole error is the rounding of the
+// inputs to 2^-63 of their row's maximum, the dropped products and one final rounding, below
+// 2^-61 |a|_2 |b|_2 + 2^-53 |a.b|, where an FP64 FMA loop also rounds each of its K sums.  Against exact
+// products, relative Frobenius error for normal entries: 4.7e-17 at every size, the FMA kernels 1.3e-16
+// (K = 100) to 8.4e-16 (640^3).
+//
+// Speed (packs included): 6400^3 10.6 ms = 49 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.27 against
+// 8.1 ms; the MMAs alone would take 79% of the GEMM's time, TMEM reads and operand copies the rest.
+//
+// That bound is relative to |a|_2 |b|_2, not to sum |a_k b_k|: rows whose large elements meet only
+// small ones of the other side (an operand graded along K) would lose relative accuracy that an
+// FMA loop keeps.  So every output tile is checked before it is stored: a tile with a row or a
+// column whose results all fall below 2^-5 / sqrt(K) of its bound, or with a row that holds a non-finite,
+// subnormal-only or extreme (beyond 2^+-400) maximum, is not stored but listed, and
+// gett_f64_tiles recomputes the listed tiles on the FP64 pipe, with the same special values as ever.
+//
+// The tile is 128 x 32: TMEM holds two buffers of 7 x 32 FP32 columns, so the drain of one chunk
+// overlaps the MMAs of the next.  With N = 32 per plane an instruction reads 4 KB of A and up to 7
+// KB of B from shared memory for 16 to 112 clocks of MMA, so a K = 16 step takes about 496 clocks
+// (448 at the dense rate); a wider tile would need TMEM that is not there.  A's planes arrive one by
+// one (64 K values x 128 rows, 16 KB, 128-byte swizzle) in a ring of ten, B's seven together.
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include <cudaTypedefs.h>
+
+#include "gett_e64.cuh"
+#include "packcache.cuh"
+#include "tcgen05.cuh"
+
+namespace jues {
+
+namespace {
+
+constexpr int NP = E64_NP;            // digit planes
+constexpr int BM = 128, BN = 32;      // output tile
+constexpr int CK = 64;                // K per chunk: 128 bytes of FP16, one swizzle row
+constexpr int SLOTS = 10;             // ring of A planes
+constexpr int A_BYTES = BM * CK * 2, B_BYTES = NP * BN * CK * 2;   // one A plane 16 KB; all of B 28 KB
+constexpr int RING_BYTES = SLOTS * A_BYTES + 2 * B_BYTES;
+constexpr int BUF_COLS = NP * BN;     // TMEM columns of one chunk buffer
+constexpr uint32_t TMEM_COLS = 512;
+constexpr int THREADS = 320, DRAIN = 256;
+constexpr int HB = BN / 2;            // columns per drain thread
+constexpr int SMEM = RING_BYTES + 256 + BN * 8 + BN * 4 + 1024;
+constexpr int E_MIN = 1023 - 400, E_MAX = 1023 + 400;   // biased exponents of regular row maxima
+
+// instruction descriptor: FP32 accumulate, FP16 A and B, both K-major, M = 128, N = n
+__host__ __device__ constexpr uint32_t idesc(int n) {
+    return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
+
+struct E64Args {
+    long long M, N;             // rows of this launch's panel, columns
+    long long row0;             // first row of the panel in the whole output
+    int k16;                    // K steps of 16
+    int mtiles, ntiles;         // of this launch
+    long long mtiles_all;       // row tiles of the whole output (tile numbers in the list)
+    const int *expA, *expB;     // biased exponent of each row's largest element (0: zero row)
+    double alpha, beta;
+    int alpha_pow2, alpha_k, alpha_neg;
+    int beta_mode;              // 0: C = v; 1: C += v in place; 2: C = Cin + v; 3: C = beta Cin + v
+    double *C;
+    const double *Cin;
+    Mode mC, nC;
+    unsigned *flags;
+    int ksplit, kper;           // K parts of kper chunks each
+    longlong2 *part;            // ksplit > 1: [part][tile][BN][BM] pairs of 64-bit sums
+    int *list;                  // tiles left to the FP64 pipe
+    int weak;                   // a row or column is weak when no result reaches 2^-weak max|a| max|b|
+};
+
+__host__ __device__ __forceinline__ long long e64_items(const E64Args &g) {
+    return (long long)g.mtiles * g.ntiles * g.ksplit;
+}
+
+// tile -> (m0, n0): groups of 16 row tiles, rows fastest within a group, so that resident CTAs share
+// a few row tiles' planes in L2
+__device__ __forceinline__ void e64_origin(const E64Args &g, int tile, int &m0, int &n0) {
+    const int G = min(g.mtiles, 16), span = G * g.ntiles;
+    const int grp = tile / span, in = tile - grp * span;
+    const int gm = min(G, g.mtiles - grp * G);
+    m0 = (grp * G + in % gm) * BM;
+    n0 = (in / gm) * BN;
+}
+
+// (hi 2^36 + lo) 2^sc as FP64 on the integer pipes, hi and lo the 64-bit sums S_0 2^18 + S_1 2^9 +
+// S_2 and S_3 2^27 + S_4 2^18 + S_5 2^9 + S_6 (|hi| < K 2^35, |lo| < K 2^46): the leading 63 bits, one
+// rounding (ties away)
+__device__ __forceinline__ double e64_value(long long hi, long long lo, int sc, int neg) {
+    hi += lo >> 36;
+    const unsigned long long rem = (unsigned long long)lo & ((1ull << 36) - 1ull);
+    // as many bits of the low part as fit below hi's leading bit
+    const int up = min(36, __clzll(hi ^ (hi >> 63)) - 1);
+    const long long t = (hi << up) | (long long)(rem >> (36 - up));
+    const unsigned long long mag = (unsigned long long)(t < 0 ? -t : t);
+    if (mag == 0) return 0.0;
+    const int lz = __clzll((long long)mag);
+    const unsigned long long nrm = mag << lz;
+    const unsigned long long r = (nrm >> 11) + ((nrm >> 10) & 1ull);
+    const int field = 1023 + 63 - lz + sc - up + 36;
+    unsigned long long bits = ((unsigned long long)(unsigned)(field - 1) << 52) + r;
+    if ((t < 0) != (neg != 0)) bits |= 1ull << 63;
+    return __longlong_as_double((long long)bits);
+}
+
+// One thread's row of a tile (16 columns): its sums become FP64 values (hi[j] is overwritten with
+// the bits), and the checks above run.  ea: the row's biased exponent (0 outside M or a zero row);
+// colE: the columns' (shared memory).  Returns whether this thread saw a reason to leave the tile
+// to the FP64 pipe; warp-uniform parts are evaluated with the whole warp.
+__device__ __forceinline__ bool e64_finish(const E64Args &g, long long (&hi)[HB], const long long (&lo)[HB], int ea,
+                                           const int *colE) {
+    const bool live = ea != 0;
+    bool bad = live && (ea < E_MIN || ea > E_MAX);
+    int nc = 0;
+#pragma unroll
+    for (int j = 0; j < HB; ++j) {
+        const int eb = colE[j];
+        nc += eb != 0;
+        bad |= eb != 0 && (eb < E_MIN || eb > E_MAX);
+    }
+    const int nr = __popc(__ballot_sync(0xffffffffu, live));
+    // one or two results of a row (column) may cancel further by chance, so they get more room
+    const int trow = g.weak + (nc >= 3 ? 0 : (nc == 2 ? 4 : 8)), tcol = g.weak + (nr >= 3 ? 0 : (nr == 2 ? 4 : 8));
+    bool strong_row = false;
+#pragma unroll
+    for (int j = 0; j < HB; ++j) {
+        const int eb = colE[j];
+        double v = 0.0;
+        int above = -4096;   // result exponent relative to the bound 2^(ea + eb)
+        if (live && eb != 0) {
+            const int sc = (ea - 1022) + (eb - 1022) - 70;
+            v = e64_value(hi[j], lo[j], sc + (g.alpha_pow2 ? g.alpha_k : 0), g.alpha_neg);
+            const int f = (int)((unsigned)__double2hiint(v) >> 20 & 0x7FFu);
+            above = v == 0.0 ? -4096 : f - 1022 - (ea - 1022) - (eb - 1022) - (g.alpha_pow2 ? g.alpha_k : 0);
+        }
+        strong_row |= above >= -trow;
+        const bool strong_col = __ballot_sync(0xffffffffu, above >= -tcol) != 0u;
+        bad |= nr > 0 && eb != 0 && !strong_col;
+        hi[j] = __double_as_longlong(g.alpha_pow2 ? v : g.alpha * v);
+    }
+    return bad || (live && nc > 0 && !strong_row);
+}
+
+// store one thread's row through the output modes (co: column offsets, -1 past N)
+__device__ __forceinline__ void e64_store(const E64Args &g, const long long (&val)[HB], const long long *co,
+                                          long long rowoff) {
+    double *out = g.C + rowoff;
+    if (g.beta_mode == 0) {
+#pragma unroll
+        for (int j = 0; j < HB; ++j)
+            if (co[j] >= 0) out[co[j]] = __longlong_as_double(val[j]);
+    } else if (g.beta_mode == 1) {
+        // one owner per element: the L2's FP64 add gives the same sum as a load, add and store
+#pragma unroll
+        for (int j = 0; j < HB; ++j)
+            if (co[j] >= 0) red_add_f64(out + co[j], __longlong_as_double(val[j]));
+    } else {
+        const double *in = g.Cin + rowoff;
+        double cin[HB];
+#pragma unroll
+        for (int j = 0; j < HB; ++j) cin[j] = co[j] >= 0 ? __ldcs(in + co[j]) : 0.0;
+#pragma unroll
+        for (int j = 0; j < HB; ++j) {
+            if (co[j] < 0) continue;
+            const double v = __longlong_as_double(val[j]);
+            out[co[j]] = g.beta_mode == 2 ? cin[j] + v : fma(g.beta, cin[j], v);
+        }
+    }
+}
+
+__device__ __forceinline__ void e64_list_tile(const E64Args &g, int m0, int n0) {
+    const long long t = (g.row0 + m0) / BM + g.mtiles_all * (n0 / BN);
+    g.list[1 + atomicAdd(g.list, 1)] = (int)t;
+}
+
+// barrier over the drain threads (named barrier 1) that ORs a predicate over them
+__device__ __forceinline__ bool drain_any(bool pred) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.or.pred q, 1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)pred), "n"(DRAIN)
+        : "memory");
+    return r != 0;
+}
+
+__device__ __forceinline__ int f2i(uint32_t x) { return __float2int_rn(__uint_as_float(x)); }
+
+// Persistent: CTA b takes work items b, b + gridDim.x, ... (an item is one tile over one K part).
+// Warp 0 issues TMA, warp 1 owns TMEM and issues the MMAs, warps 2-9 drain (two per 32-lane TMEM
+// quarter, 16 columns each).  Every wait is bounded; on expiry the CTA raises FLAG_TIMEOUT, skips its
+// stores, waits for its own copies, frees TMEM and returns.
+__global__ void __launch_bounds__(THREADS, 1)
+    gett_e64_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                    const __grid_constant__ E64Args g) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t *ringB = smem + SLOTS * A_BYTES;
+    uint64_t *afull = reinterpret_cast<uint64_t *>(smem + RING_BYTES);
+    uint64_t *aempty = afull + SLOTS;
+    uint64_t *bfull = aempty + SLOTS;    // [2]
+    uint64_t *bempty = bfull + 2;
+    uint64_t *cfull = bempty + 2;        // [2] chunk accumulated in TMEM buffer
+    uint64_t *cempty = cfull + 2;        // [2] chunk drained
+    uint64_t *fin = cempty + 2;          // the MMA thread's last commit
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fin + 1);
+    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    long long *coloff = reinterpret_cast<long long *>(smem + RING_BYTES + 256);
+    int *colE = reinterpret_cast<int *>(coloff + BN);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int nchunks_all = (g.k16 + 3) / 4;
+    const int tiles = g.mtiles * g.ntiles;
+    const int nitems = tiles * g.ksplit;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SLOTS; ++s) {
+            mbar_init(&afull[s], 1);
+            mbar_init(&aempty[s], 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&bfull[b], 1);
+            mbar_init(&bempty[b], 1);
+            mbar_init(&cfull[b], 1);
+            mbar_init(&cempty[b], DRAIN);
+        }
+        mbar_init(fin, 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        tmem_alloc(tmem_slot, TMEM_COLS);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // TMA: per chunk B's planes, then A's one by one; it counts A planes, gc chunks
+            unsigned it = 0, gc = 0;
+            bool stop = false;
+            auto wait = [&](uint64_t *bar, unsigned parity) {
+                if (mbar_wait(bar, parity, abort_flag, g.flags)) return true;
+                *abort_flag = 1;
+                stop = true;
+                return false;
+            };
+            for (int w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
+                const int tile = w % tiles, part = w / tiles;
+                int m0, n0;
+                e64_origin(g, tile, m0, n0);
+                const int c0 = part * g.kper, c1 = min(nchunks_all, c0 + g.kper);
+                for (int c = c0; c < c1 && !stop; ++c, ++gc) {
+                    const unsigned b = gc & 1u;
+                    if (!wait(&bempty[b], ((gc >> 1) & 1u) ^ 1u)) break;
+                    mbar_expect_tx(&bfull[b], B_BYTES);
+                    tma_load_3d(ringB + b * B_BYTES, &mapB, &bfull[b], c * CK, n0, 0);
+                    for (int p = 0; p < NP; ++p, ++it) {
+                        const unsigned s = it % SLOTS;
+                        if (!wait(&aempty[s], ((it / SLOTS) & 1u) ^ 1u)) break;
+                        mbar_expect_tx(&afull[s], A_BYTES);
+                        tma_load_3d(smem + s * A_BYTES, &mapA, &afull[s], c * CK, m0, p);
+                    }
+                }
+            }
+            // the last copy into each buffer has landed (immediate unless an abort cut the MMA
+            // thread short), so none is in flight when the CTA exits
+            for (unsigned s = 0; s < SLOTS; ++s)
+                if (it > s) mbar_wait_quiet(&afull[s], ((s + (it - 1 - s) / SLOTS * SLOTS) / SLOTS) & 1u);
+            for (unsigned b = 0; b < 2; ++b)
+                if (gc > b) mbar_wait_quiet(&bfull[b], ((b + (gc - 1 - b) / 2 * 2) >> 1) & 1u);
+        }
+    } else if (warp == 1) {
+        // The whole warp walks the loops in step (see umma_warp)
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        unsigned s = 0, ph = 0, gc = 0;   // ring slot and its phase, chunks
+        bool stop = false;
+        for (int w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
+            const int part = w / tiles;
+            const int c0 = part * g.kper, c1 = min(nchunks_all, c0 + g.kper);
+            for (int c = c0; c < c1; ++c, ++gc) {
+                const unsigned b = gc & 1u;
+                if ((gc >= 2 && !mbar_wait_warp(&cempty[b], ((gc >> 1) - 1u) & 1u, abort_flag, g.flags)) ||
+                    !mbar_wait_warp(&bfull[b], (gc >> 1) & 1u, abort_flag, g.flags)) {
+                    stop = true;
+                    break;
+                }
+                const uint32_t b0 = sw128_lo(ringB + b * B_BYTES);
+                const uint32_t dbuf = tm + b * BUF_COLS;
+                const int steps = min(4, g.k16 - 4 * c);
+#pragma unroll
+                for (int p = 0; p < NP; ++p) {
+                    if (!mbar_wait_warp(&afull[s], ph, abort_flag, g.flags)) {
+                        stop = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t a0 = sw128_lo(smem + s * A_BYTES);
+                    if (steps == 4) {
+                        umma_warp_x4(dbuf + (uint32_t)(p * BN), a0, b0, idesc((NP - p) * BN), p == 0 ? 0u : 1u);
+                    } else {
+                        for (int kk = 0; kk < steps; ++kk)   // 32 bytes per K = 16 step
+                            umma_warp(dbuf + (uint32_t)(p * BN), a0 + 2 * kk, b0 + 2 * kk, idesc((NP - p) * BN),
+                                      (p == 0 && kk == 0) ? 0u : 1u);
+                    }
+                    umma_commit_warp(&aempty[s]);
+                    if (++s == SLOTS) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
+                }
+                if (stop) break;
+                umma_commit_warp(&bempty[b]);
+                umma_commit_warp(&cfull[b]);
+            }
+        }
+        if (stop) *abort_flag = 1;
+        __syncwarp();
+        // every MMA this warp issued has completed before TMEM is freed
+        umma_commit_warp(fin);
+        mbar_wait_quiet(fin, 0u);
+    } else {
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int dt = threadIdx.x - 64;
+        long long gc = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
+            const int tile = w % tiles, part = w / tiles;
+            int m0, n0;
+            e64_origin(g, tile, m0, n0);
+            const int nchunks = min(nchunks_all, (part + 1) * g.kper) - part * g.kper;
+            // every drain thread has finished the previous item (which reads coloff and colE)
+            if (drain_any(*abort_flag != 0)) {
+                ok = false;
+                break;
+            }
+            const long long mrow = (long long)m0 + quarter * 32 + lane;
+            int ea = 0;
+            if (g.ksplit == 1) {
+                if (dt < BN) {
+                    const long long n = (long long)n0 + dt;
+                    coloff[dt] = n < g.N ? mode_off(g.nC, n) : -1;
+                    colE[dt] = n < g.N ? __ldg(g.expB + n) : 0;
+                }
+                ea = mrow < g.M ? __ldg(g.expA + mrow) : 0;
+            }
+            long long hi[HB], lo[HB];
+#pragma unroll
+            for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
+            bool bad = false;
+            for (int c = 0; c < nchunks; ++c, ++gc) {
+                const int buf = (int)(gc & 1);
+                const bool got = mbar_wait(&cfull[buf], (uint32_t)(gc >> 1) & 1u, abort_flag, g.flags);
+                if (!__all_sync(0xffffffffu, got)) {
+                    *abort_flag = 1;
+                    bad = true;   // the barrier below takes every drain thread out
+                    break;
+                }
+                __syncwarp();
+                tc_fence_after();
+                const uint32_t base =
+                    tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BUF_COLS + half * HB);
+                uint32_t r0[HB], r1[HB];
+                tmem_ld16(base, r0);
+                tmem_ld16(base + BN, r1);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < HB; ++j)
+                    hi[j] += (long long)f2i(r0[j]) * (1 << 18) + (long long)f2i(r1[j]) * (1 << 9);
+                tmem_ld16(base + 2 * BN, r0);
+                tmem_ld16(base + 3 * BN, r1);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < HB; ++j) {
+                    hi[j] += f2i(r0[j]);
+                    lo[j] += (long long)f2i(r1[j]) * (1 << 27);
+                }
+                tmem_ld16(base + 4 * BN, r0);
+                tmem_ld16(base + 5 * BN, r1);
+                tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < HB; ++j)
+                    lo[j] += (long long)f2i(r0[j]) * (1 << 18) + (long long)f2i(r1[j]) * (1 << 9);
+                tmem_ld16(base + 6 * BN, r0);
+                tmem_ld_wait();
+                tc_fence_before();
+                mbar_arrive(&cempty[buf]);
+#pragma unroll
+                for (int j = 0; j < HB; ++j) lo[j] += f2i(r0[j]);
+            }
+            if (drain_any(bad)) {   // also orders the coloff and colE stores
+                ok = false;
+                break;
+            }
+            if (g.ksplit > 1) {
+                longlong2 *dst = g.part + (((long long)part * tiles + tile) * BN + half * HB) * BM + quarter * 32 + lane;
+#pragma unroll
+                for (int j = 0; j < HB; ++j) dst[(long long)j * BM] = make_longlong2(hi[j], lo[j]);
+                continue;
+            }
+            const bool weak = e64_finish(g, hi, lo, ea, colE + half * HB);
+            if (drain_any(weak)) {
+                if (dt == 0) e64_list_tile(g, m0, n0);
+            } else if (mrow < g.M) {
+                e64_store(g, hi, coloff + half * HB, mode_off(g.mC, g.row0 + mrow));
+            }
+        }
+        if (!ok && lane == 0) atomicOr(g.flags, FLAG_TIMEOUT);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, TMEM_COLS);
+    }
+}
+
+// K parts: one block per tile adds the parts' 64-bit sums (exact, so their number does not matter)
+// and finishes the tile as the main kernel does
+__global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
+    __shared__ long long coloff[BN];
+    __shared__ int colE[BN];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int quarter = warp & 3, half = warp >> 2;
+    const int tile = blockIdx.x, tiles = g.mtiles * g.ntiles;
+    int m0, n0;
+    e64_origin(g, tile, m0, n0);
+    if (threadIdx.x < BN) {
+        const long long n = (long long)n0 + threadIdx.x;
+        coloff[threadIdx.x] = n < g.N ? mode_off(g.nC, n) : -1;
+        colE[threadIdx.x] = n < g.N ? __ldg(g.expB + n) : 0;
+    }
+    const long long mrow = (long long)m0 + quarter * 32 + lane;
+    const int ea = mrow < g.M ? __ldg(g.expA + mrow) : 0;
+    long long hi[HB], lo[HB];
+#pragma unroll
+    for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
+    for (int s = 0; s < g.ksplit; ++s) {
+        const longlong2 *src = g.part + (((long long)s * tiles + tile) * BN + half * HB) * BM + quarter * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < HB; ++j) {
+            const longlong2 p = src[(long long)j * BM];
+            hi[j] += p.x;
+            lo[j] += p.y;
+        }
+    }
+    __syncthreads();
+    const bool weak = e64_finish(g, hi, lo, ea, colE + half * HB);
+    if (__syncthreads_or(weak)) {
+        if (threadIdx.x == 0) e64_list_tile(g, m0, n0);
+    } else if (mrow < g.M) {
+        e64_store(g, hi, coloff + half * HB, mode_off(g.mC, g.row0 + mrow));
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// operand digits
+// ---------------------------------------------------------------------------------------------
+constexpr int PR = 16, PK = 128, PPITCH = PK / 2 + 2;   // pack block: 16 rows x 128 K; staged row pitch in words
+
+// one operand of a pack launch: rows [row0, row0 + R) of src into digit planes [NP][Rpad][Kpad] and
+// the rows' exponents
+struct PackArgs {
+    const double *src;
+    Mode rm, km;
+    long long row0, R, K, Rpad, Kpad;
+    int *exps;
+    __half *dst;
+    unsigned blocks;   // of this operand in the launch
+    int kfast;         // K (else the row index) is the source's unit-stride index
+    int kseg;          // row-maximum pass: K chunks per block
+};
+
+// biased exponent; 1 for subnormals, which mark a row the tensor cores do not take
+__device__ __forceinline__ int exp_of(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
+    const int e = (int)(hi >> 20);
+    return e ? e : ((hi | (unsigned)__double2loint(x)) ? 1 : 0);
+}
+
+// the seven digits of x in a row whose largest biased exponent is E, each + 256 (0..512)
+__device__ __forceinline__ void digits(double x, int E, unsigned (&u)[NP]) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const int e = (int)(hi >> 20 & 0x7FFu);
+    const int sh = E - e;
+    long long q = 0;
+    if (e != 0 && sh < 64) {
+        // m 2^9 >> sh, ties away from zero (exact for sh <= 9)
+        const unsigned long long m = (((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << 9;
+        q = sh == 0 ? (long long)m : (long long)((m + (1ull << (sh - 1))) >> sh);
+        if (hi >> 31) q = -q;
+    }
+    // + 256 in every digit: q + 256 (2^54 + 2^45 + ... + 1) is positive and its 9-bit fields are the
+    // balanced digits + 256
+    constexpr unsigned long long OFF = 256ull * ((1ull << 54) + (1ull << 45) + (1ull << 36) + (1ull << 27) +
+                                                 (1ull << 18) + (1ull << 9) + 1ull);
+    const unsigned long long s = (unsigned long long)q + OFF;
+    u[0] = (unsigned)(s >> 54);
+#pragma unroll
+    for (int p = 1; p < NP; ++p) u[p] = (unsigned)(s >> (9 * (NP - 1 - p))) & 511u;
+}
+
+// digit pair -> two FP16 integers: 0x6400 | u is 1024 + u
+__device__ __forceinline__ uint32_t digit_pair(unsigned u0, unsigned u1) {
+    const uint32_t w = u0 | (u1 << 16) | 0x64006400u, b = 0x65006500u;   // 1280
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&w), *reinterpret_cast<const __half2 *>(&b));
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+struct PackSmem {
+    uint32_t outp[NP][PR][PPITCH];
+    long long roff[PR], koff[PK];
+    int rowE[PR];
+};
+
+// LOCALMAX: K <= 128, the block sees whole rows and writes their exponents; else they are read
+template <bool KFAST, bool LOCALMAX>
+__device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, long long k0, PackSmem &sm) {
+    auto &outp = sm.outp;
+    auto &roff = sm.roff;
+    auto &koff = sm.koff;
+    auto &rowE = sm.rowE;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < PR) {
+        const long long r = r0 + tid;
+        roff[tid] = r < a.R ? mode_off(a.rm, a.row0 + r) : -1;
+        rowE[tid] = LOCALMAX ? 0 : (r < a.R ? a.exps[r] : 0);
+    } else if (tid >= 64 && tid < 64 + PK) {
+        const long long k = k0 + tid - 64;
+        koff[tid - 64] = k < a.K ? mode_off(a.km, k) : -1;
+    }
+    __syncthreads();
+    auto row_of = [&](int i) { return KFAST ? (tid >> 6) + 4 * i : (tid & 15); };
+    auto pair_of = [&](int i) { return KFAST ? (tid & 63) : (tid >> 4) + 16 * i; };
+    double x[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const long long ro = roff[row_of(i)], ko = koff[2 * pair_of(i) + h];
+            x[i][h] = (ro >= 0 && ko >= 0) ? __ldg(a.src + ro + ko) : 0.0;
+        }
+    if constexpr (LOCALMAX) {
+        if constexpr (KFAST) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int m = __reduce_max_sync(0xffffffffu, max(exp_of(x[i][0]), exp_of(x[i][1])));
+                if (lane == 0) atomicMax(&rowE[row_of(i)], m);
+            }
+        } else {
+            int m = 0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) m = max(m, max(exp_of(x[i][0]), exp_of(x[i][1])));
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            if (lane < 16) atomicMax(&rowE[lane], m);
+        }
+        __syncthreads();
+        if (tid < PR) a.exps[r0 + tid] = rowE[tid];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = row_of(i), E = rowE[r];
+        unsigned u0[NP], u1[NP];
+        digits(x[i][0], E, u0);
+        digits(x[i][1], E, u1);
+#pragma unroll
+        for (int p = 0; p < NP; ++p) outp[p][r][pair_of(i)] = digit_pair(u0[p], u1[p]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < (NP * PR * 32) / 256; ++j) {
+        const int idx = tid + 256 * j;
+        const int seg = idx & 31, row = (idx >> 5) & (PR - 1), plane = idx >> 9;
+        const long long k = k0 + 4 * seg;
+        if (k >= a.Kpad) continue;
+        *reinterpret_cast<uint2 *>(a.dst + ((size_t)plane * a.Rpad + (size_t)(r0 + row)) * a.Kpad + k) =
+            *reinterpret_cast<const uint2 *>(&outp[plane][row][2 * seg]);
+    }
+}
+
+// both operands of a GEMM in one launch: blocks [0, a.blocks) pack a, the rest b
+template <bool LOCALMAX>
+__global__ void __launch_bounds__(256, 4) e64_pack_kernel(const __grid_constant__ PackArgs a,
+                                                          const __grid_constant__ PackArgs b) {
+    __shared__ __align__(16) PackSmem sm;
+    const bool second = blockIdx.x >= a.blocks;
+    const PackArgs &P = second ? b : a;
+    const unsigned blk = second ? blockIdx.x - a.blocks : blockIdx.x;
+    const unsigned kb = (unsigned)((P.Kpad + PK - 1) / PK), rb = (unsigned)(P.Rpad / PR);
+    if (P.kfast)
+        e64_pack_block<true, LOCALMAX>(P, (long long)(blk / kb) * PR, (long long)(blk % kb) * PK, sm);
+    else
+        e64_pack_block<false, LOCALMAX>(P, (long long)(blk % rb) * PR, (long long)(blk / rb) * PK, sm);
+}
+
+// the rows' largest biased exponents for K > 128 (exps cleared before): a block covers 16 rows x kseg
+// chunks of 128 K
+template <bool KFAST>
+__device__ __forceinline__ void e64_rowmax_block(const PackArgs &a, long long r0, long long k0) {
+    __shared__ long long roff[PR], koff[PK];
+    __shared__ int rowE[PR];
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid < PR) {
+        const long long r = r0 + tid;
+        roff[tid] = r < a.R ? mode_off(a.rm, a.row0 + r) : -1;
+        rowE[tid] = 0;
+    }
+    int m[4] = {0, 0, 0, 0};
+    for (int c = 0; c < a.kseg && k0 + (long long)c * PK < a.K; ++c) {
+        __syncthreads();
+        if (tid >= 64 && tid < 64 + PK) {
+            const long long k = k0 + (long long)c * PK + tid - 64;
+            koff[tid - 64] = k < a.K ? mode_off(a.km, k) : -1;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int row = KFAST ? (tid >> 6) + 4 * i : (tid & 15);
+            const int pair = KFAST ? (tid & 63) : (tid >> 4) + 16 * i;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const long long ro = roff[row], ko = koff[2 * pair + h];
+                if (ro >= 0 && ko >= 0) m[i] = max(m[i], exp_of(__ldg(a.src + ro + ko)));
+            }
+        }
+    }
+    __syncthreads();
+    if constexpr (KFAST) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int x = __reduce_max_sync(0xffffffffu, m[i]);
+            if (lane == 0) atomicMax(&rowE[(tid >> 6) + 4 * i], x);
+        }
+    } else {
+        int x = max(max(m[0], m[1]), max(m[2], m[3]));
+        x = max(x, __shfl_xor_sync(0xffffffffu, x, 16));
+        if (lane < 16) atomicMax(&rowE[lane], x);
+    }
+    __syncthreads();
+    if (tid < PR && r0 + tid < a.R && rowE[tid]) atomicMax(&a.exps[r0 + tid], rowE[tid]);
+}
+
+__global__ void __launch_bounds__(256) e64_rowmax_kernel(const __grid_constant__ PackArgs a,
+                                                         const __grid_constant__ PackArgs b) {
+    const unsigned na = (unsigned)(a.blocks ? (a.Rpad / PR) * ((a.K + PK * a.kseg - 1) / (PK * a.kseg)) : 0);
+    const bool second = blockIdx.x >= na;
+    const PackArgs &P = second ? b : a;
+    const unsigned blk = second ? blockIdx.x - na : blockIdx.x;
+    const unsigned rb = (unsigned)(P.Rpad / PR), ks = (unsigned)((P.K + PK * P.kseg - 1) / (PK * P.kseg));
+    if (P.kfast)
+        e64_rowmax_block<true>(P, (long long)(blk / ks) * PR, (long long)(blk % ks) * PK * P.kseg);
+    else
+        e64_rowmax_block<false>(P, (long long)(blk % rb) * PR, (long long)(blk / rb) * PK * P.kseg);
+}
+
+long long roundup(long long x, long long m) { return (x + m - 1) / m * m; }
+
+PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
+    static std::atomic<void *> fn{nullptr};
+    void *p = fn.load();
+    if (!p) {
+        cudaDriverEntryPointQueryResult q;
+        JUES_CHECK_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q));
+        if (q != cudaDriverEntryPointSuccess || !p)
+            throw Error(JUES_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
+        fn.store(p);
+    }
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+}
+
+// digit planes [NP][rows][kpad]; one box = 64 K values (past kpad: zeros) x box_rows rows x box_planes
+CUtensorMap plane_map(const __half *base, long long rows, long long kpad, int box_rows, int box_planes) {
+    CUtensorMap m;
+    std::memset(&m, 0, sizeof(m));
+    cuuint64_t dims[3] = {(cuuint64_t)kpad, (cuuint64_t)rows, (cuuint64_t)NP};
+    cuuint64_t strides[2] = {(cuuint64_t)kpad * 2, (cuuint64_t)rows * kpad * 2};
+    cuuint32_t box[3] = {(cuuint32_t)CK, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half *>(base), dims, strides, box,
+                             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) throw Error(JUES_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
+    return m;
+}
+
+PackArgs pack_args(const double *src, const Mode &rm, const Mode &km, long long row0, long long R, long long K,
+                   long long Rpad, long long Kpad, int *exps, __half *dst) {
+    PackArgs p;
+    p.src = src; p.rm = rm; p.km = km;
+    p.row0 = row0; p.R = R; p.K = K; p.Rpad = Rpad; p.Kpad = Kpad;
+    p.exps = exps; p.dst = dst;
+    p.blocks = (unsigned)((Rpad / PR) * ((Kpad + PK - 1) / PK));
+    p.kfast = km.s0 == 1 && km.d0 > 1;
+    // about 16 blocks per SM in the row-maximum pass, at most 16 chunks a block
+    const long long chunks = (K + PK - 1) / PK;
+    p.kseg = (int)std::max<long long>(1, std::min<long long>(16, (Rpad / PR) * chunks / (152 * 16)));
+    return p;
+}
+
+// digits of up to two operands (b may be null)
+void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
+    PackArgs none{};
+    const PackArgs &B = b ? *b : none;
+    if (a.K <= PK) {
+        Ctx::Scope s(ctx, "pack_e64");
+        e64_pack_kernel<true><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+        JUES_CHECK_CUDA(cudaGetLastError());
+        return;
+    }
+    JUES_CHECK_CUDA(cudaMemsetAsync(a.exps, 0, (size_t)a.Rpad * sizeof(int), ctx->stream));
+    if (b) JUES_CHECK_CUDA(cudaMemsetAsync(b->exps, 0, (size_t)b->Rpad * sizeof(int), ctx->stream));
+    auto rblocks = [](const PackArgs &p) {
+        return p.blocks ? (unsigned)((p.Rpad / PR) * ((p.K + PK * p.kseg - 1) / (PK * p.kseg))) : 0u;
+    };
+    {
+        Ctx::Scope s(ctx, "pack_e64");
+        e64_rowmax_kernel<<<rblocks(a) + rblocks(B), 256, 0, ctx->stream>>>(a, B);
+        JUES_CHECK_CUDA(cudaGetLastError());
+    }
+    Ctx::Scope s(ctx, "pack_e64");
+    e64_pack_kernel<false><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+    JUES_CHECK_CUDA(cudaGetLastError());
+}
+
+// Whether the tensor cores take a contraction.  Measured through jues_gemm (packs, GEMM and the listed
+// tiles' launch against the FP64 pipe, us): 640^3 51 against 763; 400^3 45 / 475; 200^3 (2^16 outputs or
+// fewer: a warp per output element on the FP64 pipe) 38 / 45; 150^3 35 / 25; 2304 x 48 x 48 (tiles on the
+// FP64 pipe) 30 / 63; 4000 x 16 x 25 31 / 41.  The line lies where the sides meet.  A side below 16 pads
+// too much, and |lo| < K 2^46 must stay below 2^63.
+bool wanted(long long M, long long N, long long K) {
+    if (std::min(M, N) < 16 || K < 8 || K >= (1 << 17)) return false;
+    const double flops = 2.0 * (double)M * (double)N * (double)K;
+    return flops >= (M * N <= (1LL << 16) && K <= 8192 ? 1.6e7 : 3e6);
+}
+
+struct Busy {
+    PackCache &c;
+    explicit Busy(PackCache &x) : c(x) { c.busy = true; }
+    ~Busy() { c.busy = false; }
+};
+
+PackEntry *find_entry(PackCache &pc, const double *src, const Mode &rm, const Mode &km, long long R, long long K,
+                      long long Rpad, long long Kpad) {
+    for (auto &e : pc.cached)
+        if (e->np == NP && e->src == src && e->R == R && e->K == K && e->Rpad == Rpad && e->Kpad == Kpad &&
+            same_mode(e->r, rm) && same_mode(e->k, km))
+            return e.get();
+    return nullptr;
+}
+
+template <class T>
+void grow(Ctx *ctx, DBuf<T> &b, size_t need) {
+    if (b.n >= need) return;
+    b.reset();
+    b = DBuf<T>(ctx, need);
+}
+
+// a whole operand's digits are kept between calls when the caller declares it constant; a short-K
+// one (an integral transform's) only while it is small, since reading the source again moves
+// fewer bytes than its planes
+bool keep_planes(bool is_const, long long K, size_t halves) {
+    if (!is_const) return false;
+    return K > 512 || halves * 2 <= (size_t(128) << 20);
+}
+constexpr size_t PANEL_HALVES = size_t(64) << 20;   // transient planes: panels of 128 MB
+
+}  // namespace
+
+bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
+    if (!wanted(a0.M, a0.N, a0.K)) return false;
+    GettArgs a = a0;
+    // the output's unit-stride mode on the TMEM-lane side (coalesced stores) unless padding says
+    // otherwise (rows pad to 128, columns to 32)
+    const bool m_unit = a.mC.s0 == 1 && a.mC.d0 > 1, n_unit = a.nC.s0 == 1 && a.nC.d0 > 1;
+    auto cost = [](long long M, long long N, bool unit) {
+        return (double)roundup(M, BM) * (double)roundup(N, BN) * (unit ? 1.0 : 1.2);
+    };
+    if (cost(a.N, a.M, n_unit) < cost(a.M, a.N, m_unit)) {
+        std::swap(a.M, a.N);
+        std::swap(a.A, a.B);
+        std::swap(a.mA, a.nB);
+        std::swap(a.kA, a.kB);
+        std::swap(a.mC, a.nC);
+        std::swap(a.a_const, a.b_const);
+    }
+    const long long Kpad = roundup(a.K, 16);   // rows of planes start on 32 bytes
+    const long long Mall = roundup(a.M, BM), Nall = roundup(a.N, BM);
+    if (Mall >= (1LL << 31) || Nall >= (1LL << 31) || Kpad >= (1LL << 30)) return false;
+    const long long mtiles_all = Mall / BM, ntiles = roundup(a.N, BN) / BN;
+    if (mtiles_all * ntiles >= (1LL << 30) || (Nall / PR) * ((Kpad + PK - 1) / PK) >= (1LL << 31)) return false;
+    if (!ctx->pack) ctx->pack = new PackCache();
+    PackCache &pc = *ctx->pack;
+    const size_t hA = (size_t)NP * Mall * Kpad, hB = (size_t)NP * Nall * Kpad;
+    const bool keepA = keep_planes(a.a_const, a.K, hA), keepB = keep_planes(a.b_const, a.K, hB);
+    // rows per panel of A when its planes are transient
+    long long prow = Mall;
+    if (!keepA && hA > PANEL_HALVES)
+        prow = std::max<long long>(BM, (long long)(PANEL_HALVES / ((size_t)NP * Kpad)) / BM * BM);
+    if ((prow / PR) * ((Kpad + PK - 1) / PK) >= (1LL << 31)) return false;
+
+    PackEntry *eA = keepA ? find_entry(pc, a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad) : nullptr;
+    PackEntry *eB = keepB ? find_entry(pc, a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad) : nullptr;
+    std::unique_ptr<PackEntry> newA, newB;
+    // K parts of a grid too small for the GPU (chunks of 64 K); exact whatever their number
+    const int k16 = (int)((a.K + 15) / 16), chunks = (k16 + 3) / 4;
+    const long long panel_tiles = prow / BM * ntiles;
+    int ksplit = 1, kper = chunks;
+    {
+        // rounds of the 152 SMs times (chunks a part + about two for the tile's epilogue), plus the
+        // parts' own pass
+        auto time = [&](int ks) {
+            const long long rounds = (panel_tiles * ks + 151) / 152;
+            return (double)rounds * ((chunks + ks - 1) / ks + 2) + (ks > 1 ? 4.0 + 0.02 * (double)(panel_tiles * ks) / 152 : 0.0);
+        };
+        for (int ks = 2; ks <= 64 && ks <= chunks; ++ks)
+            if (panel_tiles * ks <= 152LL * 8 && time(ks) < 0.9 * time(ksplit)) ksplit = ks;
+        kper = (chunks + ksplit - 1) / ksplit;
+        ksplit = (chunks + kper - 1) / kper;
+    }
+    longlong2 *part = nullptr;
+    try {
+        Busy busy(pc);
+        if (keepA && !eA)
+            newA.reset(new PackEntry{a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad, NP, take_buffer(ctx, pc.free_planes, hA),
+                                     take_buffer(ctx, pc.free_exps, (size_t)Mall)});
+        if (keepB && !eB)
+            newB.reset(new PackEntry{a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad, NP, take_buffer(ctx, pc.free_planes, hB),
+                                     take_buffer(ctx, pc.free_exps, (size_t)Nall)});
+        if (!keepA) {
+            grow(ctx, pc.e64_planes[0], (size_t)NP * prow * Kpad);
+            grow(ctx, pc.e64_exps[0], (size_t)prow);
+        }
+        if (!keepB) {
+            grow(ctx, pc.e64_planes[1], hB);
+            grow(ctx, pc.e64_exps[1], (size_t)Nall);
+        }
+        grow(ctx, pc.e64_list, (size_t)(mtiles_all * ntiles + 1));
+        if (ksplit > 1)
+            part = static_cast<longlong2 *>(
+                ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN * sizeof(longlong2)));
+    } catch (const Error &e) {
+        if (e.code != JUES_ENOMEM) throw;
+        return false;   // the FP64 pipe needs no planes
+    }
+    static std::atomic<unsigned long long> attr_set{0};
+    const unsigned long long bit = ctx->device >= 0 && ctx->device < 64 ? 1ull << ctx->device : 0ull;
+    if (!bit || !(attr_set.load() & bit)) {
+        JUES_CHECK_CUDA(cudaFuncSetAttribute(gett_e64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+        attr_set.fetch_or(bit);
+    }
+    // C = Cin + alpha AB into a dense column-major C: copy Cin over and add in place, off the FP64 pipe
+    const double *Cin = a.Cin ? a.Cin : a.C;
+    const bool disjoint = Cin + a.M * a.N <= a.C || a.C + a.M * a.N <= Cin;
+    if (a.beta == 1.0 && Cin != a.C && disjoint && a.mC.d0 == MODE_BIG && a.mC.s0 == 1 && a.nC.d0 == MODE_BIG &&
+        a.nC.s0 == a.M) {
+        JUES_CHECK_CUDA(cudaMemcpyAsync(a.C, Cin, (size_t)(a.M * a.N) * sizeof(double), cudaMemcpyDeviceToDevice,
+                                        ctx->stream));
+        Cin = a.C;
+    }
+    a.Cin = Cin;
+
+    __half *planesB = eB ? eB->buf.p : newB ? newB->buf.p : pc.e64_planes[1].p;
+    int *expsB = eB ? eB->exps.p : newB ? newB->exps.p : pc.e64_exps[1].p;
+    JUES_CHECK_CUDA(cudaMemsetAsync(pc.e64_list.p, 0, sizeof(int), ctx->stream));
+    for (long long r0 = 0; r0 < a.M; r0 += prow) {
+        const long long R = std::min(prow, a.M - r0), Rpad = roundup(R, BM);
+        __half *planesA = eA ? eA->buf.p : newA ? newA->buf.p : pc.e64_planes[0].p;
+        int *expsA = eA ? eA->exps.p : newA ? newA->exps.p : pc.e64_exps[0].p;
+        const bool packB = r0 == 0 && !eB;
+        const PackArgs pb = pack_args(a.B, a.nB, a.kB, 0, a.N, a.K, Nall, Kpad, expsB, planesB);
+        if (!eA)
+            run_pack(ctx, pack_args(a.A, a.mA, a.kA, r0, R, a.K, Rpad, Kpad, expsA, planesA), packB ? &pb : nullptr);
+        else if (packB)
+            run_pack(ctx, pb, nullptr);
+        E64Args g;
+        g.M = R; g.N = a.N; g.row0 = r0;
+        g.k16 = k16;
+        g.mtiles = (int)(Rpad / BM); g.ntiles = (int)ntiles;
+        g.mtiles_all = mtiles_all;
+        g.expA = expsA; g.expB = expsB;
+        g.alpha = a.alpha; g.beta = a.beta;
+        int ak = 0;
+        g.alpha_pow2 = std::frexp(std::fabs(a.alpha), &ak) == 0.5 && ak - 1 >= -8 && ak - 1 <= 8;
+        g.alpha_k = g.alpha_pow2 ? ak - 1 : 0;
+        g.alpha_neg = g.alpha_pow2 && a.alpha < 0;
+        g.beta_mode = a.beta == 0.0 ? 0 : (a.beta == 1.0 ? (Cin == a.C ? 1 : 2) : 3);
+        g.C = a.C; g.Cin = Cin; g.mC = a.mC; g.nC = a.nC;
+        g.flags = ctx->d_flags;
+        g.ksplit = ksplit; g.kper = kper;
+        g.part = part;
+        g.list = pc.e64_list.p;
+        // an FMA loop's own error grows as sqrt(K): 2^-weak keeps 2^-61 2^weak at its level
+        int kl = 0;
+        while ((1LL << kl) < a.K) ++kl;
+        g.weak = 5 + kl / 2;
+        const CUtensorMap ma = plane_map(planesA, Rpad, Kpad, BM, 1), mb = plane_map(planesB, Nall, Kpad, BN, NP);
+        const long long items = e64_items(g);
+        {
+            Ctx::Scope s(ctx, name);
+            gett_e64_kernel<<<(unsigned)std::min<long long>(items, 152), THREADS, SMEM, ctx->stream>>>(ma, mb, g);
+            JUES_CHECK_CUDA(cudaGetLastError());
+        }
+        if (ksplit > 1) {
+            const std::string nm = std::string(name) + ".reduce";
+            Ctx::Scope s(ctx, nm.c_str());
+            e64_parts_kernel<<<(unsigned)(g.mtiles * g.ntiles), DRAIN, 0, ctx->stream>>>(g);
+            JUES_CHECK_CUDA(cudaGetLastError());
+        }
+    }
+    if (newA) pc.cached.push_back(std::move(newA));
+    if (newB) pc.cached.push_back(std::move(newB));
+    gett_f64_tiles(ctx, a, pc.e64_list.p, mtiles_all, name);
+    return true;
+}
+
+}  // namespace jues

@@ -11,6 +11,7 @@
 
 #include "common.cuh"
 #include "convert.cuh"
+#include "gett_e64.cuh"
 #include "gett_f64.cuh"
 
 namespace jues {
@@ -187,6 +188,19 @@ __global__ void __launch_bounds__(NT) gett_f64_grouped(const GroupProblem *__res
             if (probs[mid].tile_start <= t) lo = mid; else hi = mid - 1;
         }
         gett_tile<BM, BN>(probs[lo], t - probs[lo].tile_start, sm, 0, probs[lo].K);
+    }
+}
+
+// the tiles the tensor-core form left out (gett_e64.cu): entry t of the list is the 128 x 32 tile
+// (t % mtiles, t / mtiles), here two 64 x 32 ones.  The list is nearly always empty.
+__global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(GroupProblem g, const int *__restrict__ list,
+                                                            long long mtiles128) {
+    __shared__ TileSmem<64, 32> sm;
+    const int n = 2 * list[0];
+    for (int x = blockIdx.x; x < n; x += gridDim.x) {
+        const long long t = list[1 + x / 2];
+        const long long mt = 2 * (t % mtiles128) + (x & 1);
+        if (mt < g.mtiles) gett_tile<64, 32>(g, mt + g.mtiles * (t / mtiles128), sm, 0, g.K);
     }
 }
 
@@ -374,8 +388,18 @@ GroupProblem to_problem(const GettArgs &a) {
     return g;
 }
 
+void gett_f64_tiles(Ctx *ctx, const GettArgs &a, const int *list, long long mtiles, const char *name) {
+    GroupProblem g = to_problem(a);
+    g.mtiles = (a.M + 63) / 64;
+    const std::string nm = std::string(name) + ".rest";
+    Ctx::Scope s(ctx, nm.c_str());
+    gett_f64_tiles_kernel<<<152 * 4, NT, 0, ctx->stream>>>(g, list, mtiles);
+    JUES_CHECK_CUDA(cudaGetLastError());
+}
+
 void gett_f64(Ctx *ctx, const GettArgs &a, const char *name) {
     if (a.M <= 0 || a.N <= 0) return;
+    if (gett_e64(ctx, a, name)) return;
     GroupProblem g = to_problem(a);
     if (a.N > 8 && a.M * a.N <= (1LL << 16) && a.K <= 8192) {
         Ctx::Scope s(ctx, name);

@@ -36,6 +36,8 @@
 
 #include "common.cuh"
 #include "convert.cuh"
+#include "packcache.cuh"
+#include "tcgen05.cuh"
 
 namespace jues {
 
@@ -43,65 +45,7 @@ namespace {
 
 constexpr int TBM = 128;   // tile rows (TMEM lanes)
 constexpr int TBK = 64;    // K elements per stage: 128 bytes of FP16 = one swizzle atom row
-constexpr unsigned long long WAIT_LIMIT_NS = 2ull * 1000 * 1000 * 1000;    // 2 s: legitimate waits last microseconds
 
-__device__ __forceinline__ uint32_t smem_u32(const void *p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ unsigned long long gtimer() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
-                 : "memory");
-}
-// try_wait with a suspend-time hint: a waiting thread sleeps until the phase completes (or up to
-// 20 us) instead of polling, which keeps the spinning warps off the shared-memory pipe the
-// tensor cores read their operands through
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
-        : "memory");
-    return ok != 0;
-}
-// bounded wait; false when the time limit expired, another thread of the CTA aborted, or
-// another CTA already raised FLAG_TIMEOUT
-__device__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag,
-                          const volatile unsigned *gflags) {
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 15u) == 15u) {
-            if (*abort_flag || (*gflags & FLAG_TIMEOUT)) return false;
-            unsigned long long t = gtimer();
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > WAIT_LIMIT_NS) return false;
-        }
-    }
-}
-// bounded wait that ignores the abort flags: used only to let this CTA's own asynchronous
-// copies and MMAs settle before it frees TMEM and exits
-__device__ bool mbar_wait_quiet(uint64_t *bar, uint32_t parity) {
-    unsigned long long t0 = 0;
-    for (uint32_t it = 0;; ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((it & 15u) == 15u) {
-            unsigned long long t = gtimer();
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > WAIT_LIMIT_NS) return false;
-        }
-    }
-}
 // a wait on a barrier phase that nothing completes: the bounded wait expires and the kernel
 // raises FLAG_TIMEOUT, the failure path of every pipeline wait, exercised without a fault
 __global__ void expired_wait_kernel(unsigned *flags) {
@@ -114,88 +58,6 @@ __global__ void expired_wait_kernel(unsigned *flags) {
     }
     __syncthreads();
     if (threadIdx.x == 0 && !mbar_wait(&bar, 0u, &abort_flag, flags)) atomicOr(flags, FLAG_TIMEOUT);
-}
-
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y,
-                                            int z) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
-        "[%5];" ::"r"(smem_u32(dst)),
-        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-                 "r"(ncols)
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_relinquish() {
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// D[tmem] (+)= A[smem desc] . B[smem desc]^T, 16-bit inputs, FP32 accumulation
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
-}
-// 32 lanes x 32 consecutive 32-bit TMEM columns -> 32 registers per thread
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-          "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]),
-          "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]),
-          "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr));
-}
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// packed FP32 pairs (sm_100+): two round-to-nearest operations per instruction
-__device__ __forceinline__ uint64_t pk2(uint32_t lo, uint32_t hi) {
-    uint64_t r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(lo), "r"(hi));
-    return r;
-}
-__device__ __forceinline__ uint64_t pk2f(float lo, float hi) { return pk2(__float_as_uint(lo), __float_as_uint(hi)); }
-__device__ __forceinline__ uint64_t ffma2(uint64_t a, uint64_t b, uint64_t c) {
-    uint64_t d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ uint64_t fmul2(uint64_t a, uint64_t b) {
-    uint64_t d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ float lo_f(uint64_t x) { return __uint_as_float((uint32_t)x); }
-__device__ __forceinline__ float hi_f(uint64_t x) { return __uint_as_float((uint32_t)(x >> 32)); }
-__device__ __forceinline__ void red_add_f64(double *p, double v) {
-    asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
-}
-
-// UMMA shared-memory descriptor of a K-major tile written by TMA with 128-byte swizzle:
-// start address >> 4, LBO unused (1), SBO = 1024 bytes between 8-row groups, version 1,
-// layout type 2 = SWIZZLE_128B.
-__device__ __forceinline__ uint64_t sw128_desc(const void *smem) {
-    const uint64_t a = smem_u32(smem);
-    return ((a & 0x3FFFFull) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
 
 struct TcArgs {
@@ -265,10 +127,6 @@ struct TcCfg {
     static_assert(2 * BUF_COLS <= 512, "TMEM holds 512 columns");
     static_assert(NP * BN <= 256, "one MMA instruction spans at most N = 256");
 };
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
 
 // output tile index -> (m0, n0).  Raster: groups of (up to) 16 row tiles, rows fastest within a
 // group, so the CTAs resident at one time reuse a few row tiles' operand rows from L2 across
@@ -970,46 +828,9 @@ CUtensorMap make_map(const __half *base, long long rows_pad, long long kpad, int
 
 long long roundup(long long x, long long m) { return (x + m - 1) / m * m; }
 
-bool same_mode(const Mode &a, const Mode &b) {
-    return a.d0 == b.d0 && a.d1 == b.d1 && a.s0 == b.s0 && a.s1 == b.s1 && a.s2 == b.s2;
-}
-
 }  // namespace
 
-// ---------------------------------------------------------------------------------------
-// packed-operand cache: scratch planes for transient operands, persistent planes for
-// operands declared constant (integrals), dropped explicitly.
-// ---------------------------------------------------------------------------------------
-struct PackEntry {
-    const double *src;
-    Mode r, k;
-    long long R, K, Rpad, Kpad;
-    int np;
-    DBuf<__half> buf;
-    DBuf<int> exps;
-};
-struct PackCache {
-    bool busy = false;   // inside a cache operation: frees of the cache's own buffers are not lookups
-    std::vector<std::unique_ptr<PackEntry>> cached;
-    DBuf<__half> scratch[2];
-    DBuf<int> scratch_exp[2];
-    // buffers of dropped entries, reused by later entries (no cudaFree/cudaMalloc per sweep)
-    std::vector<DBuf<__half>> free_planes;
-    std::vector<DBuf<int>> free_exps;
-};
-
-template <class T>
-static DBuf<T> take_buffer(Ctx *ctx, std::vector<DBuf<T>> &pool, size_t need) {
-    int best = -1;
-    for (int i = 0; i < (int)pool.size(); ++i)
-        if (pool[i].n >= need && (best < 0 || pool[i].n < pool[best].n)) best = i;
-    if (best >= 0 && pool[best].n <= 2 * need) {
-        DBuf<T> b = std::move(pool[best]);
-        pool.erase(pool.begin() + best);
-        return b;
-    }
-    return DBuf<T>(ctx, need);
-}
+// the packed-operand cache (packcache.cuh)
 struct Packed {
     const __half *planes;
     const int *exps;
@@ -1027,6 +848,28 @@ void pack_cache_clear(Ctx *ctx) {
         ctx->pack->free_exps.clear();
         ctx->pack->busy = false;
     }
+}
+// Device memory wanted elsewhere: give back what the FP64 digit planes hold (they are formed again, or
+// the FP64 pipe runs instead).  Frees are stream-ordered, so queued readers are safe.
+bool pack_cache_reclaim(Ctx *ctx) {
+    if (!ctx->pack || ctx->pack->busy) return false;
+    PackCache &pc = *ctx->pack;
+    pc.busy = true;
+    bool any = false;
+    auto e64 = [](const std::unique_ptr<PackEntry> &x) { return x->np == E64_NP; };
+    const size_t before = pc.cached.size();
+    pc.cached.erase(std::remove_if(pc.cached.begin(), pc.cached.end(), e64), pc.cached.end());
+    any = pc.cached.size() != before;
+    for (auto *b : {&pc.e64_planes[0], &pc.e64_planes[1]}) {
+        any = any || b->p;
+        b->reset();
+    }
+    for (auto *b : {&pc.e64_exps[0], &pc.e64_exps[1], &pc.e64_list}) {
+        any = any || b->p;
+        b->reset();
+    }
+    pc.busy = false;
+    return any;
 }
 // Entries are keyed by their source address.  Device memory is reused quickly (the context's
 // pool hands freed blocks out again), so every free of device memory forgets the entries whose
