@@ -18,14 +18,16 @@
 // products, relative Frobenius error for normal entries: 4.7e-17 at every size, the FMA kernels 1.3e-16
 // (K = 100) to 8.4e-16 (640^3).
 //
-// Speed (packs included): 6400^3 10.6 ms = 49 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.27 against
-// 8.1 ms; the MMAs alone would take 79% of the GEMM's time, TMEM reads and operand copies the rest.
+// Speed (packs included): 6400^3 10.6 ms = 49 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.25 against
+// 8.1 ms, 500000 x 100 x 100 0.93 against 11.8 ms.  At long K the MMAs paced by shared memory take about
+// four fifths of the time; at K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about
+// 8000 clocks a tile) does.
 //
 // That bound is relative to |a|_2 |b|_2, not to sum |a_k b_k|: rows whose large elements meet only
 // small ones of the other side (an operand graded along K) would lose relative accuracy that an
 // FMA loop keeps.  So every output tile is checked before it is stored: a tile with a row or a
 // column whose results all fall below 2^-5 / sqrt(K) of its bound, or with a row that holds a non-finite,
-// subnormal-only or extreme (beyond 2^+-400) maximum, is not stored but listed, and
+// subnormal-only or extreme (beyond 2^+-400) maximum, is not stored but listed (by halves), and
 // gett_f64_tiles recomputes the listed tiles on the FP64 pipe, with the same special values as ever.
 //
 // The tile is 128 x 32: TMEM holds two buffers of 7 x 32 FP32 columns, so the drain of one chunk
@@ -50,17 +52,27 @@ namespace jues {
 
 namespace {
 
-constexpr int NP = E64_NP;            // digit planes
+constexpr int NP = E64_NP;            // digit planes of the FP64 form (the kernels take 3 too)
 constexpr int BM = 128, BN = 32;      // output tile
 constexpr int CK = 64;                // K per chunk: 128 bytes of FP16, one swizzle row
 constexpr int SLOTS = 10;             // ring of A planes
-constexpr int A_BYTES = BM * CK * 2, B_BYTES = NP * BN * CK * 2;   // one A plane 16 KB; all of B 28 KB
-constexpr int RING_BYTES = SLOTS * A_BYTES + 2 * B_BYTES;
-constexpr int BUF_COLS = NP * BN;     // TMEM columns of one chunk buffer
-constexpr uint32_t TMEM_COLS = 512;
-constexpr int THREADS = 320, DRAIN = 256;
-constexpr int HB = BN / 2;            // columns per drain thread
-constexpr int SMEM = RING_BYTES + 256 + BN * 8 + BN * 4 + 1024;
+constexpr int A_BYTES = BM * CK * 2;  // one A plane, 16 KB
+constexpr int b_bytes(int np) { return np * BN * CK * 2; }   // all of B: 28 KB for seven planes
+constexpr int ring_bytes(int np) { return SLOTS * A_BYTES + 2 * b_bytes(np); }
+constexpr uint32_t TMEM_COLS = 512;   // two chunk buffers of np x 32 columns
+// sixteen drain warps: the drain and the epilogue are chains of short integer operations, and with
+// two warps per scheduler (eight in all) they issued one instruction in three clocks
+constexpr int THREADS = 576, DRAIN = 512;
+constexpr int HB = BN / 4;            // columns per drain thread
+constexpr int VN = BN / 2;            // columns of a vote: eight drain warps
+constexpr int BAR_BYTES = 512, ITEMS = 8;
+// what the drain warps of one half need of a tile
+struct Tables {
+    long long rowoff[BM], coloff[VN];
+    E64Out g;   // grouped: the problem's
+    short rowE[BM], colE[VN];
+};
+constexpr int smem_bytes(int np) { return ring_bytes(np) + BAR_BYTES + ITEMS * 16 + 6 * (int)sizeof(Tables) + 1024; }
 constexpr int E_MIN = 1023 - 400, E_MAX = 1023 + 400;   // biased exponents of regular row maxima
 
 // instruction descriptor: FP32 accumulate, FP16 A and B, both K-major, M = 128, N = n
@@ -68,100 +80,81 @@ __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
 
-struct E64Args {
-    long long M, N;             // rows of this launch's panel, columns
-    long long row0;             // first row of the panel in the whole output
-    int k16;                    // K steps of 16
-    int mtiles, ntiles;         // of this launch
-    long long mtiles_all;       // row tiles of the whole output (tile numbers in the list)
-    const int *expA, *expB;     // biased exponent of each row's largest element (0: zero row)
-    double alpha, beta;
-    int alpha_pow2, alpha_k, alpha_neg;
-    int beta_mode;              // 0: C = v; 1: C += v in place; 2: C = Cin + v; 3: C = beta Cin + v
-    double *C;
-    const double *Cin;
-    Mode mC, nC;
-    unsigned *flags;
-    int ksplit, kper;           // K parts of kper chunks each
-    longlong2 *part;            // ksplit > 1: [part][tile][BN][BM] pairs of 64-bit sums
-    int *list;                  // tiles left to the FP64 pipe
-    int weak;                   // a row or column is weak when no result reaches 2^-weak max|a| max|b|
-};
-
 __host__ __device__ __forceinline__ long long e64_items(const E64Args &g) {
     return (long long)g.mtiles * g.ntiles * g.ksplit;
 }
 
 // tile -> (m0, n0): groups of 16 row tiles, rows fastest within a group, so that resident CTAs share
 // a few row tiles' planes in L2
-__device__ __forceinline__ void e64_origin(const E64Args &g, int tile, int &m0, int &n0) {
-    const int G = min(g.mtiles, 16), span = G * g.ntiles;
+__device__ __forceinline__ void e64_origin(int mtiles, int ntiles, int tile, int &m0, int &n0) {
+    const int G = min(mtiles, 16), span = G * ntiles;
     const int grp = tile / span, in = tile - grp * span;
-    const int gm = min(G, g.mtiles - grp * G);
+    const int gm = min(G, mtiles - grp * G);
     m0 = (grp * G + in % gm) * BM;
     n0 = (in / gm) * BN;
 }
 
-// (hi 2^36 + lo) 2^sc as FP64 on the integer pipes, hi and lo the 64-bit sums S_0 2^18 + S_1 2^9 +
-// S_2 and S_3 2^27 + S_4 2^18 + S_5 2^9 + S_6 (|hi| < K 2^35, |lo| < K 2^46): the leading 63 bits, one
-// rounding (ties away)
-__device__ __forceinline__ double e64_value(long long hi, long long lo, int sc, int neg) {
+// The sums of one element, V = hi 2^36 + lo with hi = S_0 2^18 + S_1 2^9 + S_2 (|hi| < 1.01 K 2^34) and
+// lo = S_3 2^27 + S_4 2^18 + S_5 2^9 + S_6, as T = V 2^(up - 36) in 64 bits: up shifts hi's leading bit to bit 61
+// (at most by 30: then |hi| < 2^32), the bits of lo that fit follow.  The conversion of T is the one
+// rounding; 500000 x 100 x 100 takes 0.58 ms with the conversion instruction, 0.61 ms with the same done in
+// integer operations (about 25 on the half-rate integer pipe) and 0.71 ms with two FP64 additions.
+__device__ __forceinline__ long long e64_join(long long hi, long long lo, int &up) {
     hi += lo >> 36;
-    const unsigned long long rem = (unsigned long long)lo & ((1ull << 36) - 1ull);
-    // as many bits of the low part as fit below hi's leading bit
-    const int up = min(36, __clzll(hi ^ (hi >> 63)) - 1);
-    const long long t = (hi << up) | (long long)(rem >> (36 - up));
-    const unsigned long long mag = (unsigned long long)(t < 0 ? -t : t);
-    if (mag == 0) return 0.0;
-    const int lz = __clzll((long long)mag);
-    const unsigned long long nrm = mag << lz;
-    const unsigned long long r = (nrm >> 11) + ((nrm >> 10) & 1ull);
-    const int field = 1023 + 63 - lz + sc - up + 36;
-    unsigned long long bits = ((unsigned long long)(unsigned)(field - 1) << 52) + r;
-    if ((t < 0) != (neg != 0)) bits |= 1ull << 63;
-    return __longlong_as_double((long long)bits);
+    const unsigned r = (unsigned)(((unsigned long long)lo << 28) >> 32);   // lo mod 2^36, its top 32 bits
+    const unsigned h0 = (unsigned)hi;
+    const int h1 = (int)(hi >> 32);
+    up = min(30, __clz(h1 ^ (h1 >> 31)) - 2);
+    const unsigned t1 = __funnelshift_l(h0, (unsigned)h1, up), t0 = __funnelshift_l(r, h0, up);
+    return (long long)((unsigned long long)t1 << 32 | t0);
 }
 
-// One thread's row of a tile (16 columns): its sums become FP64 values (hi[j] is overwritten with
+// One thread's row of a tile (8 columns): its sums become FP64 values (hi[j] is overwritten with
 // the bits), and the checks above run.  ea: the row's biased exponent (0 outside M or a zero row);
-// colE: the columns' (shared memory).  Returns whether this thread saw a reason to leave the tile
-// to the FP64 pipe; warp-uniform parts are evaluated with the whole warp.
-__device__ __forceinline__ bool e64_finish(const E64Args &g, long long (&hi)[HB], const long long (&lo)[HB], int ea,
-                                           const int *colE) {
+// colE: the columns' (shared memory).  V's exponent before scaling compares a result with 2^-weak of its
+// bound 2^(ea + eb) whatever the exponents are.  Returns whether this thread saw a reason to leave the
+// tile to the FP64 pipe.
+template <bool LOW, class E>
+__device__ __forceinline__ bool e64_finish(const E64Out &g, long long (&hi)[HB], const long long (&lo)[HB], int ea,
+                                           const E *colE) {
     const bool live = ea != 0;
     bool bad = live && (ea < E_MIN || ea > E_MAX);
-    int nc = 0;
+    int eb[HB];
+    unsigned cols = 0;   // columns that are not zero
 #pragma unroll
     for (int j = 0; j < HB; ++j) {
-        const int eb = colE[j];
-        nc += eb != 0;
-        bad |= eb != 0 && (eb < E_MIN || eb > E_MAX);
+        eb[j] = colE[j];
+        if (eb[j]) cols |= 1u << j;
+        bad |= eb[j] != 0 && (unsigned)(eb[j] - E_MIN) > (unsigned)(E_MAX - E_MIN);
     }
-    const int nr = __popc(__ballot_sync(0xffffffffu, live));
     // one or two results of a row (column) may cancel further by chance, so they get more room
-    const int trow = g.weak + (nc >= 3 ? 0 : (nc == 2 ? 4 : 8)), tcol = g.weak + (nr >= 3 ? 0 : (nr == 2 ? 4 : 8));
-    bool strong_row = false;
+    const int few = min(__popc(cols), __popc(__ballot_sync(0xffffffffu, live)));
+    // |V 2^-36| >= 2^(34 - weak) in the exponent field
+    const unsigned thr = (unsigned)(1023 + 34 - g.weak - (few >= 3 ? 0 : (few == 2 ? 4 : 8))) << 20;
+    const int neg = g.alpha_neg ? (int)0x80000000 : 0;
+    const int sc0 = ea - 2 * 1022 - 70 + 36 + g.alpha_k;
+    unsigned strong = 0;
 #pragma unroll
     for (int j = 0; j < HB; ++j) {
-        const int eb = colE[j];
-        double v = 0.0;
-        int above = -4096;   // result exponent relative to the bound 2^(ea + eb)
-        if (live && eb != 0) {
-            const int sc = (ea - 1022) + (eb - 1022) - 70;
-            v = e64_value(hi[j], lo[j], sc + (g.alpha_pow2 ? g.alpha_k : 0), g.alpha_neg);
-            const int f = (int)((unsigned)__double2hiint(v) >> 20 & 0x7FFu);
-            above = v == 0.0 ? -4096 : f - 1022 - (ea - 1022) - (eb - 1022) - (g.alpha_pow2 ? g.alpha_k : 0);
-        }
-        strong_row |= above >= -trow;
-        const bool strong_col = __ballot_sync(0xffffffffu, above >= -tcol) != 0u;
-        bad |= nr > 0 && eb != 0 && !strong_col;
-        hi[j] = __double_as_longlong(g.alpha_pow2 ? v : g.alpha * v);
+        int up = 0;
+        const double v = __ll2double_rn(LOW ? e64_join(hi[j], lo[j], up) : hi[j]);   // 0 for a zero row or column
+        const int vh = __double2hiint(v);
+        const unsigned mag = (unsigned)vh & 0x7FFFFFFFu;
+        if (mag >= thr + (up << 20)) strong |= 1u << j;
+        const int sc = mag ? (sc0 + eb[j] - up) << 20 : 0;
+        hi[j] = __double_as_longlong(__hiloint2double((vh + sc) ^ neg, __double2loint(v)));
     }
-    return bad || (live && nc > 0 && !strong_row);
+    if (!g.alpha_pow2) {
+#pragma unroll
+        for (int j = 0; j < HB; ++j) hi[j] = __double_as_longlong(g.alpha * __longlong_as_double(hi[j]));
+    }
+    if (live) bad |= cols && !(strong & cols);
+    const unsigned any = __reduce_or_sync(0xffffffffu, live ? strong | 1u << 31 : 0u);
+    return bad || (any && (cols & ~any));
 }
 
 // store one thread's row through the output modes (co: column offsets, -1 past N)
-__device__ __forceinline__ void e64_store(const E64Args &g, const long long (&val)[HB], const long long *co,
+__device__ __forceinline__ void e64_store(const E64Out &g, const long long (&val)[HB], const long long *co,
                                           long long rowoff) {
     double *out = g.C + rowoff;
     if (g.beta_mode == 0) {
@@ -187,34 +180,46 @@ __device__ __forceinline__ void e64_store(const E64Args &g, const long long (&va
     }
 }
 
-__device__ __forceinline__ void e64_list_tile(const E64Args &g, int m0, int n0) {
-    const long long t = (g.row0 + m0) / BM + g.mtiles_all * (n0 / BN);
-    g.list[1 + atomicAdd(g.list, 1)] = (int)t;
+// tiles are listed by halves (16 columns), the unit of a vote
+__device__ __forceinline__ void e64_list_tile(const E64Out &g, int prob, int m0, int n0) {
+    const long long t = (g.row0 + m0) / BM + g.mtiles_all * (n0 / VN);
+    const int at = atomicAdd(g.list, 1);
+    g.list[1 + 2 * at] = prob;
+    g.list[2 + 2 * at] = (int)t;
 }
 
-// barrier over the drain threads (named barrier 1) that ORs a predicate over them
-__device__ __forceinline__ bool drain_any(bool pred) {
+// barrier over the 256 drain threads of one half (named barrier 1 or 2) that ORs a predicate over them
+__device__ __forceinline__ bool vote_any(int half, bool pred) {
     uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.or.pred q, 1, %2, p;\n\t"
+        "bar.red.or.pred q, %3, %2, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
-        : "r"((uint32_t)pred), "n"(DRAIN)
+        : "r"((uint32_t)pred), "n"(DRAIN / 2), "r"(half + 1)
         : "memory");
     return r != 0;
 }
 
-__device__ __forceinline__ int f2i(uint32_t x) { return __float2int_rn(__uint_as_float(x)); }
+// acc += integer(x) 2^sh, x the bits of an integer-valued FP32 sum
+template <int SH>
+__device__ __forceinline__ void add_sum(long long &acc, uint32_t x) {
+    asm("mad.wide.s32 %0, %1, %2, %0;" : "+l"(acc) : "r"(__float2int_rn(__uint_as_float(x))), "n"(1 << SH));
+}
 
 // Persistent: CTA b takes work items b, b + gridDim.x, ... (an item is one tile over one K part).
-// Warp 0 issues TMA, warp 1 owns TMEM and issues the MMAs, warps 2-9 drain (two per 32-lane TMEM
-// quarter, 16 columns each).  Every wait is bounded; on expiry the CTA raises FLAG_TIMEOUT, skips its
+// Warp 0 issues TMA, warp 1 owns TMEM and issues the MMAs, warps 2-17 drain (four per 32-lane TMEM
+// quarter, 8 columns each).  Every wait is bounded; on expiry the CTA raises FLAG_TIMEOUT, skips its
 // stores, waits for its own copies, frees TMEM and returns.
+// GROUPED: the launch covers ngp problems (gp, in order of item0) whose operand rows lie in shared planes;
+// item w belongs to the last problem with item0 <= w.  PL planes: 7 (FP64), or 3 = 27 bits with the six
+// products of j < 3 (split precision).
+template <int PL, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
     gett_e64_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-                    const __grid_constant__ E64Args g) {
+                    const __grid_constant__ E64Args g0, const E64Args *__restrict__ gp, int ngp, int nitems) {
+    constexpr int B_BYTES = b_bytes(PL), RING_BYTES = ring_bytes(PL), BUF_COLS = PL * BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *ringB = smem + SLOTS * A_BYTES;
@@ -225,15 +230,32 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint64_t *cfull = bempty + 2;        // [2] chunk accumulated in TMEM buffer
     uint64_t *cempty = cfull + 2;        // [2] chunk drained
     uint64_t *fin = cempty + 2;          // the MMA thread's last commit
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(fin + 1);
+    uint64_t *ifull = fin + 1;           // [ITEMS] an item's place is in the queue
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ifull + ITEMS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    long long *coloff = reinterpret_cast<long long *>(smem + RING_BYTES + 256);
-    int *colE = reinterpret_cast<int *>(coloff + BN);
+    int4 *queue = reinterpret_cast<int4 *>(smem + RING_BYTES + BAR_BYTES);   // [ITEMS] m0, n0, chunks, problem | part
+    Tables *tabs = reinterpret_cast<Tables *>(queue + ITEMS);                // three sets per half
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int nchunks_all = (g.k16 + 3) / 4;
-    const int tiles = g.mtiles * g.ntiles;
-    const int nitems = tiles * g.ksplit;
+    // the problem of item w, cur running on from the item before; what the loops need of it in registers
+    struct Shape {
+        int mtiles, ntiles, item0, k16, kper, rowA, rowB;
+    };
+    auto load_shape = [](const E64Args &g) {
+        return Shape{g.mtiles, g.ntiles, g.item0, g.k16, g.kper, g.rowA, g.rowB};
+    };
+    auto locate = [&](int w, int &cur, Shape &h) {
+        if constexpr (GROUPED) {
+            bool moved = false;
+            while (cur + 1 < ngp && gp[cur + 1].item0 <= w) {
+                ++cur;
+                moved = true;
+            }
+            if (moved) h = load_shape(gp[cur]);
+        }
+    };
+    auto first_shape = [&]() { return load_shape(GROUPED ? gp[0] : g0); };
+    unsigned *const flags = g0.flags;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < SLOTS; ++s) {
@@ -246,6 +268,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             mbar_init(&cfull[b], 1);
             mbar_init(&cempty[b], DRAIN);
         }
+        for (int i = 0; i < ITEMS; ++i) mbar_init(&ifull[i], 1);
         mbar_init(fin, 1);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -264,24 +287,36 @@ __global__ void __launch_bounds__(THREADS, 1)
         if (lane == 0) {
             // TMA: per chunk B's planes, then A's one by one; it counts A planes, gc chunks
             unsigned it = 0, gc = 0;
+            int cur = 0;
+            Shape g = first_shape();
             bool stop = false;
             auto wait = [&](uint64_t *bar, unsigned parity) {
-                if (mbar_wait(bar, parity, abort_flag, g.flags)) return true;
+                if (mbar_wait(bar, parity, abort_flag, flags)) return true;
                 *abort_flag = 1;
                 stop = true;
                 return false;
             };
-            for (int w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
-                const int tile = w % tiles, part = w / tiles;
+            unsigned ni = 0;
+            for (int w = blockIdx.x; w < nitems && !stop; w += gridDim.x, ++ni) {
+                locate(w, cur, g);
+                const int tiles = g.mtiles * g.ntiles, x = w - g.item0;
+                const int tile = x % tiles, part = x / tiles;
                 int m0, n0;
-                e64_origin(g, tile, m0, n0);
-                const int c0 = part * g.kper, c1 = min(nchunks_all, c0 + g.kper);
+                e64_origin(g.mtiles, g.ntiles, tile, m0, n0);
+                const int c0 = part * g.kper, c1 = min((g.k16 + 3) / 4, c0 + g.kper);
+                // the item's place for the drain warps.  Entry ni - 8 is read by then: B's buffer of item ni is
+                // free once the MMAs of item ni - 2 are done, whose accumulators item ni - 4 has left.
+                if (!wait(&bempty[gc & 1u], ((gc >> 1) & 1u) ^ 1u)) break;
+                queue[ni % ITEMS] = make_int4(m0, n0, c1 - c0, GROUPED ? cur : part * tiles + tile);
+                mbar_arrive(&ifull[ni % ITEMS]);
+                m0 += g.rowA;
+                n0 += g.rowB;
                 for (int c = c0; c < c1 && !stop; ++c, ++gc) {
                     const unsigned b = gc & 1u;
-                    if (!wait(&bempty[b], ((gc >> 1) & 1u) ^ 1u)) break;
+                    if (c > c0 && !wait(&bempty[b], ((gc >> 1) & 1u) ^ 1u)) break;
                     mbar_expect_tx(&bfull[b], B_BYTES);
                     tma_load_3d(ringB + b * B_BYTES, &mapB, &bfull[b], c * CK, n0, 0);
-                    for (int p = 0; p < NP; ++p, ++it) {
+                    for (int p = 0; p < PL; ++p, ++it) {
                         const unsigned s = it % SLOTS;
                         if (!wait(&aempty[s], ((it / SLOTS) & 1u) ^ 1u)) break;
                         mbar_expect_tx(&afull[s], A_BYTES);
@@ -300,33 +335,41 @@ __global__ void __launch_bounds__(THREADS, 1)
         // The whole warp walks the loops in step (see umma_warp)
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         unsigned s = 0, ph = 0, gc = 0;   // ring slot and its phase, chunks
+        int cur = 0;
+        Shape g = first_shape();
         bool stop = false;
         for (int w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
-            const int part = w / tiles;
-            const int c0 = part * g.kper, c1 = min(nchunks_all, c0 + g.kper);
+            locate(w, cur, g);
+            const int part = (w - g.item0) / (g.mtiles * g.ntiles);
+            int k16 = g.k16, c0 = part * g.kper, c1 = min((k16 + 3) / 4, c0 + g.kper);
+            if constexpr (GROUPED) {   // read from memory: warp-uniform by construction
+                k16 = __shfl_sync(0xffffffffu, k16, 0);
+                c0 = __shfl_sync(0xffffffffu, c0, 0);
+                c1 = __shfl_sync(0xffffffffu, c1, 0);
+            }
             for (int c = c0; c < c1; ++c, ++gc) {
                 const unsigned b = gc & 1u;
-                if ((gc >= 2 && !mbar_wait_warp(&cempty[b], ((gc >> 1) - 1u) & 1u, abort_flag, g.flags)) ||
-                    !mbar_wait_warp(&bfull[b], (gc >> 1) & 1u, abort_flag, g.flags)) {
+                if ((gc >= 2 && !mbar_wait_warp(&cempty[b], ((gc >> 1) - 1u) & 1u, abort_flag, flags)) ||
+                    !mbar_wait_warp(&bfull[b], (gc >> 1) & 1u, abort_flag, flags)) {
                     stop = true;
                     break;
                 }
                 const uint32_t b0 = sw128_lo(ringB + b * B_BYTES);
                 const uint32_t dbuf = tm + b * BUF_COLS;
-                const int steps = min(4, g.k16 - 4 * c);
+                const int steps = min(4, k16 - 4 * c);
 #pragma unroll
-                for (int p = 0; p < NP; ++p) {
-                    if (!mbar_wait_warp(&afull[s], ph, abort_flag, g.flags)) {
+                for (int p = 0; p < PL; ++p) {
+                    if (!mbar_wait_warp(&afull[s], ph, abort_flag, flags)) {
                         stop = true;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t a0 = sw128_lo(smem + s * A_BYTES);
                     if (steps == 4) {
-                        umma_warp_x4(dbuf + (uint32_t)(p * BN), a0, b0, idesc((NP - p) * BN), p == 0 ? 0u : 1u);
+                        umma_warp_x4(dbuf + (uint32_t)(p * BN), a0, b0, idesc((PL - p) * BN), p == 0 ? 0u : 1u);
                     } else {
                         for (int kk = 0; kk < steps; ++kk)   // 32 bytes per K = 16 step
-                            umma_warp(dbuf + (uint32_t)(p * BN), a0 + 2 * kk, b0 + 2 * kk, idesc((NP - p) * BN),
+                            umma_warp(dbuf + (uint32_t)(p * BN), a0 + 2 * kk, b0 + 2 * kk, idesc((PL - p) * BN),
                                       (p == 0 && kk == 0) ? 0u : 1u);
                     }
                     umma_commit_warp(&aempty[s]);
@@ -346,92 +389,128 @@ __global__ void __launch_bounds__(THREADS, 1)
         umma_commit_warp(fin);
         mbar_wait_quiet(fin, 0u);
     } else {
-        const int quarter = warp & 3, half = (warp - 2) >> 2;
-        const int dt = threadIdx.x - 64;
-        long long gc = 0;
-        bool ok = true;
-        for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
-            const int tile = w % tiles, part = w / tiles;
-            int m0, n0;
-            e64_origin(g, tile, m0, n0);
-            const int nchunks = min(nchunks_all, (part + 1) * g.kper) - part * g.kper;
-            // every drain thread has finished the previous item (which reads coloff and colE)
-            if (drain_any(*abort_flag != 0)) {
-                ok = false;
-                break;
-            }
-            const long long mrow = (long long)m0 + quarter * 32 + lane;
-            int ea = 0;
-            if (g.ksplit == 1) {
-                if (dt < BN) {
-                    const long long n = (long long)n0 + dt;
-                    coloff[dt] = n < g.N ? mode_off(g.nC, n) : -1;
-                    colE[dt] = n < g.N ? __ldg(g.expB + n) : 0;
+        // Per tile: add the chunks up, read the next tile's place and make its tables (their latency overlaps
+        // the conversion), finish, vote, store.  Each half of the tile's columns belongs to eight warps
+        // that vote and list by themselves, so that the halves drift apart and one's conversions overlap
+        // the other's waits.  The vote is the only barrier: the tables of tile w + 1 are written before the
+        // vote of tile w, and a thread still storing tile w - 1 reads others (three sets).  A failed wait
+        // makes the warp skip TMEM from then on but keep voting (its tiles count as weak), so no thread is
+        // left waiting at a barrier.
+        const int quarter = warp & 3, eighth = (warp - 2) >> 2, half = eighth >> 1, sub = (eighth & 1) * HB;
+        const int dt = (threadIdx.x - 64) & 255;   // within the half: warps 2-9 are half 0, 10-17 half 1
+        unsigned gc = 0, ni = 0;
+        int set = 0;
+        bool bad = false;
+        Tables *const mine = tabs + 3 * half;
+        // the next item's place (m0, n0, chunks, problem or part's tile), its tables into set tb
+        auto open = [&](int tb) -> int4 {
+            if (!bad) {
+                const bool got = mbar_wait(&ifull[ni % ITEMS], (ni / ITEMS) & 1u, abort_flag, flags);
+                if (!__all_sync(0xffffffffu, got)) {
+                    *abort_flag = 1;
+                    bad = true;
                 }
-                ea = mrow < g.M ? __ldg(g.expA + mrow) : 0;
             }
+            if (bad) return make_int4(0, 0, 0, 0);
+            const int4 I = queue[ni % ITEMS];
+            ++ni;
+            const E64Args &g = GROUPED ? gp[I.w] : g0;
+            Tables &T = mine[tb];
+            if constexpr (GROUPED) {
+                if (dt >= 160 && dt - 160 < (int)(sizeof(E64Out) / 8))
+                    reinterpret_cast<long long *>(&T.g)[dt - 160] =
+                        reinterpret_cast<const long long *>(static_cast<const E64Out *>(&g))[dt - 160];
+            }
+            if (GROUPED || g.ksplit == 1) {
+                if (dt < BM) {
+                    const long long m = (long long)I.x + dt;
+                    T.rowoff[dt] = m < g.M ? mode_off(g.mC, g.row0 + m) : -1;
+                    T.rowE[dt] = (short)(m < g.M ? __ldg(g.expA + m) : 0);
+                } else if (dt < BM + VN) {
+                    const int c = dt - BM;
+                    const long long n = (long long)I.y + half * VN + c;
+                    T.coloff[c] = n < g.N ? mode_off(g.nC, n) : -1;
+                    T.colE[c] = (short)(n < g.N ? __ldg(g.expB + n) : 0);
+                }
+            }
+            return I;
+        };
+        int4 I = make_int4(0, 0, 0, 0);
+        if ((int)blockIdx.x < nitems) I = open(0);
+        vote_any(half, false);
+        for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
+            const Tables &T = mine[set];
+            const E64Out &g = GROUPED ? T.g : static_cast<const E64Out &>(g0);
             long long hi[HB], lo[HB];
 #pragma unroll
             for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
-            bool bad = false;
-            for (int c = 0; c < nchunks; ++c, ++gc) {
-                const int buf = (int)(gc & 1);
-                const bool got = mbar_wait(&cfull[buf], (uint32_t)(gc >> 1) & 1u, abort_flag, g.flags);
-                if (!__all_sync(0xffffffffu, got)) {
-                    *abort_flag = 1;
-                    bad = true;   // the barrier below takes every drain thread out
-                    break;
+            for (int c = 0; c < I.z; ++c, ++gc) {
+                const unsigned buf = gc & 1u;
+                if (!bad) {
+                    const bool got = mbar_wait(&cfull[buf], (gc >> 1) & 1u, abort_flag, flags);
+                    if (!__all_sync(0xffffffffu, got)) {
+                        *abort_flag = 1;
+                        bad = true;   // the whole warp
+                    }
                 }
+                if (bad) continue;
                 __syncwarp();
                 tc_fence_after();
                 const uint32_t base =
-                    tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BUF_COLS + half * HB);
-                uint32_t r0[HB], r1[HB];
-                tmem_ld16(base, r0);
-                tmem_ld16(base + BN, r1);
+                    tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BUF_COLS + eighth * HB);
+                uint32_t r0[HB], r1[HB], r2[HB];
+                tmem_ld8(base, r0);
+                tmem_ld8(base + BN, r1);
+                tmem_ld8(base + 2 * BN, r2);
                 tmem_ld_wait();
-#pragma unroll
-                for (int j = 0; j < HB; ++j)
-                    hi[j] += (long long)f2i(r0[j]) * (1 << 18) + (long long)f2i(r1[j]) * (1 << 9);
-                tmem_ld16(base + 2 * BN, r0);
-                tmem_ld16(base + 3 * BN, r1);
-                tmem_ld_wait();
+                if constexpr (PL == 3) {
+                    tc_fence_before();
+                    mbar_arrive(&cempty[buf]);
+                }
 #pragma unroll
                 for (int j = 0; j < HB; ++j) {
-                    hi[j] += f2i(r0[j]);
-                    lo[j] += (long long)f2i(r1[j]) * (1 << 27);
+                    add_sum<18>(hi[j], r0[j]);
+                    add_sum<9>(hi[j], r1[j]);
+                    add_sum<0>(hi[j], r2[j]);
                 }
-                tmem_ld16(base + 4 * BN, r0);
-                tmem_ld16(base + 5 * BN, r1);
-                tmem_ld_wait();
+                if constexpr (PL > 3) {
+                    uint32_t r3[HB];
+                    tmem_ld8(base + 3 * BN, r0);
+                    tmem_ld8(base + 4 * BN, r1);
+                    tmem_ld8(base + 5 * BN, r2);
+                    tmem_ld8(base + 6 * BN, r3);
+                    tmem_ld_wait();
+                    tc_fence_before();
+                    mbar_arrive(&cempty[buf]);
 #pragma unroll
-                for (int j = 0; j < HB; ++j)
-                    lo[j] += (long long)f2i(r0[j]) * (1 << 18) + (long long)f2i(r1[j]) * (1 << 9);
-                tmem_ld16(base + 6 * BN, r0);
-                tmem_ld_wait();
-                tc_fence_before();
-                mbar_arrive(&cempty[buf]);
-#pragma unroll
-                for (int j = 0; j < HB; ++j) lo[j] += f2i(r0[j]);
+                    for (int j = 0; j < HB; ++j) {
+                        add_sum<27>(lo[j], r0[j]);
+                        add_sum<18>(lo[j], r1[j]);
+                        add_sum<9>(lo[j], r2[j]);
+                        add_sum<0>(lo[j], r3[j]);
+                    }
+                }
             }
-            if (drain_any(bad)) {   // also orders the coloff and colE stores
-                ok = false;
-                break;
-            }
-            if (g.ksplit > 1) {
-                longlong2 *dst = g.part + (((long long)part * tiles + tile) * BN + half * HB) * BM + quarter * 32 + lane;
+            const int m0 = I.x, n0 = I.y + half * VN, at = I.w;
+            set = set == 2 ? 0 : set + 1;
+            if (w + (int)gridDim.x < nitems) I = open(set);
+            if (!GROUPED && g0.ksplit > 1) {
+                longlong2 *dst = g0.part + ((long long)at * BN + eighth * HB) * BM + quarter * 32 + lane;
 #pragma unroll
                 for (int j = 0; j < HB; ++j) dst[(long long)j * BM] = make_longlong2(hi[j], lo[j]);
                 continue;
             }
-            const bool weak = e64_finish(g, hi, lo, ea, colE + half * HB);
-            if (drain_any(weak)) {
-                if (dt == 0) e64_list_tile(g, m0, n0);
-            } else if (mrow < g.M) {
-                e64_store(g, hi, coloff + half * HB, mode_off(g.mC, g.row0 + mrow));
+            const int row = quarter * 32 + lane;
+            const bool weak = e64_finish<(PL > 3)>(g, hi, lo, T.rowE[row], T.colE + sub);
+            if (vote_any(half, weak || bad)) {
+                // after a failed wait nothing is listed: the host reports the time-out
+                if (dt == 0 && *abort_flag == 0 && n0 < g.N) e64_list_tile(g, GROUPED ? at : 0, m0, n0);
+            } else if (T.rowoff[row] >= 0) {
+                e64_store(g, hi, T.coloff + sub, T.rowoff[row]);
             }
         }
-        if (!ok && lane == 0) atomicOr(g.flags, FLAG_TIMEOUT);
+        const bool ok = !bad;
+        if (!ok && lane == 0) atomicOr(flags, FLAG_TIMEOUT);
     }
     tc_fence_before();
     __syncthreads();
@@ -447,10 +526,10 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
     __shared__ long long coloff[BN];
     __shared__ int colE[BN];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int quarter = warp & 3, half = warp >> 2;
+    const int quarter = warp & 3, eighth = warp >> 2, half = eighth >> 1;
     const int tile = blockIdx.x, tiles = g.mtiles * g.ntiles;
     int m0, n0;
-    e64_origin(g, tile, m0, n0);
+    e64_origin(g.mtiles, g.ntiles, tile, m0, n0);
     if (threadIdx.x < BN) {
         const long long n = (long long)n0 + threadIdx.x;
         coloff[threadIdx.x] = n < g.N ? mode_off(g.nC, n) : -1;
@@ -462,7 +541,7 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
 #pragma unroll
     for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
     for (int s = 0; s < g.ksplit; ++s) {
-        const longlong2 *src = g.part + (((long long)s * tiles + tile) * BN + half * HB) * BM + quarter * 32 + lane;
+        const longlong2 *src = g.part + (((long long)s * tiles + tile) * BN + eighth * HB) * BM + quarter * 32 + lane;
 #pragma unroll
         for (int j = 0; j < HB; ++j) {
             const longlong2 p = src[(long long)j * BM];
@@ -471,11 +550,11 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
         }
     }
     __syncthreads();
-    const bool weak = e64_finish(g, hi, lo, ea, colE + half * HB);
-    if (__syncthreads_or(weak)) {
-        if (threadIdx.x == 0) e64_list_tile(g, m0, n0);
+    const bool weak = e64_finish<true>(g, hi, lo, ea, colE + eighth * HB);
+    if (vote_any(half, weak)) {
+        if ((threadIdx.x & 255) == 0 && n0 + half * VN < g.N) e64_list_tile(g, 0, m0, n0 + half * VN);
     } else if (mrow < g.M) {
-        e64_store(g, hi, coloff + half * HB, mode_off(g.mC, g.row0 + mrow));
+        e64_store(g, hi, coloff + eighth * HB, mode_off(g.mC, g.row0 + mrow));
     }
 }
 
@@ -504,26 +583,28 @@ __device__ __forceinline__ int exp_of(double x) {
     return e ? e : ((hi | (unsigned)__double2loint(x)) ? 1 : 0);
 }
 
-// the seven digits of x in a row whose largest biased exponent is E, each + 256 (0..512)
-__device__ __forceinline__ void digits(double x, int E, unsigned (&u)[NP]) {
+// the PL digits of x in a row whose largest biased exponent is E, each + 256 (0..512)
+template <int PL>
+__device__ __forceinline__ void digits(double x, int E, unsigned (&u)[PL]) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const int e = (int)(hi >> 20 & 0x7FFu);
-    const int sh = E - e;
+    // m 2^(9 PL - 54) >> (E - e), ties away from zero: m 2^9 >> sh
+    constexpr int DROP = 9 * (E64_NP - PL);
+    const int sh = E - e + DROP;
     long long q = 0;
     if (e != 0 && sh < 64) {
-        // m 2^9 >> sh, ties away from zero (exact for sh <= 9)
         const unsigned long long m = (((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << 9;
         q = sh == 0 ? (long long)m : (long long)((m + (1ull << (sh - 1))) >> sh);
         if (hi >> 31) q = -q;
     }
-    // + 256 in every digit: q + 256 (2^54 + 2^45 + ... + 1) is positive and its 9-bit fields are the
-    // balanced digits + 256
-    constexpr unsigned long long OFF = 256ull * ((1ull << 54) + (1ull << 45) + (1ull << 36) + (1ull << 27) +
-                                                 (1ull << 18) + (1ull << 9) + 1ull);
-    const unsigned long long s = (unsigned long long)q + OFF;
-    u[0] = (unsigned)(s >> 54);
+    // + 256 in every digit: the sum is positive and its 9-bit fields are the balanced digits + 256
+    unsigned long long OFF = 0;
 #pragma unroll
-    for (int p = 1; p < NP; ++p) u[p] = (unsigned)(s >> (9 * (NP - 1 - p))) & 511u;
+    for (int p = 0; p < PL; ++p) OFF += 256ull << (9 * p);
+    const unsigned long long s = (unsigned long long)q + OFF;
+    u[0] = (unsigned)(s >> (9 * (PL - 1)));
+#pragma unroll
+    for (int p = 1; p < PL; ++p) u[p] = (unsigned)(s >> (9 * (PL - 1 - p))) & 511u;
 }
 
 // digit pair -> two FP16 integers: 0x6400 | u is 1024 + u
@@ -533,15 +614,16 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned u0, unsigned u1) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
+template <int PL>
 struct PackSmem {
-    uint32_t outp[NP][PR][PPITCH];
+    uint32_t outp[PL][PR][PPITCH];
     long long roff[PR], koff[PK];
     int rowE[PR];
 };
 
 // LOCALMAX: K <= 128, the block sees whole rows and writes their exponents; else they are read
-template <bool KFAST, bool LOCALMAX>
-__device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, long long k0, PackSmem &sm) {
+template <int PL, bool KFAST, bool LOCALMAX>
+__device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, long long k0, PackSmem<PL> &sm) {
     auto &outp = sm.outp;
     auto &roff = sm.roff;
     auto &koff = sm.koff;
@@ -586,15 +668,15 @@ __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, 
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int r = row_of(i), E = rowE[r];
-        unsigned u0[NP], u1[NP];
-        digits(x[i][0], E, u0);
-        digits(x[i][1], E, u1);
+        unsigned u0[PL], u1[PL];
+        digits<PL>(x[i][0], E, u0);
+        digits<PL>(x[i][1], E, u1);
 #pragma unroll
-        for (int p = 0; p < NP; ++p) outp[p][r][pair_of(i)] = digit_pair(u0[p], u1[p]);
+        for (int p = 0; p < PL; ++p) outp[p][r][pair_of(i)] = digit_pair(u0[p], u1[p]);
     }
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < (NP * PR * 32) / 256; ++j) {
+    for (int j = 0; j < (PL * PR * 32) / 256; ++j) {
         const int idx = tid + 256 * j;
         const int seg = idx & 31, row = (idx >> 5) & (PR - 1), plane = idx >> 9;
         const long long k = k0 + 4 * seg;
@@ -605,18 +687,18 @@ __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, 
 }
 
 // both operands of a GEMM in one launch: blocks [0, a.blocks) pack a, the rest b
-template <bool LOCALMAX>
+template <int PL, bool LOCALMAX>
 __global__ void __launch_bounds__(256, 4) e64_pack_kernel(const __grid_constant__ PackArgs a,
                                                           const __grid_constant__ PackArgs b) {
-    __shared__ __align__(16) PackSmem sm;
+    __shared__ __align__(16) PackSmem<PL> sm;
     const bool second = blockIdx.x >= a.blocks;
     const PackArgs &P = second ? b : a;
     const unsigned blk = second ? blockIdx.x - a.blocks : blockIdx.x;
     const unsigned kb = (unsigned)((P.Kpad + PK - 1) / PK), rb = (unsigned)(P.Rpad / PR);
     if (P.kfast)
-        e64_pack_block<true, LOCALMAX>(P, (long long)(blk / kb) * PR, (long long)(blk % kb) * PK, sm);
+        e64_pack_block<PL, true, LOCALMAX>(P, (long long)(blk / kb) * PR, (long long)(blk % kb) * PK, sm);
     else
-        e64_pack_block<false, LOCALMAX>(P, (long long)(blk % rb) * PR, (long long)(blk / rb) * PK, sm);
+        e64_pack_block<PL, false, LOCALMAX>(P, (long long)(blk % rb) * PR, (long long)(blk / rb) * PK, sm);
 }
 
 // the rows' largest biased exponents for K > 128 (exps cleared before): a block covers 16 rows x kseg
@@ -695,10 +777,10 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 // digit planes [NP][rows][kpad]; one box = 64 K values (past kpad: zeros) x box_rows rows x box_planes
-CUtensorMap plane_map(const __half *base, long long rows, long long kpad, int box_rows, int box_planes) {
+CUtensorMap plane_map(const __half *base, long long rows, long long kpad, int np, int box_rows, int box_planes) {
     CUtensorMap m;
     std::memset(&m, 0, sizeof(m));
-    cuuint64_t dims[3] = {(cuuint64_t)kpad, (cuuint64_t)rows, (cuuint64_t)NP};
+    cuuint64_t dims[3] = {(cuuint64_t)kpad, (cuuint64_t)rows, (cuuint64_t)np};
     cuuint64_t strides[2] = {(cuuint64_t)kpad * 2, (cuuint64_t)rows * kpad * 2};
     cuuint32_t box[3] = {(cuuint32_t)CK, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
     cuuint32_t estr[3] = {1, 1, 1};
@@ -724,12 +806,13 @@ PackArgs pack_args(const double *src, const Mode &rm, const Mode &km, long long 
 }
 
 // digits of up to two operands (b may be null)
+template <int PL>
 void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
     PackArgs none{};
     const PackArgs &B = b ? *b : none;
     if (a.K <= PK) {
         Ctx::Scope s(ctx, "pack_e64");
-        e64_pack_kernel<true><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+        e64_pack_kernel<PL, true><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
         JUES_CHECK_CUDA(cudaGetLastError());
         return;
     }
@@ -744,7 +827,7 @@ void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
         JUES_CHECK_CUDA(cudaGetLastError());
     }
     Ctx::Scope s(ctx, "pack_e64");
-    e64_pack_kernel<false><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+    e64_pack_kernel<PL, false><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
     JUES_CHECK_CUDA(cudaGetLastError());
 }
 
@@ -752,11 +835,38 @@ void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
 // tiles' launch against the FP64 pipe, us): 640^3 51 against 763; 400^3 45 / 475; 200^3 (2^16 outputs or
 // fewer: a warp per output element on the FP64 pipe) 38 / 45; 150^3 35 / 25; 2304 x 48 x 48 (tiles on the
 // FP64 pipe) 30 / 63; 4000 x 16 x 25 31 / 41.  The line lies where the sides meet.  A side below 16 pads
-// too much, and |lo| < K 2^46 must stay below 2^63.
+// too much; K <= 2^16 keeps the 64-bit sums far from overflow (|lo| < K 2^46).
 bool wanted(long long M, long long N, long long K) {
-    if (std::min(M, N) < 16 || K < 8 || K >= (1 << 17)) return false;
+    if (std::min(M, N) < 16 || K < 8 || K > (1 << 16)) return false;
     const double flops = 2.0 * (double)M * (double)N * (double)K;
     return flops >= (M * N <= (1LL << 16) && K <= 8192 ? 1.6e7 : 3e6);
+}
+
+// the shared-memory limit is a per-device attribute of each kernel
+template <int PL, bool GROUPED>
+void allow_smem(Ctx *ctx) {
+    static std::atomic<unsigned long long> set{0};
+    const unsigned long long bit = ctx->device >= 0 && ctx->device < 64 ? 1ull << ctx->device : 0ull;
+    if (bit && (set.load() & bit)) return;
+    JUES_CHECK_CUDA(cudaFuncSetAttribute(gett_e64_kernel<PL, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         smem_bytes(PL)));
+    set.fetch_or(bit);
+}
+
+// an FMA loop's own error grows as sqrt(K): 2^-weak keeps 2^-61 2^weak at its level
+int weak_level(long long K) {
+    int kl = 0;
+    while ((1LL << kl) < K) ++kl;
+    return 5 + kl / 2;
+}
+
+void set_scaling(E64Args &g, double alpha, double beta, bool in_place) {
+    g.alpha = alpha; g.beta = beta;
+    int ak = 0;
+    g.alpha_pow2 = std::frexp(std::fabs(alpha), &ak) == 0.5 && ak - 1 >= -8 && ak - 1 <= 8;
+    g.alpha_k = g.alpha_pow2 ? ak - 1 : 0;
+    g.alpha_neg = g.alpha_pow2 && alpha < 0;
+    g.beta_mode = beta == 0.0 ? 0 : (beta == 1.0 ? (in_place ? 1 : 2) : 3);
 }
 
 struct Busy {
@@ -860,7 +970,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
             grow(ctx, pc.e64_planes[1], hB);
             grow(ctx, pc.e64_exps[1], (size_t)Nall);
         }
-        grow(ctx, pc.e64_list, (size_t)(mtiles_all * ntiles + 1));
+        grow(ctx, pc.e64_list, (size_t)(4 * mtiles_all * ntiles + 1));
         if (ksplit > 1)
             part = static_cast<longlong2 *>(
                 ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN * sizeof(longlong2)));
@@ -868,12 +978,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         if (e.code != JUES_ENOMEM) throw;
         return false;   // the FP64 pipe needs no planes
     }
-    static std::atomic<unsigned long long> attr_set{0};
-    const unsigned long long bit = ctx->device >= 0 && ctx->device < 64 ? 1ull << ctx->device : 0ull;
-    if (!bit || !(attr_set.load() & bit)) {
-        JUES_CHECK_CUDA(cudaFuncSetAttribute(gett_e64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
-        attr_set.fetch_or(bit);
-    }
+    allow_smem<NP, false>(ctx);
     // C = Cin + alpha AB into a dense column-major C: copy Cin over and add in place, off the FP64 pipe
     const double *Cin = a.Cin ? a.Cin : a.C;
     const bool disjoint = Cin + a.M * a.N <= a.C || a.C + a.M * a.N <= Cin;
@@ -895,35 +1000,29 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         const bool packB = r0 == 0 && !eB;
         const PackArgs pb = pack_args(a.B, a.nB, a.kB, 0, a.N, a.K, Nall, Kpad, expsB, planesB);
         if (!eA)
-            run_pack(ctx, pack_args(a.A, a.mA, a.kA, r0, R, a.K, Rpad, Kpad, expsA, planesA), packB ? &pb : nullptr);
+            run_pack<NP>(ctx, pack_args(a.A, a.mA, a.kA, r0, R, a.K, Rpad, Kpad, expsA, planesA), packB ? &pb : nullptr);
         else if (packB)
-            run_pack(ctx, pb, nullptr);
+            run_pack<NP>(ctx, pb, nullptr);
         E64Args g;
+        g.rowA = g.rowB = g.item0 = 0;
         g.M = R; g.N = a.N; g.row0 = r0;
         g.k16 = k16;
         g.mtiles = (int)(Rpad / BM); g.ntiles = (int)ntiles;
         g.mtiles_all = mtiles_all;
         g.expA = expsA; g.expB = expsB;
-        g.alpha = a.alpha; g.beta = a.beta;
-        int ak = 0;
-        g.alpha_pow2 = std::frexp(std::fabs(a.alpha), &ak) == 0.5 && ak - 1 >= -8 && ak - 1 <= 8;
-        g.alpha_k = g.alpha_pow2 ? ak - 1 : 0;
-        g.alpha_neg = g.alpha_pow2 && a.alpha < 0;
-        g.beta_mode = a.beta == 0.0 ? 0 : (a.beta == 1.0 ? (Cin == a.C ? 1 : 2) : 3);
+        set_scaling(g, a.alpha, a.beta, Cin == a.C);
         g.C = a.C; g.Cin = Cin; g.mC = a.mC; g.nC = a.nC;
         g.flags = ctx->d_flags;
         g.ksplit = ksplit; g.kper = kper;
         g.part = part;
         g.list = pc.e64_list.p;
-        // an FMA loop's own error grows as sqrt(K): 2^-weak keeps 2^-61 2^weak at its level
-        int kl = 0;
-        while ((1LL << kl) < a.K) ++kl;
-        g.weak = 5 + kl / 2;
-        const CUtensorMap ma = plane_map(planesA, Rpad, Kpad, BM, 1), mb = plane_map(planesB, Nall, Kpad, BN, NP);
+        g.weak = weak_level(a.K);
+        const CUtensorMap ma = plane_map(planesA, Rpad, Kpad, NP, BM, 1), mb = plane_map(planesB, Nall, Kpad, NP, BN, NP);
         const long long items = e64_items(g);
         {
             Ctx::Scope s(ctx, name);
-            gett_e64_kernel<<<(unsigned)std::min<long long>(items, 152), THREADS, SMEM, ctx->stream>>>(ma, mb, g);
+            gett_e64_kernel<NP, false><<<(unsigned)std::min<long long>(items, 152), THREADS, smem_bytes(NP),
+                                         ctx->stream>>>(ma, mb, g, nullptr, 0, (int)items);
             JUES_CHECK_CUDA(cudaGetLastError());
         }
         if (ksplit > 1) {
@@ -935,8 +1034,76 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     }
     if (newA) pc.cached.push_back(std::move(newA));
     if (newB) pc.cached.push_back(std::move(newB));
-    gett_f64_tiles(ctx, a, pc.e64_list.p, mtiles_all, name);
+    gett_f64_tiles(ctx, &a, nullptr, pc.e64_list.p, name);
     return true;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Grouped form: many contractions over row ranges of two sets of shared planes, one launch
+// ---------------------------------------------------------------------------------------------
+void e64_alloc(Ctx *ctx, E64Planes &P, long long rows, long long K, int np) {
+    JUES_REQUIRE(np == 3 || np == E64_NP, "digit planes must be 3 or 7");
+    JUES_REQUIRE(K >= 1 && K <= (1 << 16), "K out of range for the digit planes");
+    P.np = np;
+    P.rows = roundup(rows, BM);
+    P.K = K;
+    P.Kpad = roundup(K, 16);
+    JUES_REQUIRE(P.rows < (1LL << 31) && (P.rows / PR) * ((P.Kpad + PK - 1) / PK) < (1LL << 31), "too many operand rows");
+    P.planes = DBuf<__half>(ctx, (size_t)np * P.rows * P.Kpad);
+    P.exps = DBuf<int>(ctx, (size_t)P.rows);
+}
+
+void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const Mode &km, long long R) {
+    JUES_REQUIRE(R <= P.rows, "operand does not fit its planes");
+    const PackArgs a = pack_args(src, rm, km, 0, R, P.K, P.rows, P.Kpad, P.exps.p, P.planes.p);
+    if (P.np == 3)
+        run_pack<3>(ctx, a, nullptr);
+    else
+        run_pack<NP>(ctx, a, nullptr);
+}
+
+E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long rowA, long long M, long long rowB,
+                    long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
+                    int *list) {
+    E64Args g{};
+    g.M = M; g.N = N; g.row0 = 0;
+    g.rowA = (int)rowA; g.rowB = (int)rowB; g.item0 = item0;
+    g.k16 = (int)((A.K + 15) / 16);
+    g.mtiles = (int)(roundup(M, BM) / BM); g.ntiles = (int)(roundup(N, BN) / BN);
+    g.mtiles_all = g.mtiles;
+    g.expA = A.exps.p + rowA; g.expB = B.exps.p + rowB;
+    set_scaling(g, alpha, beta, true);
+    g.C = C; g.Cin = C; g.mC = mC; g.nC = nC;
+    g.flags = ctx->d_flags;
+    g.ksplit = 1; g.kper = (g.k16 + 3) / 4;
+    g.part = nullptr;
+    g.list = list;
+    g.weak = weak_level(A.K);
+    return g;
+}
+
+void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Args *probs, const GroupProblem *f64,
+                   int n, long long items, int *list, const char *name) {
+    if (n <= 0 || items <= 0) return;
+    JUES_REQUIRE(A.np == B.np && A.Kpad == B.Kpad && items < (1LL << 31), "mismatched planes");
+    const CUtensorMap ma = plane_map(A.planes.p, A.rows, A.Kpad, A.np, BM, 1),
+                      mb = plane_map(B.planes.p, B.rows, B.Kpad, B.np, BN, B.np);
+    JUES_CHECK_CUDA(cudaMemsetAsync(list, 0, sizeof(int), ctx->stream));
+    E64Args g{};
+    g.flags = ctx->d_flags;
+    const unsigned grid = (unsigned)std::min<long long>(items, 152);
+    {
+        Ctx::Scope s(ctx, name);
+        if (A.np == 3) {
+            allow_smem<3, true>(ctx);
+            gett_e64_kernel<3, true><<<grid, THREADS, smem_bytes(3), ctx->stream>>>(ma, mb, g, probs, n, (int)items);
+        } else {
+            allow_smem<NP, true>(ctx);
+            gett_e64_kernel<NP, true><<<grid, THREADS, smem_bytes(NP), ctx->stream>>>(ma, mb, g, probs, n, (int)items);
+        }
+        JUES_CHECK_CUDA(cudaGetLastError());
+    }
+    gett_f64_tiles(ctx, nullptr, f64, list, name);
 }
 
 }  // namespace jues

@@ -191,16 +191,19 @@ __global__ void __launch_bounds__(NT) gett_f64_grouped(const GroupProblem *__res
     }
 }
 
-// the tiles the tensor-core form left out (gett_e64.cu): entry t of the list is the 128 x 32 tile
-// (t % mtiles, t / mtiles), here two 64 x 32 ones.  The list is nearly always empty.
-__global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(GroupProblem g, const int *__restrict__ list,
-                                                            long long mtiles128) {
-    __shared__ TileSmem<64, 32> sm;
+// the tiles the tensor-core form left out (gett_e64.cu): an entry is a 128 x 16 tile of one problem,
+// here two 64 x 16 ones.  The list is nearly always empty.
+__global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(const GroupProblem one,
+                                                            const GroupProblem *__restrict__ probs,
+                                                            const int *__restrict__ list) {
+    __shared__ TileSmem<64, 16> sm;
     const int n = 2 * list[0];
     for (int x = blockIdx.x; x < n; x += gridDim.x) {
-        const long long t = list[1 + x / 2];
-        const long long mt = 2 * (t % mtiles128) + (x & 1);
-        if (mt < g.mtiles) gett_tile<64, 32>(g, mt + g.mtiles * (t / mtiles128), sm, 0, g.K);
+        GroupProblem g = probs ? probs[list[1 + (x & ~1)]] : one;
+        const long long t = list[2 + (x & ~1)], mt128 = (g.M + 127) / 128;
+        const long long mt = 2 * (t % mt128) + (x & 1);
+        g.mtiles = (g.M + 63) / 64;
+        if (mt < g.mtiles) gett_tile<64, 16>(g, mt + g.mtiles * (t / mt128), sm, 0, g.K);
     }
 }
 
@@ -388,12 +391,12 @@ GroupProblem to_problem(const GettArgs &a) {
     return g;
 }
 
-void gett_f64_tiles(Ctx *ctx, const GettArgs &a, const int *list, long long mtiles, const char *name) {
-    GroupProblem g = to_problem(a);
-    g.mtiles = (a.M + 63) / 64;
+void gett_f64_tiles(Ctx *ctx, const GettArgs *one, const GroupProblem *probs, const int *list, const char *name) {
+    GroupProblem g{};
+    if (one) g = to_problem(*one);
     const std::string nm = std::string(name) + ".rest";
     Ctx::Scope s(ctx, nm.c_str());
-    gett_f64_tiles_kernel<<<152 * 4, NT, 0, ctx->stream>>>(g, list, mtiles);
+    gett_f64_tiles_kernel<<<152 * 4, NT, 0, ctx->stream>>>(g, probs, list);
     JUES_CHECK_CUDA(cudaGetLastError());
 }
 
