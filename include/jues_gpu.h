@@ -55,7 +55,9 @@ extern "C" {
  * ("planes") carried exactly in FP16, with a power-of-two scale per 128-wide K chunk of a row.
  * Two planes (hi + lo, three products) keep ~2^-20 relative; three (hi + mid + lo, six products)
  * keep ~2^-24, the FP32 rounding of the chunk sums. */
-#define JUES_PREC_FP64 0       /* plain FP64 (the drop-in form)                                   */
+#define JUES_PREC_FP64 0       /* plain FP64 (the drop-in form): contractions of 3e6 flop and more run on the
+                                  tensor cores as exact sums of 9-bit digit products, rounded once; the
+                                  others, and tiles whose operands do not suit that, as FP64 FMAs  */
 #define JUES_PREC_SPLIT 1      /* the split form at <= 1 uEh: three planes for every contraction
                                   that produces integrals (four-index transforms, get_eri blocks,
                                   DF factors, the MP2 adjoint's back-transforms), two planes for
@@ -208,7 +210,8 @@ JUES_API int jues_rmp2_adjoint(jues_ctx *ctx, const double *gao, int n, const do
  * Energies and, when the pointer arrays are given, adjoints of many independent closed-shell
  * systems of uneven size.  All systems run in one CUDA graph of grouped persistent launches (one
  * per stage, 12 stages with the adjoint); the graph is cached for a repeated batch signature.
- * precision: JUES_PREC_FP64 runs every stage as a grouped FP64 GETT; the split forms add, for
+ * precision: JUES_PREC_FP64 runs every stage as a grouped FP64 GETT, on the tensor cores (exact
+ * digit products) where the stage is large enough; the split forms add, for
  * every stage whose contractions all have K <= 64 (all but the final dE/dC stage when every
  * nbf <= 64), the grouped three-plane tcgen05 GEMM as a candidate.  On first use each stage's
  * form is chosen by timing the candidates (autotuning).  Host arrays; gao_bar / C_bar are arrays
@@ -226,7 +229,8 @@ typedef struct {
     int tuned;            /* 1 if this call built, autotuned and captured the plan       */
     int nstages;          /* grouped GETT stages                                         */
     int tile_shape[16];   /* chosen form per stage: FP64 tiles 0 64x64, 1 32x64, 2 64x32,
-                             3 32x32; 4 the grouped three-plane tcgen05 GEMM             */
+                             3 32x32; 4 the grouped three-plane tcgen05 GEMM; 5 the grouped
+                             FP64 contraction on the tensor cores (FP64 only)            */
 } jues_batch_info;
 
 /* Which forms the batched entry point's autotuning may pick (no reference counterpart):

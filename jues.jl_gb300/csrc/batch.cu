@@ -18,6 +18,7 @@
 
 #include "common.cuh"
 #include "staging.cuh"
+#include "gett_e64.cuh"
 #include "gett_f64.cuh"
 #include "transform.cuh"
 
@@ -112,25 +113,54 @@ __global__ void __launch_bounds__(256) mp2_energy_grouped(const SysDesc *__restr
     if (threadIdx.x == 0) *S.e = acc;
 }
 
-// tile shape index kShapeTC: the grouped three-plane tcgen05 GEMM (gett_tc.cu)
-constexpr int kShapeTC = kNumTileShapes;
+// tile shape index kShapeTC: the grouped three-plane tcgen05 GEMM (gett_tc.cu); kShapeE64: the grouped FP64
+// form on the tensor cores (gett_e64.cu)
+constexpr int kShapeTC = kNumTileShapes, kShapeE64 = kNumTileShapes + 1;
+
+// K parts of one problem: the dense M x N sums at ws + part M N, added in part order into C
+struct PartSum {
+    const double *ws;
+    double *C;
+    Mode mC, nC;
+    long long M, N;
+    int parts;
+    double alpha;
+};
+__global__ void __launch_bounds__(256) part_sum_kernel(const PartSum *__restrict__ ps) {
+    const PartSum P = ps[blockIdx.x];
+    const long long n = P.M * P.N;
+    for (long long x = threadIdx.x + 256LL * blockIdx.y; x < n; x += 256LL * gridDim.y) {
+        double v = 0.0;
+        for (int s = 0; s < P.parts; ++s) v += P.ws[s * n + x];
+        P.C[mode_off(P.mC, x % P.M) + mode_off(P.nC, x / P.M)] = P.alpha * v;
+    }
+}
 
 struct Stage {
     std::vector<GroupProblem> probs;
     std::vector<GettArgs> args;   // the same problems, for the grouped tcgen05 form
     DBuf<GroupProblem> dev;
     TcGroup *tc = nullptr;        // built when the batch runs split precision and every K <= 64
+    E64Group *e64 = nullptr;      // built when the batch runs FP64, every K <= 128 and the stage is large enough
+    int parts = 0;                // K-split problems whose sums part_sum_kernel adds (0: none)
+    DBuf<double> ws;
+    DBuf<PartSum> sums;
     long long total = 0;
     int shape = 0;
     std::string name;
     Stage() = default;
     Stage(Stage &&o) noexcept
-        : probs(std::move(o.probs)), args(std::move(o.args)), dev(std::move(o.dev)), tc(o.tc), total(o.total),
-          shape(o.shape), name(std::move(o.name)) {
+        : probs(std::move(o.probs)), args(std::move(o.args)), dev(std::move(o.dev)), tc(o.tc), e64(o.e64),
+          parts(o.parts), ws(std::move(o.ws)), sums(std::move(o.sums)), total(o.total), shape(o.shape),
+          name(std::move(o.name)) {
         o.tc = nullptr;
+        o.e64 = nullptr;
     }
     Stage &operator=(Stage &&) = delete;
-    ~Stage() { tc_group_destroy(tc); }
+    ~Stage() {
+        tc_group_destroy(tc);
+        e64_group_destroy(e64);
+    }
 };
 
 }  // namespace
@@ -161,10 +191,79 @@ struct BatchCache {
 void batch_cache_destroy(BatchCache *c) { delete c; }
 
 static void run_stage(Ctx *ctx, Stage &st) {
-    if (st.shape == kShapeTC)
+    if (st.shape == kShapeE64) {
+        e64_group_exec(ctx, st.e64);
+        return;
+    }
+    if (st.shape == kShapeTC) {
         tc_group_run(ctx, st.tc);
-    else
-        gett_f64_grouped_launch(ctx, st.dev.p, (int)st.probs.size(), st.total, st.shape, st.name.c_str());
+        return;
+    }
+    gett_f64_grouped_launch(ctx, st.dev.p, (int)st.probs.size(), st.total, st.shape, st.name.c_str());
+    if (st.parts) {
+        Ctx::Scope s(ctx, "batch_part_sum");
+        part_sum_kernel<<<dim3((unsigned)st.parts, 4), 256, 0, ctx->stream>>>(st.sums.p);
+        JUES_CHECK_CUDA(cudaGetLastError());
+    }
+}
+
+// Long contractions with few output tiles (the final dE/dC stage: M, N <= nbf, K up to o v^2) leave the GPU to
+// a few blocks that walk all of K on the FP64 pipe; their K is cut into parts of about 1024 whose sums are
+// added in part order.  Cuts lie on multiples of d0 d1 of a three-index K mode, so a part is the same
+// contraction from another address.
+static void split_long_k(Ctx *ctx, Stage &st) {
+    std::vector<GroupProblem> out;
+    std::vector<PartSum> sums;
+    std::vector<size_t> at;
+    size_t words = 0;
+    for (const GroupProblem &p : st.probs) {
+        auto unit = [](const Mode &m) {
+            return m.d0 == MODE_BIG ? 1LL : (m.d1 == MODE_BIG ? m.d0 : m.d0 * m.d1);
+        };
+        const long long ua = unit(p.kA), ub = unit(p.kB), u = ua == ub ? ua : (ua == 1 ? ub : (ub == 1 ? ua : ua * ub));
+        const long long kper = std::max<long long>(u, 1024 / u * u), parts = (p.K + kper - 1) / kper;
+        if (p.K < 4096 || parts < 2 || p.beta != 0.0) {
+            out.push_back(p);
+            continue;
+        }
+        for (long long s = 0; s < parts; ++s) {
+            GroupProblem q = p;
+            q.K = std::min(kper, p.K - s * kper);
+            q.A = p.A + mode_off(p.kA, s * kper);
+            q.B = p.B + mode_off(p.kB, s * kper);
+            q.C = nullptr;   // ws + words, once it is allocated
+            q.mC = plain(1);
+            q.nC = plain(p.M);
+            q.alpha = 1.0;
+            at.push_back(out.size());
+            out.push_back(q);
+        }
+        sums.push_back(PartSum{nullptr, p.C, p.mC, p.nC, p.M, p.N, (int)parts, p.alpha});
+        words += (size_t)(parts * p.M * p.N);
+    }
+    if (sums.empty()) return;
+    try {
+        st.ws = DBuf<double>(ctx, words);
+        st.sums = DBuf<PartSum>(ctx, sums.size());
+    } catch (const Error &e) {
+        if (e.code != JUES_ENOMEM) throw;
+        st.ws.reset();
+        return;
+    }
+    size_t w = 0, k = 0;
+    for (PartSum &s : sums) {
+        s.ws = st.ws.p + w;
+        for (int i = 0; i < s.parts; ++i, ++k) {
+            out[at[k]].C = st.ws.p + w;
+            out[at[k]].Cin = out[at[k]].C;
+            w += (size_t)(s.M * s.N);
+        }
+    }
+    JUES_CHECK_CUDA(cudaMemcpyAsync(st.sums.p, sums.data(), sums.size() * sizeof(PartSum), cudaMemcpyHostToDevice,
+                                    ctx->stream));
+    ctx->sync();
+    st.parts = (int)sums.size();
+    st.probs = std::move(out);
 }
 
 static void run_gamma(Ctx *ctx, BatchPlan &bp) {
@@ -197,6 +296,12 @@ static void autotune(Ctx *ctx, BatchPlan &bp) {
     JUES_CHECK_CUDA(cudaEventCreate(&e1));
     for (size_t k = 0; k < bp.stages.size(); ++k) {
         Stage &st = bp.stages[k];
+        if (st.e64) {   // by its sizes, not by timing
+            st.shape = kShapeE64;
+            run_stage(ctx, st);
+            if ((int)k + 1 == bp.n_forward) run_gamma(ctx, bp);
+            continue;
+        }
         float best = -1.f;
         int best_shape = 0;
         // the FP64 tile shapes, and the grouped tcgen05 form where it was built
@@ -281,6 +386,11 @@ static std::unique_ptr<BatchPlan> make_plan(Ctx *ctx, const std::string &key, in
             int d[4] = {o, v, o, v};
             long long ostr[4] = {1, o, ov, ov * o};
             auto st = transform4_plan(A + f.g, n, Cs, d, A + f.K, ostr, A + f.b0, A + f.b1);
+            if (want_cb && o <= v) {
+                // the first quarter, sum_mu C_occ[mu,i] g[mu,nu,lam,sig], is also H''s first step: kept in b2
+                st[0].C = A + f.b2;
+                st[1].A = A + f.b2;
+            }
             for (int k = 0; k < 4; ++k) {
                 fwd[k].probs.push_back(to_problem(st[k]));
                 fwd[k].args.push_back(st[k]);
@@ -310,15 +420,20 @@ static std::unique_ptr<BatchPlan> make_plan(Ctx *ctx, const std::string &key, in
             int d1[4] = {n, v, o, v};
             long long os1[4] = {1, n, (long long)n * v, (long long)n * v * o};
             auto h = transform4_plan(A + f.g, n, C1, d1, A + f.H, os1, A + f.b0, A + f.b1);
-            const double *C2[4] = {Co, nullptr, Co, Cv};
+            const bool kept = o <= v;   // the forward transform started with C_occ on index 0
+            const double *C2[4] = {kept ? nullptr : Co, nullptr, Co, Cv};
             int d2[4] = {o, n, o, v};
             long long os2[4] = {1, o, (long long)o * n, (long long)o * n * o};
-            auto hp = transform4_plan(A + f.g, n, C2, d2, A + f.Hp, os2, A + f.b2, A + f.b3);
+            const long long in2[4] = {kept ? o : n, n, n, n};
+            auto hp = transform4_plan(kept ? A + f.b2 : A + f.g, n, C2, d2, A + f.Hp, os2, kept ? A + f.b3 : A + f.b2,
+                                      A + f.b3, in2);
             for (int k = 0; k < 3; ++k) {
                 third[k].probs.push_back(to_problem(h[k]));
-                third[k].probs.push_back(to_problem(hp[k]));
                 third[k].args.push_back(h[k]);
-                third[k].args.push_back(hp[k]);
+                if (k < (int)hp.size()) {
+                    third[k].probs.push_back(to_problem(hp[k]));
+                    third[k].args.push_back(hp[k]);
+                }
             }
             GettArgs a;   // dE/dC[mu,i] = 2 sum_{ajb} H[mu,(ajb)] G[i,(ajb)]
             a.M = n; a.N = o; a.K = ov * v;
@@ -357,6 +472,10 @@ static std::unique_ptr<BatchPlan> make_plan(Ctx *ctx, const std::string &key, in
     // dE/dC one when nbf <= 64) gets the grouped three-plane tcgen05 form as a tuning candidate
     if (split)
         for (Stage &st : bp->stages) st.tc = tc_group_build(ctx, st.args, (st.name + "_tc").c_str());
+    else if (ctx->batch_form != 1)
+        for (Stage &st : bp->stages) st.e64 = e64_group_build(ctx, st.args, (st.name + "_e64").c_str());
+    for (Stage &st : bp->stages)
+        if (!st.e64) split_long_k(ctx, st);
     return bp;
 }
 

@@ -561,7 +561,10 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
 // ---------------------------------------------------------------------------------------------
 // operand digits
 // ---------------------------------------------------------------------------------------------
-constexpr int PR = 16, PK = 128, PPITCH = PK / 2 + 2;   // pack block: 16 rows x 128 K; staged row pitch in words
+// pack block: 2048 elements, 32 rows x 64 K where K <= 64 and 16 rows x 128 K above
+constexpr int PK = 128;
+constexpr int pack_rows(long long kpad) { return kpad <= 64 ? 32 : 16; }
+constexpr int pack_k(long long kpad) { return kpad <= 64 ? 64 : 128; }
 
 // one operand of a pack launch: rows [row0, row0 + R) of src into digit planes [NP][Rpad][Kpad] and
 // the rows' exponents
@@ -588,15 +591,12 @@ template <int PL>
 __device__ __forceinline__ void digits(double x, int E, unsigned (&u)[PL]) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
     const int e = (int)(hi >> 20 & 0x7FFu);
-    // m 2^(9 PL - 54) >> (E - e), ties away from zero: m 2^9 >> sh
+    // m 2^(9 PL - 54) >> (E - e), ties away from zero: ((m 2^10 >> sh) + 1) >> 1
     constexpr int DROP = 9 * (E64_NP - PL);
     const int sh = E - e + DROP;
-    long long q = 0;
-    if (e != 0 && sh < 64) {
-        const unsigned long long m = (((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << 9;
-        q = sh == 0 ? (long long)m : (long long)((m + (1ull << (sh - 1))) >> sh);
-        if (hi >> 31) q = -q;
-    }
+    const unsigned long long m = (((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << 10;
+    long long q = (long long)(((sh < 64 && e != 0 ? m >> sh : 0ull) + 1ull) >> 1);
+    if (hi >> 31) q = -q;
     // + 256 in every digit: the sum is positive and its 9-bit fields are the balanced digits + 256
     unsigned long long OFF = 0;
 #pragma unroll
@@ -614,95 +614,115 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned u0, unsigned u1) {
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
-template <int PL>
+template <int PL, int KW>
 struct PackSmem {
-    uint32_t outp[PL][PR][PPITCH];
-    long long roff[PR], koff[PK];
+    static constexpr int PR = 2048 / KW;
+    uint32_t outp[PL][PR][KW / 2 + 2];   // pitch: the pair stores of both layouts free of bank conflicts
+    long long roff[PR], koff[KW];
     int rowE[PR];
 };
 
-// LOCALMAX: K <= 128, the block sees whole rows and writes their exponents; else they are read
-template <int PL, bool KFAST, bool LOCALMAX>
-__device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, long long k0, PackSmem<PL> &sm) {
-    auto &outp = sm.outp;
-    auto &roff = sm.roff;
-    auto &koff = sm.koff;
-    auto &rowE = sm.rowE;
+// LOCALMAX: the block sees whole rows (K <= KW) and writes their exponents; else they are read
+template <int PL, int KW, bool KFAST, bool LOCALMAX>
+__device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, long long k0, PackSmem<PL, KW> &sm) {
+    constexpr int PR = 2048 / KW, PAIRS = KW / 2;
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid < PR) {
         const long long r = r0 + tid;
-        roff[tid] = r < a.R ? mode_off(a.rm, a.row0 + r) : -1;
-        rowE[tid] = LOCALMAX ? 0 : (r < a.R ? a.exps[r] : 0);
-    } else if (tid >= 64 && tid < 64 + PK) {
+        sm.roff[tid] = r < a.R ? mode_off(a.rm, a.row0 + r) : -1;
+        sm.rowE[tid] = LOCALMAX ? 0 : (r < a.R ? a.exps[r] : 0);
+    } else if (tid >= 64 && tid < 64 + KW) {
         const long long k = k0 + tid - 64;
-        koff[tid - 64] = k < a.K ? mode_off(a.km, k) : -1;
+        sm.koff[tid - 64] = k < a.K ? mode_off(a.km, k) : -1;
     }
     __syncthreads();
-    auto row_of = [&](int i) { return KFAST ? (tid >> 6) + 4 * i : (tid & 15); };
-    auto pair_of = [&](int i) { return KFAST ? (tid & 63) : (tid >> 4) + 16 * i; };
+    auto row_of = [&](int i) { return KFAST ? tid / PAIRS + (256 / PAIRS) * i : tid & (PR - 1); };
+    auto pair_of = [&](int i) { return KFAST ? tid & (PAIRS - 1) : tid / PR + (256 / PR) * i; };
     double x[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const long long ro = roff[row_of(i)], ko = koff[2 * pair_of(i) + h];
+            const long long ro = sm.roff[row_of(i)], ko = sm.koff[2 * pair_of(i) + h];
             x[i][h] = (ro >= 0 && ko >= 0) ? __ldg(a.src + ro + ko) : 0.0;
         }
     if constexpr (LOCALMAX) {
         if constexpr (KFAST) {
+            // a warp's lanes share each of its four rows
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int m = __reduce_max_sync(0xffffffffu, max(exp_of(x[i][0]), exp_of(x[i][1])));
-                if (lane == 0) atomicMax(&rowE[row_of(i)], m);
+                if (lane == 0) atomicMax(&sm.rowE[row_of(i)], m);
             }
         } else {
             int m = 0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) m = max(m, max(exp_of(x[i][0]), exp_of(x[i][1])));
-            m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-            if (lane < 16) atomicMax(&rowE[lane], m);
+            if (PR == 16) m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            if (lane < PR) atomicMax(&sm.rowE[lane], m);
         }
         __syncthreads();
-        if (tid < PR) a.exps[r0 + tid] = rowE[tid];
+        if (tid < PR) a.exps[r0 + tid] = sm.rowE[tid];
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = row_of(i), E = rowE[r];
+        const int r = row_of(i), E = sm.rowE[r];
         unsigned u0[PL], u1[PL];
         digits<PL>(x[i][0], E, u0);
         digits<PL>(x[i][1], E, u1);
 #pragma unroll
-        for (int p = 0; p < PL; ++p) outp[p][r][pair_of(i)] = digit_pair(u0[p], u1[p]);
+        for (int p = 0; p < PL; ++p) sm.outp[p][r][pair_of(i)] = digit_pair(u0[p], u1[p]);
     }
     __syncthreads();
+    // PL planes x PR rows x KW / 4 pieces of 4 halves
 #pragma unroll
-    for (int j = 0; j < (PL * PR * 32) / 256; ++j) {
+    for (int j = 0; j < (PL * 512) / 256; ++j) {
         const int idx = tid + 256 * j;
-        const int seg = idx & 31, row = (idx >> 5) & (PR - 1), plane = idx >> 9;
+        const int seg = idx & (KW / 4 - 1), row = (idx / (KW / 4)) & (PR - 1), plane = idx >> 9;
         const long long k = k0 + 4 * seg;
         if (k >= a.Kpad) continue;
         *reinterpret_cast<uint2 *>(a.dst + ((size_t)plane * a.Rpad + (size_t)(r0 + row)) * a.Kpad + k) =
-            *reinterpret_cast<const uint2 *>(&outp[plane][row][2 * seg]);
+            *reinterpret_cast<const uint2 *>(&sm.outp[plane][row][2 * seg]);
     }
 }
 
 // both operands of a GEMM in one launch: blocks [0, a.blocks) pack a, the rest b
-template <int PL, bool LOCALMAX>
-__global__ void __launch_bounds__(256, 4) e64_pack_kernel(const __grid_constant__ PackArgs a,
+template <int PL, int KW, bool LOCALMAX>
+__global__ void __launch_bounds__(256, 5) e64_pack_kernel(const __grid_constant__ PackArgs a,
                                                           const __grid_constant__ PackArgs b) {
-    __shared__ __align__(16) PackSmem<PL> sm;
+    __shared__ __align__(16) PackSmem<PL, KW> sm;
     const bool second = blockIdx.x >= a.blocks;
     const PackArgs &P = second ? b : a;
     const unsigned blk = second ? blockIdx.x - a.blocks : blockIdx.x;
-    const unsigned kb = (unsigned)((P.Kpad + PK - 1) / PK), rb = (unsigned)(P.Rpad / PR);
+    const unsigned kb = (unsigned)((P.Kpad + KW - 1) / KW), rb = (unsigned)(P.Rpad / (2048 / KW));
     if (P.kfast)
-        e64_pack_block<PL, true, LOCALMAX>(P, (long long)(blk / kb) * PR, (long long)(blk % kb) * PK, sm);
+        e64_pack_block<PL, KW, true, LOCALMAX>(P, (long long)(blk / kb) * (2048 / KW), (long long)(blk % kb) * KW, sm);
     else
-        e64_pack_block<PL, false, LOCALMAX>(P, (long long)(blk % rb) * PR, (long long)(blk / rb) * PK, sm);
+        e64_pack_block<PL, KW, false, LOCALMAX>(P, (long long)(blk % rb) * (2048 / KW), (long long)(blk / rb) * KW, sm);
+}
+
+// many operands with K <= KW (a batch): block b packs the rows of the last operand with first[] <= b; Rpad is
+// the rows of the shared planes, dst and exps start at the operand's own rows
+template <int PL, int KW>
+__global__ void __launch_bounds__(256, 5) e64_pack_grouped_kernel(const PackArgs *__restrict__ ops,
+                                                                  const unsigned *__restrict__ first, int nops) {
+    __shared__ __align__(16) PackSmem<PL, KW> sm;
+    int lo = 0, hi = nops - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (first[mid] <= blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const PackArgs P = ops[lo];
+    const long long r0 = (long long)(blockIdx.x - first[lo]) * (2048 / KW);
+    if (P.kfast)
+        e64_pack_block<PL, KW, true, true>(P, r0, 0, sm);
+    else
+        e64_pack_block<PL, KW, false, true>(P, r0, 0, sm);
 }
 
 // the rows' largest biased exponents for K > 128 (exps cleared before): a block covers 16 rows x kseg
 // chunks of 128 K
+constexpr int PR = 16;
 template <bool KFAST>
 __device__ __forceinline__ void e64_rowmax_block(const PackArgs &a, long long r0, long long k0) {
     __shared__ long long roff[PR], koff[PK];
@@ -797,7 +817,7 @@ PackArgs pack_args(const double *src, const Mode &rm, const Mode &km, long long 
     p.src = src; p.rm = rm; p.km = km;
     p.row0 = row0; p.R = R; p.K = K; p.Rpad = Rpad; p.Kpad = Kpad;
     p.exps = exps; p.dst = dst;
-    p.blocks = (unsigned)((Rpad / PR) * ((Kpad + PK - 1) / PK));
+    p.blocks = (unsigned)((Rpad / pack_rows(Kpad)) * ((Kpad + pack_k(Kpad) - 1) / pack_k(Kpad)));
     p.kfast = km.s0 == 1 && km.d0 > 1;
     // about 16 blocks per SM in the row-maximum pass, at most 16 chunks a block
     const long long chunks = (K + PK - 1) / PK;
@@ -812,7 +832,10 @@ void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
     const PackArgs &B = b ? *b : none;
     if (a.K <= PK) {
         Ctx::Scope s(ctx, "pack_e64");
-        e64_pack_kernel<PL, true><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+        if (a.Kpad <= 64)
+            e64_pack_kernel<PL, 64, true><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+        else
+            e64_pack_kernel<PL, 128, true><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
         JUES_CHECK_CUDA(cudaGetLastError());
         return;
     }
@@ -827,7 +850,7 @@ void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
         JUES_CHECK_CUDA(cudaGetLastError());
     }
     Ctx::Scope s(ctx, "pack_e64");
-    e64_pack_kernel<PL, false><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
+    e64_pack_kernel<PL, 128, false><<<a.blocks + B.blocks, 256, 0, ctx->stream>>>(a, B);
     JUES_CHECK_CUDA(cudaGetLastError());
 }
 
@@ -884,6 +907,25 @@ PackEntry *find_entry(PackCache &pc, const double *src, const Mode &rm, const Mo
     return nullptr;
 }
 
+// the output's unit-stride mode on the TMEM-lane side (coalesced stores) unless padding says otherwise
+// (rows pad to 128, columns to 32)
+GettArgs orient(const GettArgs &a0) {
+    GettArgs a = a0;
+    const bool m_unit = a.mC.s0 == 1 && a.mC.d0 > 1, n_unit = a.nC.s0 == 1 && a.nC.d0 > 1;
+    auto cost = [](long long M, long long N, bool unit) {
+        return (double)roundup(M, BM) * (double)roundup(N, BN) * (unit ? 1.0 : 1.2);
+    };
+    if (cost(a.N, a.M, n_unit) < cost(a.M, a.N, m_unit)) {
+        std::swap(a.M, a.N);
+        std::swap(a.A, a.B);
+        std::swap(a.mA, a.nB);
+        std::swap(a.kA, a.kB);
+        std::swap(a.mC, a.nC);
+        std::swap(a.a_const, a.b_const);
+    }
+    return a;
+}
+
 template <class T>
 void grow(Ctx *ctx, DBuf<T> &b, size_t need) {
     if (b.n >= need) return;
@@ -904,21 +946,7 @@ constexpr size_t PANEL_HALVES = size_t(64) << 20;   // transient planes: panels 
 
 bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     if (!wanted(a0.M, a0.N, a0.K)) return false;
-    GettArgs a = a0;
-    // the output's unit-stride mode on the TMEM-lane side (coalesced stores) unless padding says
-    // otherwise (rows pad to 128, columns to 32)
-    const bool m_unit = a.mC.s0 == 1 && a.mC.d0 > 1, n_unit = a.nC.s0 == 1 && a.nC.d0 > 1;
-    auto cost = [](long long M, long long N, bool unit) {
-        return (double)roundup(M, BM) * (double)roundup(N, BN) * (unit ? 1.0 : 1.2);
-    };
-    if (cost(a.N, a.M, n_unit) < cost(a.M, a.N, m_unit)) {
-        std::swap(a.M, a.N);
-        std::swap(a.A, a.B);
-        std::swap(a.mA, a.nB);
-        std::swap(a.kA, a.kB);
-        std::swap(a.mC, a.nC);
-        std::swap(a.a_const, a.b_const);
-    }
+    GettArgs a = orient(a0);
     const long long Kpad = roundup(a.K, 16);   // rows of planes start on 32 bytes
     const long long Mall = roundup(a.M, BM), Nall = roundup(a.N, BM);
     if (Mall >= (1LL << 31) || Nall >= (1LL << 31) || Kpad >= (1LL << 30)) return false;
@@ -1062,13 +1090,13 @@ void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const M
         run_pack<NP>(ctx, a, nullptr);
 }
 
-E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long rowA, long long M, long long rowB,
-                    long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
+E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long K, long long rowA, long long M,
+                    long long rowB, long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
                     int *list) {
     E64Args g{};
     g.M = M; g.N = N; g.row0 = 0;
     g.rowA = (int)rowA; g.rowB = (int)rowB; g.item0 = item0;
-    g.k16 = (int)((A.K + 15) / 16);
+    g.k16 = (int)((K + 15) / 16);
     g.mtiles = (int)(roundup(M, BM) / BM); g.ntiles = (int)(roundup(N, BN) / BN);
     g.mtiles_all = g.mtiles;
     g.expA = A.exps.p + rowA; g.expB = B.exps.p + rowB;
@@ -1078,7 +1106,7 @@ E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long 
     g.ksplit = 1; g.kper = (g.k16 + 3) / 4;
     g.part = nullptr;
     g.list = list;
-    g.weak = weak_level(A.K);
+    g.weak = weak_level(K);
     return g;
 }
 
@@ -1105,5 +1133,111 @@ void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Ar
     }
     gett_f64_tiles(ctx, nullptr, f64, list, name);
 }
+
+// ---------------------------------------------------------------------------------------------
+// One stage of a batch: many contractions with K <= 128, their operands' rows side by side in two sets of
+// planes; one pack launch, one GEMM launch and the listed tiles' launch, which a CUDA graph can capture
+// ---------------------------------------------------------------------------------------------
+struct E64Group {
+    std::string name;
+    E64Planes A, B;
+    DBuf<E64Args> args;
+    DBuf<GroupProblem> f64;
+    DBuf<PackArgs> ops;
+    DBuf<unsigned> first;
+    DBuf<int> list;
+    int nprob = 0, nops = 0;
+    unsigned blocks = 0;
+    long long items = 0;
+};
+
+E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const char *name) {
+    // Measured on 24 systems of nbf 10 to 60: the eleven K <= 64 stages took 22 ms on the FP64 tiles and take
+    // 3 ms here; a stage below 1e8 flop in all costs its four launches more than that
+    double flops = 0.0;
+    long long kmax = 0;
+    std::vector<GettArgs> ps;
+    for (const GettArgs &a : in) {
+        if (a.M <= 0 || a.N <= 0) continue;
+        if (a.K < 1 || a.K > PK || (a.beta != 0.0 && a.beta != 1.0) || (a.beta == 1.0 && a.Cin && a.Cin != a.C))
+            return nullptr;
+        flops += 2.0 * (double)a.M * (double)a.N * (double)a.K;
+        kmax = std::max(kmax, a.K);
+        ps.push_back(orient(a));
+    }
+    if (flops < 1e8) return nullptr;
+    try {
+        std::unique_ptr<E64Group> g(new E64Group());
+        g->name = name;
+        long long rowsA = 0, rowsB = 0;
+        const long long pr = pack_rows(roundup(kmax, 16));
+        for (const GettArgs &a : ps) {
+            rowsA += roundup(a.M, pr);
+            rowsB += roundup(a.N, pr);
+        }
+        if (rowsA >= (1LL << 30) || rowsB >= (1LL << 30)) return nullptr;
+        e64_alloc(ctx, g->A, rowsA, kmax, NP);
+        e64_alloc(ctx, g->B, rowsB, kmax, NP);
+        long long items = 0;
+        for (const GettArgs &a : ps) items += e64_tiles(a.M, a.N);
+        if (items >= (1LL << 28)) return nullptr;
+        g->items = items;
+        g->list = DBuf<int>(ctx, (size_t)(4 * items + 1));
+        std::vector<E64Args> args;
+        std::vector<GroupProblem> f64;
+        std::vector<PackArgs> ops;
+        std::vector<unsigned> first;
+        long long ra = 0, rb = 0, at = 0;
+        auto pack = [&](const E64Planes &P, long long row, const double *src, const Mode &rm, const Mode &km, long long R,
+                        long long K) {
+            PackArgs p = pack_args(src, rm, km, 0, R, K, P.rows, P.Kpad, P.exps.p + row, P.planes.p + row * P.Kpad);
+            first.push_back(g->blocks);
+            g->blocks += (unsigned)(roundup(R, pr) / pr);
+            ops.push_back(p);
+        };
+        for (const GettArgs &a : ps) {
+            pack(g->A, ra, a.A, a.mA, a.kA, a.M, a.K);
+            pack(g->B, rb, a.B, a.nB, a.kB, a.N, a.K);
+            args.push_back(e64_problem(ctx, g->A, g->B, a.K, ra, a.M, rb, a.N, a.alpha, a.beta, a.C, a.mC, a.nC, (int)at,
+                                       g->list.p));
+            f64.push_back(to_problem(a));
+            ra += roundup(a.M, pr);
+            rb += roundup(a.N, pr);
+            at += e64_tiles(a.M, a.N);
+        }
+        g->nprob = (int)args.size();
+        g->nops = (int)ops.size();
+        g->args = DBuf<E64Args>(ctx, args.size());
+        g->f64 = DBuf<GroupProblem>(ctx, f64.size());
+        g->ops = DBuf<PackArgs>(ctx, ops.size());
+        g->first = DBuf<unsigned>(ctx, first.size());
+        auto up = [&](void *d, const void *h, size_t bytes) {
+            JUES_CHECK_CUDA(cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx->stream));
+        };
+        up(g->args.p, args.data(), args.size() * sizeof(E64Args));
+        up(g->f64.p, f64.data(), f64.size() * sizeof(GroupProblem));
+        up(g->ops.p, ops.data(), ops.size() * sizeof(PackArgs));
+        up(g->first.p, first.data(), first.size() * sizeof(unsigned));
+        ctx->sync();   // the host tables stay valid until then
+        return g.release();
+    } catch (const Error &e) {
+        if (e.code != JUES_ENOMEM) throw;
+        return nullptr;   // the FP64 tiles need no planes
+    }
+}
+
+void e64_group_exec(Ctx *ctx, E64Group *g) {
+    {
+        Ctx::Scope s(ctx, "pack_e64");
+        if (g->A.Kpad <= 64)
+            e64_pack_grouped_kernel<NP, 64><<<g->blocks, 256, 0, ctx->stream>>>(g->ops.p, g->first.p, g->nops);
+        else
+            e64_pack_grouped_kernel<NP, 128><<<g->blocks, 256, 0, ctx->stream>>>(g->ops.p, g->first.p, g->nops);
+        JUES_CHECK_CUDA(cudaGetLastError());
+    }
+    e64_group_run(ctx, g->A, g->B, g->args.p, g->f64.p, g->nprob, g->items, g->list.p, g->name.c_str());
+}
+
+void e64_group_destroy(E64Group *g) { delete g; }
 
 }  // namespace jues

@@ -51,14 +51,20 @@ void e64_alloc(Ctx *ctx, E64Planes &P, long long rows, long long K, int np);
 void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const Mode &km, long long R);
 // C[mC(m) + nC(n)] = alpha sum_k A[rowA + m, k] B[rowB + n, k] + beta C, beta 0 or 1; item0: the items of
 // the problems before it in the launch (e64_tiles each)
-E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long rowA, long long M, long long rowB,
-                    long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
+E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long K, long long rowA, long long M,
+                    long long rowB, long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
                     int *list);
 inline long long e64_tiles(long long M, long long N) { return ((M + 127) / 128) * ((N + 31) / 32); }
 // one launch over n problems (device tables: probs, and f64 the same contractions for the FP64 pipe);
 // list holds 4 items + 1 ints
 void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Args *probs, const GroupProblem *f64,
                    int n, long long items, int *list, const char *name);
+
+// a stage of a batch (K <= 128 throughout): null when the sizes or the memory left do not suit it
+struct E64Group;
+E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &probs, const char *name);
+void e64_group_exec(Ctx *ctx, E64Group *g);
+void e64_group_destroy(E64Group *g);
 
 // gett_f64.cu: recompute the listed output tiles on the FP64 pipe.  list[0] = count, then pairs
 // (problem, tile t): rows [128 (t % mt), + 128), columns [16 (t / mt), + 16) of the problem's output, mt =

@@ -351,7 +351,7 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
                     long long w0 = 0;
                     for (int p = 0; p < b.npair; ++p) {
                         const PtTerm m = pt_term(t, i, j, o, v);
-                        args.push_back(e64_problem(ctx, st->pr, st->pq, m.rowA, m.M, m.rowB, m.N, 1.0, t ? 1.0 : 0.0,
+                        args.push_back(e64_problem(ctx, st->pr, st->pq, st->K, m.rowA, m.M, m.rowB, m.N, 1.0, t ? 1.0 : 0.0,
                                                    W.p + w0, m.mC, m.nC, (int)n, lp));
                         GettArgs g;
                         g.M = m.M; g.N = m.N; g.K = st->K;
