@@ -143,10 +143,8 @@ static const double *ao_operand(Ctx &c, const double *gao, size_t n4, int prec, 
     return hold.p;
 }
 
-void d2h(Ctx &ctx, double *h, const double *d, size_t n) {
-    if (n) JUES_CHECK_CUDA(cudaMemcpyAsync(h, d, n * sizeof(double), cudaMemcpyDeviceToHost, ctx.stream));
-    ctx.sync();
-}
+// Device -> host copy into a caller's array (staging.cu)
+void d2h(Ctx &ctx, double *h, const double *d, size_t n) { copy_out(&ctx, h, d, n); }
 
 void check_dims(int n, int o, int v) {
     if (n <= 0) throw Error(JUES_EINVAL, "nbf must be positive");

@@ -851,8 +851,7 @@ void cc_iterate(CCState *s, int nsweeps, int *done, int *converged) {
 void cc_amplitudes(CCState *s, double *t1_host, double *t2_host) {
     Ctx *ctx = s->ctx;
     const size_t t2n = (size_t)s->o * s->o * s->v * s->v;
-    if (t2_host)
-        JUES_CHECK_CUDA(cudaMemcpyAsync(t2_host, s->T.p, t2n * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    if (t2_host) copy_out(ctx, t2_host, s->T.p, t2n);
     if (t1_host) {
         if (s->method == 1)
             JUES_CHECK_CUDA(cudaMemcpyAsync(t1_host, s->t1.p, (size_t)s->o * s->v * sizeof(double),

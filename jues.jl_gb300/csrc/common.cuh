@@ -337,6 +337,8 @@ void ooov_diag_sums(Ctx *ctx, const double *ooov, int o, int v, double *c12);
 // dots[1 + k] = olds[k].e
 void diis_error(Ctx *ctx, size_t n, const double *xn, const double *x, double *v_out, double *e_out, int nold,
                 const double *const *olds, double *dots);
+// device -> host copy of n doubles into a caller's array, complete at return (staging.cu)
+void copy_out(Ctx *ctx, double *host, const double *dev, size_t n);
 // 1 if any element of x is NaN/Inf
 bool any_nonfinite(Ctx *ctx, const double *x, size_t n);
 

@@ -124,7 +124,7 @@ std::vector<Fill> plan_fills(const std::vector<HostSeg> &segs) {
 }  // namespace
 
 struct Staging {
-    char *host = nullptr;   // kSlots x kSlot, page-locked
+    char *host[kSlots] = {};   // kSlot bytes each, page-locked when first used (about 15 ms)
     cudaEvent_t done[kSlots] = {};
     bool busy[kSlots] = {};
     WorkerPool *pool = nullptr;
@@ -134,11 +134,16 @@ static Staging *staging_of(Ctx *ctx) {
     if (ctx->staging) return ctx->staging;
     Staging *st = new Staging;
     ctx->staging = st;   // released by staging_destroy, also when a step below fails
-    JUES_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&st->host), kSlot * kSlots, cudaHostAllocDefault));
     for (int k = 0; k < kSlots; ++k) JUES_CHECK_CUDA(cudaEventCreateWithFlags(&st->done[k], cudaEventDisableTiming));
     const unsigned hw = std::thread::hardware_concurrency();
     st->pool = new WorkerPool((int)std::min(15u, hw > 1 ? hw - 1 : 0u));
     return st;
+}
+
+static char *slot_of(Staging *st, int k) {
+    if (!st->host[k])
+        JUES_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&st->host[k]), kSlot, cudaHostAllocDefault));
+    return st->host[k];
 }
 
 // host side of one fill: copy the pieces' bytes between the slot and the caller's arrays in 1 MB
@@ -168,7 +173,7 @@ void staged_h2d(Ctx *ctx, const std::vector<HostSeg> &segs) {
     for (size_t i = 0; i < fills.size(); ++i) {
         const int k = (int)(i % kSlots);
         if (st->busy[k]) JUES_CHECK_CUDA(cudaEventSynchronize(st->done[k]));   // its last copy has left
-        char *slot = st->host + k * kSlot;
+        char *slot = slot_of(st, k);
         host_copy(st, fills[i], slot, true);
         for (const Fill::Piece &p : fills[i].pcs)
             JUES_CHECK_CUDA(cudaMemcpyAsync(p.dst, slot + p.at, p.bytes, cudaMemcpyHostToDevice, ctx->stream));
@@ -185,7 +190,7 @@ void staged_d2h(Ctx *ctx, const std::vector<HostSeg> &segs) {
     auto issue = [&](size_t i) {
         const int k = (int)(i % kSlots);
         if (st->busy[k]) JUES_CHECK_CUDA(cudaEventSynchronize(st->done[k]));
-        char *slot = st->host + k * kSlot;
+        char *slot = slot_of(st, k);
         for (const Fill::Piece &p : fills[i].pcs)
             JUES_CHECK_CUDA(cudaMemcpyAsync(slot + p.at, p.src, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
         JUES_CHECK_CUDA(cudaEventRecord(st->done[k], ctx->stream));
@@ -196,8 +201,30 @@ void staged_d2h(Ctx *ctx, const std::vector<HostSeg> &segs) {
         if (i + 1 < fills.size()) issue(i + 1);
         const int k = (int)(i % kSlots);
         JUES_CHECK_CUDA(cudaEventSynchronize(st->done[k]));
-        host_copy(st, fills[i], st->host + k * kSlot, false);
+        host_copy(st, fills[i], slot_of(st, k), false);
     }
+}
+
+// Device -> host into a caller's array, complete at return.  A copy into pageable memory of 16 MB and more
+// goes through the ring: the driver's own staging writes it with one host thread, page faults included
+// (the MP2 gradient at nbf=120, 1.66 GB into fresh arrays: 82 ms a call, 50 ms through the ring).  Smaller
+// copies and page-locked arrays are copied directly.
+void copy_out(Ctx *ctx, double *h, const double *d, size_t n) {
+    const size_t bytes = n * sizeof(double);
+    bool staged = bytes >= (size_t(16) << 20);
+    if (staged) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, h) != cudaSuccess) {
+            cudaGetLastError();
+            at.type = cudaMemoryTypeUnregistered;
+        }
+        staged = at.type == cudaMemoryTypeUnregistered;
+    }
+    if (staged)
+        staged_d2h(ctx, {HostSeg{h, d, bytes}});
+    else if (n)
+        JUES_CHECK_CUDA(cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    ctx->sync();
 }
 
 void staging_destroy(Staging *st) {
@@ -207,7 +234,8 @@ void staging_destroy(Staging *st) {
             cudaEventSynchronize(st->done[k]);
             cudaEventDestroy(st->done[k]);
         }
-    if (st->host) cudaFreeHost(st->host);
+    for (char *h : st->host)
+        if (h) cudaFreeHost(h);
     delete st->pool;
     delete st;
 }
