@@ -361,62 +361,55 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer: chunk gc (counted across items) accumulates into TMEM buffer gc & 1
-            long long it = 0, gc = 0;
-            bool stop = false;
-            for (long long w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
-                const TcArgs *G;
-                int ra, rb;
-                const TcItem I = locate(w, G, ra, rb);
-                for (int kb = 0; kb < I.nk; ++kb, ++it) {
-                    const int buf = (int)(gc & 1);
-                    const bool first = (kb % KC) == 0;
-                    if (first && gc >= 2) {
-                        if (!mbar_wait(&cempty[buf], (uint32_t)((gc >> 1) - 1) & 1u, abort_flag, g.flags)) {
-                            *abort_flag = 1;
-                            stop = true;
-                            break;
-                        }
-                        tc_fence_after();
-                    }
-                    const int s = (int)(it % STAGES);
-                    const uint32_t ph = (uint32_t)(it / STAGES) & 1u;
-                    if (!mbar_wait(&full[s], ph, abort_flag, g.flags)) {
-                        *abort_flag = 1;
-                        stop = true;
-                        break;
-                    }
-                    tc_fence_after();
-                    uint8_t *st = stages + s * Cfg::STAGE_BYTES;
-                    const uint64_t b0 = sw128_desc(st + NP * Cfg::A_BYTES);
-                    const uint32_t dbuf = tmem + (uint32_t)(buf * Cfg::BUF_COLS);
-                    // The B planes' rows are stacked in shared memory (B_BYTES = BN 128-byte rows,
-                    // whole 8-row swizzle groups) and the NP accumulators of a buffer are adjacent
-                    // TMEM column ranges, so plane p of A against B planes 0..NP-1-p is one
-                    // instruction with N = (NP - p) BN writing accumulators p..NP-1: accumulator
-                    // j collects every product A_p B_q with p + q = j (j < NP), and the products
-                    // with p + q >= NP (lo.lo, 2^-20 or 2^-30 smaller) are left out.
+        // MMA issuer (the whole warp in step, see umma_warp): chunk gc (counted across items)
+        // accumulates into TMEM buffer gc & 1
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        unsigned slot = 0, ph = 0, gc = 0;   // ring slot and its phase, chunks
+        bool stop = false;
+        for (long long w = blockIdx.x; w < nitems && !stop; w += gridDim.x) {
+            const TcArgs *G;
+            int ra, rb;
+            int nk = locate(w, G, ra, rb).nk;
+            nk = __shfl_sync(0xffffffffu, nk, 0);   // warp-uniform by construction
+            for (int kb = 0; kb < nk; ++kb) {
+                const unsigned buf = gc & 1u;
+                const bool first = (kb % KC) == 0;
+                if ((first && gc >= 2 && !mbar_wait_warp(&cempty[buf], ((gc >> 1) - 1u) & 1u, abort_flag, g.flags)) ||
+                    !mbar_wait_warp(&full[slot], ph, abort_flag, g.flags)) {
+                    stop = true;
+                    break;
+                }
+                tc_fence_after();
+                const uint32_t st = sw128_lo(stages + slot * Cfg::STAGE_BYTES), b0 = st + (NP * Cfg::A_BYTES >> 4);
+                const uint32_t dbuf = tm + buf * Cfg::BUF_COLS;
+                // The B planes' rows are stacked in shared memory (B_BYTES = BN 128-byte rows,
+                // whole 8-row swizzle groups) and the NP accumulators of a buffer are adjacent
+                // TMEM column ranges, so plane p of A against B planes 0..NP-1-p is one
+                // instruction with N = (NP - p) BN writing accumulators p..NP-1: accumulator
+                // j collects every product A_p B_q with p + q = j (j < NP), and the products
+                // with p + q >= NP (lo.lo, 2^-20 or 2^-30 smaller) are left out.
 #pragma unroll
-                    for (int kk = 0; kk < TBK / 16; ++kk) {
-                        const uint64_t off = (uint64_t)((kk * 16 * 2) >> 4);   // 32 bytes per K=16 step
-                        const uint32_t acc = (first && kk == 0) ? 0u : 1u;
+                for (int kk = 0; kk < TBK / 16; ++kk)   // 32 bytes per K = 16 step
 #pragma unroll
-                        for (int p = 0; p < NP; ++p)
-                            umma_bf16(dbuf + (uint32_t)(p * BN), sw128_desc(st + p * Cfg::A_BYTES) + off, b0 + off,
-                                      tc_idesc((NP - p) * BN), p == 0 ? acc : 1u);
-                    }
-                    umma_commit(&empty[s]);   // stage s free once these complete
-                    if ((kb % KC) == KC - 1 || kb == I.nk - 1) {
-                        umma_commit(&cfull[buf]);   // chunk done
-                        ++gc;
-                    }
+                    for (int p = 0; p < NP; ++p)
+                        umma_warp(dbuf + (uint32_t)(p * BN), st + (uint32_t)((p * Cfg::A_BYTES >> 4) + 2 * kk), b0 + 2 * kk,
+                                  tc_idesc((NP - p) * BN), (p == 0 && kk == 0 && first) ? 0u : 1u);
+                umma_commit_warp(&empty[slot]);   // the stage is free once these complete
+                if ((kb % KC) == KC - 1 || kb == nk - 1) {
+                    umma_commit_warp(&cfull[buf]);   // chunk done
+                    ++gc;
+                }
+                if (++slot == STAGES) {
+                    slot = 0;
+                    ph ^= 1u;
                 }
             }
-            // every MMA this thread issued has completed before TMEM is freed
-            umma_commit(fin);
-            mbar_wait_quiet(fin, 0u);
         }
+        if (stop) *abort_flag = 1;
+        __syncwarp();
+        // every MMA this warp issued has completed before TMEM is freed
+        umma_commit_warp(fin);
+        mbar_wait_quiet(fin, 0u);
     } else {
         // drain warps 2-9: TMEM lane quarter (warp % 4), one tile row per thread, half the columns.
         // They leave their loops only together: every exit test follows a barrier that ORs the
