@@ -860,7 +860,7 @@ void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
 // FP64 pipe) 30 / 63; 4000 x 16 x 25 31 / 41.  The line lies where the sides meet.  A side below 16 pads
 // too much; K <= 2^16 keeps the 64-bit sums far from overflow (|lo| < K 2^46).
 bool wanted(long long M, long long N, long long K) {
-    if (std::min(M, N) < 16 || K < 8 || K > (1 << 16)) return false;
+    if (std::min(M, N) <= 8 || K < 8 || K > (1 << 16)) return false;
     const double flops = 2.0 * (double)M * (double)N * (double)K;
     return flops >= (M * N <= (1LL << 16) && K <= 8192 ? 1.6e7 : 3e6);
 }

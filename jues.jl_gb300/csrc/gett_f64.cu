@@ -191,19 +191,26 @@ __global__ void __launch_bounds__(NT) gett_f64_grouped(const GroupProblem *__res
     }
 }
 
-// the tiles the tensor-core form left out (gett_e64.cu): an entry is a 128 x 16 tile of one problem,
-// here two 64 x 16 ones.  The list is nearly always empty.
+// the tiles the tensor-core form left out (gett_e64.cu): an entry is a 128 x 16 tile of one problem.  The
+// list is nearly always empty; a short one is spread as 16 x 16 tiles (one block walking a 64 x 16 tile's K of
+// 2500 takes a millisecond), a long one as 64 x 16.
 __global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(const GroupProblem one,
                                                             const GroupProblem *__restrict__ probs,
                                                             const int *__restrict__ list) {
     __shared__ TileSmem<64, 16> sm;
-    const int n = 2 * list[0];
-    for (int x = blockIdx.x; x < n; x += gridDim.x) {
-        GroupProblem g = probs ? probs[list[1 + (x & ~1)]] : one;
-        const long long t = list[2 + (x & ~1)], mt128 = (g.M + 127) / 128;
-        const long long mt = 2 * (t % mt128) + (x & 1);
-        g.mtiles = (g.M + 63) / 64;
-        if (mt < g.mtiles) gett_tile<64, 16>(g, mt + g.mtiles * (t / mt128), sm, 0, g.K);
+    const int n = list[0];
+    const int sub = n <= 512 ? 8 : 2, rows = 128 / sub;
+    for (int x = blockIdx.x; x < n * sub; x += gridDim.x) {
+        const int e = x / sub;
+        GroupProblem g = probs ? probs[list[1 + 2 * e]] : one;
+        const long long t = list[2 + 2 * e], mt128 = (g.M + 127) / 128;
+        const long long mt = sub * (t % mt128) + x % sub;
+        g.mtiles = (g.M + rows - 1) / rows;
+        if (mt >= g.mtiles) continue;
+        if (sub == 8)
+            gett_tile<16, 16>(g, mt + g.mtiles * (t / mt128), reinterpret_cast<TileSmem<16, 16> &>(sm), 0, g.K);
+        else
+            gett_tile<64, 16>(g, mt + g.mtiles * (t / mt128), sm, 0, g.K);
     }
 }
 
