@@ -856,9 +856,11 @@ void run_pack(Ctx *ctx, const PackArgs &a, const PackArgs *b) {
 
 // Whether the tensor cores take a contraction.  Measured through jues_gemm (packs, GEMM and the listed
 // tiles' launch against the FP64 pipe, us): 640^3 51 against 763; 400^3 45 / 475; 200^3 (2^16 outputs or
-// fewer: a warp per output element on the FP64 pipe) 38 / 45; 150^3 35 / 25; 2304 x 48 x 48 (tiles on the
-// FP64 pipe) 30 / 63; 4000 x 16 x 25 31 / 41.  The line lies where the sides meet.  A side below 16 pads
-// too much; K <= 2^16 keeps the 64-bit sums far from overflow (|lo| < K 2^46).
+// fewer; the FP64 side with a warp per output) 38 / 45; 150^3 35 / 25; 2304 x 48 x 48 (tiles on the
+// FP64 pipe) 30 / 63; 4000 x 16 x 25 31 / 41.  The line lies where the sides meet.  A side of 8 or
+// less has kernels of its own on the FP64 pipe; 9 to 15 pad the tile but gain all the same (13 x 50 x 8450
+// 37 to 60 / 640; CCSD with 13 occupied of 63 orbitals, six sweeps: 22.2 -> 10.3 ms).  K <= 2^16 keeps the 64-bit
+// sums far from overflow (|lo| < K 2^46).
 bool wanted(long long M, long long N, long long K) {
     if (std::min(M, N) <= 8 || K < 8 || K > (1 << 16)) return false;
     const double flops = 2.0 * (double)M * (double)N * (double)K;

@@ -356,9 +356,9 @@ __global__ void __launch_bounds__(256) gett_f64_rows(GroupProblem g, long long k
         if (j < g.N) part[(blockIdx.y * g.N + j) * g.M + m] = acc[j];
 }
 
-// small GEMM (M N <= 2^16 outputs, K <= 8192): one warp per output element, its lanes over K,
-// so that even a single-tile problem spreads over the whole GPU instead of one CTA
-__global__ void __launch_bounds__(256) gett_f64_small(GroupProblem g) {
+// Smallest GEMMs (M N <= 4096 outputs, K <= 8192): one warp per output element, its lanes over K, so that
+// even a single-tile problem spreads over the whole GPU instead of one CTA.  Latency bounds it.
+__global__ void __launch_bounds__(256) gett_f64_dots(GroupProblem g) {
     const long long w = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (w >= g.M * g.N) return;
@@ -381,6 +381,61 @@ __global__ void __launch_bounds__(256) gett_f64_small(GroupProblem g) {
         if (g.beta != 0.0) r = fma(g.beta, g.Cin[off], r);
         g.C[off] = r;
     }
+}
+
+// Small GEMM: 2^ll threads share two neighbouring outputs of a row and split K; ll is chosen for about
+// 40,000 threads in all.  FP64 issue and latency bound it, so the lanes' tree sums are kept short: with a
+// warp per output, a K = 16 product of 256 x 256 spends more on the five additions and shuffles of each
+// output than on its products (44 us, here 12).  The K offsets of both operands are tabulated once per
+// block.  kfast: neighbouring threads take neighbouring K positions of one row (A's K is its unit-stride
+// index), else neighbouring rows.  MP2 with nbf = 25 (quarter transforms with five columns): 213 -> 127 us;
+// RCCD with nbf = 25, twelve sweeps: 3.80 -> 3.20 ms.
+constexpr int SMALL_K = 512;
+__global__ void __launch_bounds__(256) gett_f64_small(GroupProblem g, int ll, int kfast) {
+    __shared__ long long ka[SMALL_K], kb[SMALL_K];
+    const int tid = threadIdx.x, lane = tid & 31, L = 1 << ll;
+    const long long t = blockIdx.x * 256LL + tid;
+    const int kl = kfast ? lane & (L - 1) : lane >> (5 - ll);
+    const long long task = kfast ? t >> ll : (t >> 5) * (32 >> ll) + (lane & ((32 >> ll) - 1));
+    const bool live = task < g.M * ((g.N + 1) / 2);
+    long long nb, m;
+    divmod_ll(live ? task : 0, g.M, nb, m);
+    const long long n0 = 2 * nb, n1 = n0 + 1 < g.N ? n0 + 1 : n0;
+    const double *pa = g.A + mode_off(g.mA, m);
+    const double *p0 = g.B + mode_off(g.nB, n0), *p1 = g.B + mode_off(g.nB, n1);
+    double acc0 = 0.0, acc1 = 0.0;
+    for (long long k0 = 0; k0 < g.K; k0 += SMALL_K) {
+        const int kn = (int)min((long long)SMALL_K, g.K - k0);
+        __syncthreads();
+        for (int k = tid; k < kn; k += 256) {
+            ka[k] = mode_off(g.kA, k0 + k);
+            kb[k] = mode_off(g.kB, k0 + k);
+        }
+        __syncthreads();
+        if (live) {
+#pragma unroll 4
+            for (int k = kl; k < kn; k += L) {
+                const double x = __ldg(pa + ka[k]);
+                acc0 = fma(x, __ldg(p0 + kb[k]), acc0);
+                acc1 = fma(x, __ldg(p1 + kb[k]), acc1);
+            }
+        }
+    }
+    for (int d = kfast ? 1 : 32 >> ll; d < (kfast ? L : 32); d <<= 1) {
+        acc0 += __shfl_xor_sync(0xffffffffu, acc0, d);
+        acc1 += __shfl_xor_sync(0xffffffffu, acc1, d);
+    }
+    if (!live || kl > 1 || (kl == 1 && n1 == n0)) return;
+    const long long om = mode_off(g.mC, m);
+    auto put = [&](long long n, double v) {
+        const long long off = om + mode_off(g.nC, n);
+        double r = g.alpha * v;
+        if (g.beta != 0.0) r = fma(g.beta, g.Cin[off], r);
+        g.C[off] = r;
+    };
+    // lanes 0 and 1 store one output each; a single lane stores both
+    if (kl == 0) put(n0, acc0);
+    if ((L > 1 ? kl == 1 : true) && n1 != n0) put(n1, acc1);
 }
 
 }  // namespace
@@ -411,9 +466,27 @@ void gett_f64(Ctx *ctx, const GettArgs &a, const char *name) {
     if (a.M <= 0 || a.N <= 0) return;
     if (gett_e64(ctx, a, name)) return;
     GroupProblem g = to_problem(a);
-    if (a.N > 8 && a.M * a.N <= (1LL << 16) && a.K <= 8192) {
+    // A warp per output up to 4096 outputs: its 32 lanes are needed to fill the GPU (us against the kernel
+    // with two outputs to a task: 9 x 9 x 9 6.0 / 7.7; 60 x 60 x 2000 32 / 38; 40 x 40 x 6000 92 / 93).
+    if (a.N > 8 && a.M * a.N <= 4096 && a.K <= 8192) {
         Ctx::Scope s(ctx, name);
-        gett_f64_small<<<(unsigned)((a.M * a.N * 32 + 255) / 256), 256, 0, ctx->stream>>>(g);
+        gett_f64_dots<<<(unsigned)((a.M * a.N * 32 + 255) / 256), 256, 0, ctx->stream>>>(g);
+        JUES_CHECK_CUDA(cudaGetLastError());
+        return;
+    }
+    // Two outputs to a task beyond that (100 x 100 x 100 16 -> 14 us; 25 x 400 x 25 13 -> 10; 25 x 400 x 400
+    // 33 / 33), and for few columns with a short K at any M, where the kernels below lose more to their tree
+    // sums and to rows that share no loads (us, M x N x K; A's K, then A's rows at unit stride: 15625 x 5 x 25
+    // 66 -> 19 and 34 -> 20; 250000 x 8 x 25 1240 -> 113 and 128 -> 113).  K = 128 is where the sides meet:
+    // 62500 x 8 x 128 160 / 155 and 250000 x 8 x 128 1260 / 1273 with A's rows at unit stride.
+    if ((a.N > 8 && a.M * a.N <= (1LL << 16) && a.K <= 8192) || (a.N > 1 && a.N <= 8 && a.K <= 128)) {
+        const long long tasks = a.M * ((a.N + 1) / 2);
+        int ll = 0;
+        while (ll < 5 && (tasks << ll) < 40000 && (2LL << ll) <= a.K) ++ll;
+        const long long blocks = ((tasks << ll) + 255) / 256;
+        JUES_REQUIRE(blocks < (1LL << 31), "GEMM too large for one launch");
+        Ctx::Scope s(ctx, name);
+        gett_f64_small<<<(unsigned)blocks, 256, 0, ctx->stream>>>(g, ll, a.kA.s0 == 1 && a.kA.d0 > 1);
         JUES_CHECK_CUDA(cudaGetLastError());
         return;
     }
