@@ -579,37 +579,40 @@ struct PackArgs {
     int kseg;          // row-maximum pass: K chunks per block
 };
 
-// biased exponent; 1 for subnormals, which mark a row the tensor cores do not take
-__device__ __forceinline__ int exp_of(double x) {
-    const unsigned hi = (unsigned)__double2hiint(x) & 0x7FFFFFFFu;
-    const int e = (int)(hi >> 20);
-    return e ? e : ((hi | (unsigned)__double2loint(x)) ? 1 : 0);
+// row maxima are taken over the magnitudes' high words, with a low bit set where the low word is not zero;
+// the biased exponent of such a maximum is 1 for subnormals, which mark a row the tensor cores do not take
+__device__ __forceinline__ unsigned mag_of(double x) {
+    return ((unsigned)__double2hiint(x) & 0x7FFFFFFFu) | min((unsigned)__double2loint(x), 1u);
 }
+__device__ __forceinline__ int exp_of(unsigned mag) { return mag >> 20 ? (int)(mag >> 20) : (mag ? 1 : 0); }
 
-// the PL digits of x in a row whose largest biased exponent is E, each + 256 (0..512)
+// x in units of 2^-(9 PL - 1) of its row's power of two, rounded with ties away from zero, with the offset
+// that makes its 9-bit fields the balanced digits + 256 (0..512).  base is shift_base() of the row
 template <int PL>
-__device__ __forceinline__ void digits(double x, int E, unsigned (&u)[PL]) {
+__device__ __forceinline__ int shift_base(int E) {
+    return (E ? E : 2000) + 9 * (E64_NP - PL);   // a row of zeros: everything is shifted out
+}
+template <int PL>
+__device__ __forceinline__ unsigned long long fixed_point(double x, int base) {
     const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
-    const int e = (int)(hi >> 20 & 0x7FFu);
-    // m 2^(9 PL - 54) >> (E - e), ties away from zero: ((m 2^10 >> sh) + 1) >> 1
-    constexpr int DROP = 9 * (E64_NP - PL);
-    const int sh = E - e + DROP;
+    // m 2^(9 PL - 54) >> (E - e): t = m 2^10 >> sh, then (t + 1) >> 1; below zero (-t) >> 1 = (~t + 1) >> 1
     const unsigned long long m = (((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << 10;
-    long long q = (long long)(((sh < 64 && e != 0 ? m >> sh : 0ull) + 1ull) >> 1);
-    if (hi >> 31) q = -q;
-    // + 256 in every digit: the sum is positive and its 9-bit fields are the balanced digits + 256
+    const long long neg = (long long)((int)hi >> 31);
+    const long long t = (long long)(m >> min(base - (int)(hi >> 20 & 0x7FFu), 63)) ^ neg;
     unsigned long long OFF = 0;
 #pragma unroll
     for (int p = 0; p < PL; ++p) OFF += 256ull << (9 * p);
-    const unsigned long long s = (unsigned long long)q + OFF;
-    u[0] = (unsigned)(s >> (9 * (PL - 1)));
-#pragma unroll
-    for (int p = 1; p < PL; ++p) u[p] = (unsigned)(s >> (9 * (PL - 1 - p))) & 511u;
+    return (unsigned long long)((t + 1) >> 1) + OFF;
 }
 
-// digit pair -> two FP16 integers: 0x6400 | u is 1024 + u
-__device__ __forceinline__ uint32_t digit_pair(unsigned u0, unsigned u1) {
-    const uint32_t w = u0 | (u1 << 16) | 0x64006400u, b = 0x65006500u;   // 1280
+// digits p of two numbers as a pair of FP16 integers: 0x6400 | u is 1024 + u (the first digit, up to 512,
+// takes ten bits of its own)
+template <int PL>
+__device__ __forceinline__ uint32_t digit_pair(unsigned long long s0, unsigned long long s1, int p) {
+    const int sh = 9 * (PL - 1 - p);
+    const uint32_t w = (__byte_perm((uint32_t)(s0 >> sh), (uint32_t)(s1 >> sh), 0x5410) &
+                        (p ? 0x01FF01FFu : 0x03FF03FFu)) | 0x64006400u;
+    const uint32_t b = 0x65006500u;   // 1280
     const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&w), *reinterpret_cast<const __half2 *>(&b));
     return *reinterpret_cast<const uint32_t *>(&h);
 }
@@ -617,12 +620,15 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned u0, unsigned u1) {
 template <int PL, int KW>
 struct PackSmem {
     static constexpr int PR = 2048 / KW;
-    uint32_t outp[PL][PR][KW / 2 + 2];   // pitch: the pair stores of both layouts free of bank conflicts
+    uint32_t outp[PL][PR][KW / 2 + 4];   // pitch: 16-byte pieces, the pair stores of both layouts free of conflicts
     long long roff[PR], koff[KW];
-    int rowE[PR];
+    unsigned rowE[PR];                   // the rows' exponents; LOCALMAX: their largest magnitudes
 };
 
-// LOCALMAX: the block sees whole rows (K <= KW) and writes their exponents; else they are read
+// LOCALMAX: the block sees whole rows (K <= KW) and writes their exponents; else they are read.  Integer issue
+// and the block's three phases bound it: 22 bytes an element (8 read, 14 written) at 3.6 to 4.1 TB/s of 6.7.
+// The digits stay one 64-bit number until two of them are put into an FP16 pair, padded K is skipped, and a
+// thread writes one 16-byte piece of each plane (500000 x 100: 345 -> 305 us; 6400^2: 352 -> 306).
 template <int PL, int KW, bool KFAST, bool LOCALMAX>
 __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, long long k0, PackSmem<PL, KW> &sm) {
     constexpr int PR = 2048 / KW, PAIRS = KW / 2;
@@ -636,8 +642,12 @@ __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, 
         sm.koff[tid - 64] = k < a.K ? mode_off(a.km, k) : -1;
     }
     __syncthreads();
-    auto row_of = [&](int i) { return KFAST ? tid / PAIRS + (256 / PAIRS) * i : tid & (PR - 1); };
-    auto pair_of = [&](int i) { return KFAST ? tid & (PAIRS - 1) : tid / PR + (256 / PR) * i; };
+    // KFAST: a warp's lanes along K; else eight rows x four pairs of K
+    constexpr int RB = PR / 8;
+    const int warp = tid >> 5;
+    auto row_of = [&](int i) { return KFAST ? tid / PAIRS + (256 / PAIRS) * i : (lane & 7) + 8 * (warp % RB); };
+    auto pair_of = [&](int i) { return KFAST ? tid & (PAIRS - 1) : (lane >> 3) + 4 * (warp / RB) + (32 / RB) * i; };
+    const int pairs = (int)min((long long)KW, a.Kpad - k0) / 2;
     double x[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
@@ -651,39 +661,38 @@ __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, 
             // a warp's lanes share each of its four rows
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int m = __reduce_max_sync(0xffffffffu, max(exp_of(x[i][0]), exp_of(x[i][1])));
+                const unsigned m = __reduce_max_sync(0xffffffffu, max(mag_of(x[i][0]), mag_of(x[i][1])));
                 if (lane == 0) atomicMax(&sm.rowE[row_of(i)], m);
             }
         } else {
-            int m = 0;
+            unsigned m = 0;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) m = max(m, max(exp_of(x[i][0]), exp_of(x[i][1])));
-            if (PR == 16) m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-            if (lane < PR) atomicMax(&sm.rowE[lane], m);
+            for (int i = 0; i < 4; ++i) m = max(m, max(mag_of(x[i][0]), mag_of(x[i][1])));
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
+            m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+            if (lane < 8) atomicMax(&sm.rowE[row_of(0)], m);
         }
         __syncthreads();
-        if (tid < PR) a.exps[r0 + tid] = sm.rowE[tid];
+        if (tid < PR) a.exps[r0 + tid] = exp_of(sm.rowE[tid]);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const int r = row_of(i), E = sm.rowE[r];
-        unsigned u0[PL], u1[PL];
-        digits<PL>(x[i][0], E, u0);
-        digits<PL>(x[i][1], E, u1);
+        const int r = row_of(i), c = pair_of(i);
+        if (c >= pairs) continue;
+        const int base = shift_base<PL>(LOCALMAX ? exp_of(sm.rowE[r]) : (int)sm.rowE[r]);
+        const unsigned long long s0 = fixed_point<PL>(x[i][0], base), s1 = fixed_point<PL>(x[i][1], base);
 #pragma unroll
-        for (int p = 0; p < PL; ++p) sm.outp[p][r][pair_of(i)] = digit_pair(u0[p], u1[p]);
+        for (int p = 0; p < PL; ++p) sm.outp[p][r][c] = digit_pair<PL>(s0, s1, p);
     }
     __syncthreads();
-    // PL planes x PR rows x KW / 4 pieces of 4 halves
+    // one piece of eight halves of each plane to a thread
+    const int seg = tid & (KW / 8 - 1), row = tid / (KW / 8);
+    if (4 * seg >= pairs) return;
+    __half *dst = a.dst + (size_t)(r0 + row) * a.Kpad + k0 + 8 * seg;
+    const size_t plane = (size_t)a.Rpad * a.Kpad;
 #pragma unroll
-    for (int j = 0; j < (PL * 512) / 256; ++j) {
-        const int idx = tid + 256 * j;
-        const int seg = idx & (KW / 4 - 1), row = (idx / (KW / 4)) & (PR - 1), plane = idx >> 9;
-        const long long k = k0 + 4 * seg;
-        if (k >= a.Kpad) continue;
-        *reinterpret_cast<uint2 *>(a.dst + ((size_t)plane * a.Rpad + (size_t)(r0 + row)) * a.Kpad + k) =
-            *reinterpret_cast<const uint2 *>(&sm.outp[plane][row][2 * seg]);
-    }
+    for (int p = 0; p < PL; ++p, dst += plane)
+        *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(&sm.outp[p][row][4 * seg]);
 }
 
 // both operands of a GEMM in one launch: blocks [0, a.blocks) pack a, the rest b
@@ -726,14 +735,14 @@ constexpr int PR = 16;
 template <bool KFAST>
 __device__ __forceinline__ void e64_rowmax_block(const PackArgs &a, long long r0, long long k0) {
     __shared__ long long roff[PR], koff[PK];
-    __shared__ int rowE[PR];
+    __shared__ unsigned rowE[PR];
     const int tid = threadIdx.x, lane = tid & 31;
     if (tid < PR) {
         const long long r = r0 + tid;
         roff[tid] = r < a.R ? mode_off(a.rm, a.row0 + r) : -1;
         rowE[tid] = 0;
     }
-    int m[4] = {0, 0, 0, 0};
+    unsigned m[4] = {0, 0, 0, 0};
     for (int c = 0; c < a.kseg && k0 + (long long)c * PK < a.K; ++c) {
         __syncthreads();
         if (tid >= 64 && tid < 64 + PK) {
@@ -744,11 +753,11 @@ __device__ __forceinline__ void e64_rowmax_block(const PackArgs &a, long long r0
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int row = KFAST ? (tid >> 6) + 4 * i : (tid & 15);
-            const int pair = KFAST ? (tid & 63) : (tid >> 4) + 16 * i;
+            const int k = KFAST ? (tid & 63) : (tid >> 4) + 16 * i;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const long long ro = roff[row], ko = koff[2 * pair + h];
-                if (ro >= 0 && ko >= 0) m[i] = max(m[i], exp_of(__ldg(a.src + ro + ko)));
+                const long long ro = roff[row], ko = koff[k + 64 * h];
+                if (ro >= 0 && ko >= 0) m[i] = max(m[i], mag_of(__ldg(a.src + ro + ko)));
             }
         }
     }
@@ -756,16 +765,16 @@ __device__ __forceinline__ void e64_rowmax_block(const PackArgs &a, long long r0
     if constexpr (KFAST) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const int x = __reduce_max_sync(0xffffffffu, m[i]);
+            const unsigned x = __reduce_max_sync(0xffffffffu, m[i]);
             if (lane == 0) atomicMax(&rowE[(tid >> 6) + 4 * i], x);
         }
     } else {
-        int x = max(max(m[0], m[1]), max(m[2], m[3]));
+        unsigned x = max(max(m[0], m[1]), max(m[2], m[3]));
         x = max(x, __shfl_xor_sync(0xffffffffu, x, 16));
         if (lane < 16) atomicMax(&rowE[lane], x);
     }
     __syncthreads();
-    if (tid < PR && r0 + tid < a.R && rowE[tid]) atomicMax(&a.exps[r0 + tid], rowE[tid]);
+    if (tid < PR && r0 + tid < a.R && rowE[tid]) atomicMax(&a.exps[r0 + tid], exp_of(rowE[tid]));
 }
 
 __global__ void __launch_bounds__(256) e64_rowmax_kernel(const __grid_constant__ PackArgs a,
@@ -942,7 +951,11 @@ bool keep_planes(bool is_const, long long K, size_t halves) {
     if (!is_const) return false;
     return K > 512 || halves * 2 <= (size_t(128) << 20);
 }
-constexpr size_t PANEL_HALVES = size_t(64) << 20;   // transient planes: panels of 128 MB
+// Transient planes go through panels of up to 1 GB, in halves down to 128 MB where memory is short.  Each
+// panel costs two launches and a last round of tiles, which outweighs keeping its planes in L2 (packs and GEMM
+// of 500000 x 16 x 100 with panels of 32, 64, 128, 256, 512 and 1024 MB: 880, 639, 560, 486, 461 and 439 us;
+// 20000 x 40 x 2000: 1098, 708, 566, 471, 439 and 416 us).  The results do not depend on it.
+constexpr size_t PANEL_MAX = size_t(512) << 20, PANEL_MIN = size_t(64) << 20;   // halves
 
 }  // namespace
 
@@ -958,55 +971,55 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     PackCache &pc = *ctx->pack;
     const size_t hA = (size_t)NP * Mall * Kpad, hB = (size_t)NP * Nall * Kpad;
     const bool keepA = keep_planes(a.a_const, a.K, hA), keepB = keep_planes(a.b_const, a.K, hB);
-    // rows per panel of A when its planes are transient
-    long long prow = Mall;
-    if (!keepA && hA > PANEL_HALVES)
-        prow = std::max<long long>(BM, (long long)(PANEL_HALVES / ((size_t)NP * Kpad)) / BM * BM);
-    if ((prow / PR) * ((Kpad + PK - 1) / PK) >= (1LL << 31)) return false;
-
     PackEntry *eA = keepA ? find_entry(pc, a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad) : nullptr;
     PackEntry *eB = keepB ? find_entry(pc, a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad) : nullptr;
     std::unique_ptr<PackEntry> newA, newB;
-    // K parts of a grid too small for the GPU (chunks of 64 K); exact whatever their number
     const int k16 = (int)((a.K + 15) / 16), chunks = (k16 + 3) / 4;
-    const long long panel_tiles = prow / BM * ntiles;
+    long long prow = Mall;   // rows per panel of A
     int ksplit = 1, kper = chunks;
-    {
+    longlong2 *part = nullptr;
+    for (size_t panel = PANEL_MAX;; panel /= 2) {
+        if (!keepA && hA > panel)
+            prow = std::max<long long>(BM, (long long)(panel / ((size_t)NP * Kpad)) / BM * BM);
+        if ((prow / PR) * ((Kpad + PK - 1) / PK) >= (1LL << 31)) return false;
+        // K parts of a grid too small for the GPU (chunks of 64 K); exact whatever their number
+        const long long panel_tiles = prow / BM * ntiles;
         // rounds of the 152 SMs times (chunks a part + about two for the tile's epilogue), plus the
         // parts' own pass
         auto time = [&](int ks) {
             const long long rounds = (panel_tiles * ks + 151) / 152;
             return (double)rounds * ((chunks + ks - 1) / ks + 2) + (ks > 1 ? 4.0 + 0.02 * (double)(panel_tiles * ks) / 152 : 0.0);
         };
+        ksplit = 1;
         for (int ks = 2; ks <= 64 && ks <= chunks; ++ks)
             if (panel_tiles * ks <= 152LL * 8 && time(ks) < 0.9 * time(ksplit)) ksplit = ks;
         kper = (chunks + ksplit - 1) / ksplit;
         ksplit = (chunks + kper - 1) / kper;
-    }
-    longlong2 *part = nullptr;
-    try {
-        Busy busy(pc);
-        if (keepA && !eA)
-            newA.reset(new PackEntry{a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad, NP, take_buffer(ctx, pc.free_planes, hA),
-                                     take_buffer(ctx, pc.free_exps, (size_t)Mall)});
-        if (keepB && !eB)
-            newB.reset(new PackEntry{a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad, NP, take_buffer(ctx, pc.free_planes, hB),
-                                     take_buffer(ctx, pc.free_exps, (size_t)Nall)});
-        if (!keepA) {
-            grow(ctx, pc.e64_planes[0], (size_t)NP * prow * Kpad);
-            grow(ctx, pc.e64_exps[0], (size_t)prow);
+        try {
+            Busy busy(pc);
+            if (keepA && !eA && !newA)
+                newA.reset(new PackEntry{a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad, NP, take_buffer(ctx, pc.free_planes, hA),
+                                         take_buffer(ctx, pc.free_exps, (size_t)Mall)});
+            if (keepB && !eB && !newB)
+                newB.reset(new PackEntry{a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad, NP, take_buffer(ctx, pc.free_planes, hB),
+                                         take_buffer(ctx, pc.free_exps, (size_t)Nall)});
+            if (!keepA) {
+                grow(ctx, pc.e64_planes[0], (size_t)NP * prow * Kpad);
+                grow(ctx, pc.e64_exps[0], (size_t)prow);
+            }
+            if (!keepB) {
+                grow(ctx, pc.e64_planes[1], hB);
+                grow(ctx, pc.e64_exps[1], (size_t)Nall);
+            }
+            grow(ctx, pc.e64_list, (size_t)(4 * mtiles_all * ntiles + 1));
+            if (ksplit > 1)
+                part = static_cast<longlong2 *>(
+                    ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN * sizeof(longlong2)));
+            break;
+        } catch (const Error &e) {
+            if (e.code != JUES_ENOMEM) throw;
+            if (keepA || hA <= PANEL_MIN || panel <= PANEL_MIN) return false;   // the FP64 pipe needs no planes
         }
-        if (!keepB) {
-            grow(ctx, pc.e64_planes[1], hB);
-            grow(ctx, pc.e64_exps[1], (size_t)Nall);
-        }
-        grow(ctx, pc.e64_list, (size_t)(4 * mtiles_all * ntiles + 1));
-        if (ksplit > 1)
-            part = static_cast<longlong2 *>(
-                ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN * sizeof(longlong2)));
-    } catch (const Error &e) {
-        if (e.code != JUES_ENOMEM) throw;
-        return false;   // the FP64 pipe needs no planes
     }
     allow_smem<NP, false>(ctx);
     // C = Cin + alpha AB into a dense column-major C: copy Cin over and add in place, off the FP64 pipe
