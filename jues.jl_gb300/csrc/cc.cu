@@ -38,8 +38,8 @@ double ccd_reference_flops(int o_, int v_) {
 
 namespace {
 
-// C = alpha * A.B + beta * Cin over the given modes.  With s->cache_operands set, split-precision
-// packs of every operand are kept until the operand's buffer is dropped (see ccd_sweep).
+// C = alpha * A.B + beta * Cin over the given modes.  With s->cache_operands set, the packs (split
+// planes or FP64 digits) of every operand are kept until the operand's buffer is dropped (see ccd_sweep).
 void G(CCState *s, int prec, const char *name, long long M, long long N, long long K, double alpha,
        const double *A, Mode mA, Mode kA, const double *B, Mode kB, Mode nB, double beta, double *C,
        Mode mC, Mode nC, const double *Cin = nullptr, bool a_const = false, bool b_const = false) {
@@ -117,6 +117,23 @@ static void ladder_stacks_l(CCState *s, const double *Tl, const char *name) {
 // ladder), O_s = 1/2 oovv folded over (a,b): two GEMMs of M = np, N = nq, K = np + nq in place
 // of one of M = o^2, N = v^2, K = o^2 + v^2, about a quarter of its work; X likewise halves.
 // ---------------------------------------------------------------------------------------
+// the folded FP64 arrays of both forms
+static void pair_arrays(CCState *s) {
+    if (s->invF.p) return;
+    Ctx *ctx = s->ctx;
+    const long long o = s->o, v = s->v, oo = o * o;
+    const long long np = o * (o + 1) / 2, nq = v * (v + 1) / 2;
+    // O_s[(i<=j), (a<=b)] = 1/2 (oovv[ij,ab] + s oovv[ij,ba])
+    s->Opm = DBuf<double>(ctx, (size_t)(2 * np * nq));
+    pair_fold(ctx, s->oovv.p, np, true, 0, 1, o, (int)v, oo, oo * v, 0.5, false, s->Opm.p);
+    s->Apm = DBuf<double>(ctx, (size_t)(2 * np * nq));
+    s->Lpm = DBuf<double>(ctx, (size_t)(2 * np * nq));
+    s->Cpm = DBuf<double>(ctx, (size_t)(2 * np * np));
+    s->Xpm = DBuf<double>(ctx, (size_t)(2 * oo * np));
+    s->invF = DBuf<double>(ctx, (size_t)(np * nq));
+    inv_denominators_folded(ctx, s->eps.p, (int)o, (int)v, s->invF.p);
+}
+
 static void pair_begin(CCState *s) {
     if (s->stackPB[0].buf.p) return;
     Ctx *ctx = s->ctx;
@@ -151,15 +168,7 @@ static void pair_begin(CCState *s) {
         }
         s->Ypm = DBuf<double>(ctx, (size_t)(2 * np * ov));
     }
-    // O_s[(i<=j), (a<=b)] = 1/2 (oovv[ij,ab] + s oovv[ij,ba])
-    s->Opm = DBuf<double>(ctx, (size_t)(2 * np * nq));
-    pair_fold(ctx, s->oovv.p, np, true, 0, 1, o, (int)v, oo, oo * v, 0.5, false, s->Opm.p);
-    s->Apm = DBuf<double>(ctx, (size_t)(2 * np * nq));
-    s->Lpm = DBuf<double>(ctx, (size_t)(2 * np * nq));
-    s->Cpm = DBuf<double>(ctx, (size_t)(2 * np * np));
-    s->Xpm = DBuf<double>(ctx, (size_t)(2 * oo * np));
-    s->invF = DBuf<double>(ctx, (size_t)(np * nq));
-    inv_denominators_folded(ctx, s->eps.p, (int)o, (int)v, s->invF.p);
+    pair_arrays(s);
     for (int k = 0; k < 2; ++k) s->stackPA[k].ensure(ctx, np, kp + kq, 2);
 }
 
@@ -193,6 +202,80 @@ static void pair_l(CCState *s, const char *name) {
         pack_stacked(ctx, s->stackPB[k], 0, s->Apm.p + k * np * nq, plain(np), plain(1), nq, np, 1.0);
         gett_tc_views(ctx, s->stackPA[k].view(0, kp + kq), s->stackPB[k].view(0, kp + kq), np, nq, 1.0, 1.0,
                       s->Lpm.p + k * np * nq, plain(1), plain(np), s->Opm.p + k * np * nq, name);
+    }
+}
+
+// ---------------------------------------------------------------------------------------
+// The same fold for CCD's FP64 sweeps, on FP64 arrays.  The particle ladder is their largest product
+// (400 x 6400 x 6400 for 20 occupied of 100 orbitals: 750 us a sweep; folded, 2 x 210 x 3240 x 3240: 300; X, both
+// ladders and the folds together 970 -> 510).
+// Taken from o^2 v^4 = 3.5e9 on, where the unfolded ladder's 170 us outweigh the folds' and the second sign's
+// launches, and only where the folded weights (half of vvvv's size) leave room for everything the solver may
+// still allocate: the DIIS vectors and the digit planes.  A split solve's few closing sweeps do not repay the
+// folding of vvvv (nbf = 90, two of them: 14.18 ms, folded 14.20) and stay unfolded.
+// ---------------------------------------------------------------------------------------
+static bool fold64_ready(CCState *s) {
+    if (s->fold64 >= 0) return s->fold64 == 1;
+    s->fold64 = 0;
+    Ctx *ctx = s->ctx;
+    const long long o = s->o, v = s->v, oo = o * o, vv = v * v;
+    const long long np = o * (o + 1) / 2, nq = v * (v + 1) / 2;
+    if (!t2_finalize_folds((int)o, (int)v) || (double)oo * (double)vv * (double)vv < 3.5e9) return false;
+    const double words = 2.0 * nq * nq + 2.0 * oo * nq + 7.0 * np * nq + 2.0 * np * np + 2.0 * oo * np;
+    const double later = 2.0 * std::max(1, s->opts.diis_size) * oo * vv + 4.0 * vv * vv + 16.0 * oo * vv;
+    const double need = 8.0 * (words + later);
+    if (ctx->mem_limit && (double)ctx->mem_used + need > (double)ctx->mem_limit) return false;
+    size_t avail = 0, total = 0;
+    JUES_CHECK_CUDA(cudaMemGetInfo(&avail, &total));
+    if (ctx->pool) {
+        uint64_t reserved = 0, used = 0;
+        JUES_CHECK_CUDA(cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
+        JUES_CHECK_CUDA(cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used));
+        avail += (size_t)(reserved - std::min(used, reserved));
+    }
+    if (need > (double)avail) return false;
+    try {
+        s->Bpm = DBuf<double>(ctx, (size_t)(2 * nq * nq));
+        s->Xw64 = DBuf<double>(ctx, (size_t)(2 * oo * nq));
+        pair_arrays(s);
+    } catch (const Error &e) {
+        if (e.code != JUES_ENOMEM) throw;
+        s->Bpm.reset();
+        s->Xw64.reset();
+        return false;
+    }
+    pair_fold(ctx, s->vvvv.p, nq, true, 0, 1, v, (int)v, vv, vv * v, 0.5, true, s->Bpm.p);
+    pair_fold(ctx, s->oovv.p, oo, false, oo, 1, 0, (int)v, oo, oo * v, 0.5, true, s->Xw64.p);
+    s->fold64 = 1;
+    return true;
+}
+
+static void fold64_x(CCState *s, const double *Tl, const char *name) {
+    Ctx *ctx = s->ctx;
+    const long long o = s->o, v = s->v, oo = o * o;
+    const long long np = o * (o + 1) / 2, nq = v * (v + 1) / 2;
+    for (int k = 0; k < 2; ++k) {
+        pack_cache_drop(ctx, s->Apm.p + k * np * nq);
+        pack_cache_drop(ctx, s->Cpm.p + k * np * np);
+    }
+    pair_fold(ctx, Tl, np, true, 0, 1, o, (int)v, oo, oo * v, 1.0, false, s->Apm.p);
+    for (int k = 0; k < 2; ++k)
+        G(s, JUES_PREC_FP64, name, oo, np, nq, 1.0, s->Xw64.p + k * oo * nq, plain(1), plain(oo),
+          s->Apm.p + k * np * nq, plain(np), plain(1), 0.0, s->Xpm.p + k * oo * np, plain(1), plain(oo));
+    pair_unfold(ctx, s->Xpm.p, oo * np, s->oooo.p, (int)o, oo, oo, 1, oo, 1, false, s->Wp.p);
+}
+
+static void fold64_l(CCState *s, const char *hh, const char *pp) {
+    Ctx *ctx = s->ctx;
+    const long long o = s->o, v = s->v, oo = o * o;
+    const long long np = o * (o + 1) / 2, nq = v * (v + 1) / 2;
+    pair_fold(ctx, s->Wp.p, np, true, 0, oo, oo * o, (int)o, 1, o, 0.5, true, s->Cpm.p);
+    for (int k = 0; k < 2; ++k) {
+        double *A = s->Apm.p + k * np * nq, *L = s->Lpm.p + k * np * nq;
+        G(s, JUES_PREC_FP64, hh, np, nq, np, 1.0, s->Cpm.p + k * np * np, plain(1), plain(np), A, plain(1),
+          plain(np), 1.0, L, plain(1), plain(np), s->Opm.p + k * np * nq);
+        G(s, JUES_PREC_FP64, pp, np, nq, nq, 1.0, A, plain(1), plain(np), s->Bpm.p + k * nq * nq, plain(nq),
+          plain(1), 1.0, L, plain(1), plain(np));
     }
 }
 
@@ -279,7 +362,7 @@ double ccd_sweep(CCState *s, int prec) {
     Ctx *ctx = s->ctx;
     const long long o = s->o, v = s->v, oo = o * o, ov = o * v, oov = oo * v, vv = v * v;
     const double *T = s->T.p;
-    // Every operand of this sweep is read-only once formed, so its split-precision packs can be
+    // Every operand of this sweep is read-only once formed, so its packs can be
     // shared between the GEMMs that use it; the buffers that change from sweep to sweep lose
     // their packs here (the integrals keep theirs).
     for (const double *p : {s->T.p, s->Tn.p, s->Wp.p, s->WJ.p, s->WK.p, s->W12.p, s->Fae.p, s->Fmi.p})
@@ -290,11 +373,14 @@ double ccd_sweep(CCState *s, int prec) {
     // In split precision the ladders and the ring contractions run on K-stacked packs (two planes).
     const bool stacked = prec == JUES_PREC_SPLIT || prec == JUES_PREC_SPLIT2;
     const bool pairl = stacked && t2_finalize_folds((int)o, (int)v);   // the folded ladders
+    const bool fold = prec == JUES_PREC_FP64 && s->precision == JUES_PREC_FP64 && fold64_ready(s);
     // W'[mn,ij] = oooo[mn,ij] + X[mn,ij], X = sum_ef oovv[mn,ef] T[ij,ef]  (Wmnij + the Wabef T-part)
     if (pairl)
         pair_x(s, T, "ccd_x");
     else if (stacked)
         ladder_stacks_x(s, T, "ccd_x");
+    else if (fold)
+        fold64_x(s, T, "ccd_x");
     else
         G(s, prec, "ccd_x", oo, oo, vv, 1.0, W, plain(1), plain(oo), T, plain(oo), plain(1), 1.0, s->Wp.p,
           plain(1), plain(oo), s->oooo.p);
@@ -308,6 +394,8 @@ double ccd_sweep(CCState *s, int prec) {
         pair_l(s, "ccd_pp_ladder");
     } else if (stacked) {
         ladder_stacks_l(s, T, "ccd_pp_ladder");
+    } else if (fold) {
+        fold64_l(s, "ccd_hh_ladder", "ccd_pp_ladder");
     } else {
         G(s, prec, "ccd_hh_ladder", oo, vv, oo, 1.0, s->Wp.p, plain(oo), plain(1), T, plain(1), plain(oo),
           1.0, s->L.p, plain(1), plain(oo), W);
@@ -365,12 +453,13 @@ double ccd_sweep(CCState *s, int prec) {
     s->cache_operands = false;
     // with DIIS the step norm comes from its error vector (the same |Tn - T|^2), so the
     // finalisation skips it: two of its five FP64 operations per element
-    const double *Lf = pairl ? s->Lpm.p : s->L.p, *Df = pairl ? s->invF.p : s->invD.p;
+    const bool folded = pairl || fold;
+    const double *Lf = folded ? s->Lpm.p : s->L.p, *Df = folded ? s->invF.p : s->invD.p;
     if (s->opts.diis) {
-        t2_finalize(ctx, Lf, Z, Df, (int)o, (int)v, nullptr, s->Tn.p, nullptr, nullptr, pairl);
+        t2_finalize(ctx, Lf, Z, Df, (int)o, (int)v, nullptr, s->Tn.p, nullptr, nullptr, folded);
         return -1.0;
     }
-    return t2_finalize(ctx, Lf, Z, Df, (int)o, (int)v, T, s->Tn.p, nullptr, nullptr, pairl);
+    return t2_finalize(ctx, Lf, Z, Df, (int)o, (int)v, T, s->Tn.p, nullptr, nullptr, folded);
 }
 
 // ---------------------------------------------------------------------------------------

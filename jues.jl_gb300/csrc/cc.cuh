@@ -55,6 +55,10 @@ struct CCState {
     DBuf<double> Apm, Cpm, Lpm, Opm, Xpm, Ypm;
     DBuf<double> invF;           // the folded 1/D, np x nq (the finalisation of the folded form)
     StackedPack stackPA[2], stackPB[2], stackPX[2], stackPY[2];
+    // CCD's FP64 sweeps in the same form: B_s and Xw_s as FP64 arrays, and whether the form is taken
+    // (-1: not decided yet)
+    DBuf<double> Bpm, Xw64;
+    int fold64 = -1;
     // CCSD, split precision: [2 Fme | -Fme] (one row, K = the ring blocks R1 and R23 of stackT),
     // so T1's T2.Fme terms are one GEMM on T2's ring packs
     StackedPack stackF;
@@ -67,7 +71,7 @@ struct CCState {
     double energy = 0.0, e_prev = 0.0;
     int iters = 0;
     int refine_left = -1;          // split precision: closing FP64 sweeps left (-1 = not started)
-    bool cache_operands = false;   // keep split packs of every sweep operand (CCD)
+    bool cache_operands = false;   // keep the packs of every sweep operand (CCD)
     bool converged = false;
     bool reference_df_wmbej = false;   // DF-RCCD.jl's index order in WmBeJ's last term
     // general (non-canonical) Fock matrix, AutoRCCSD.jl: off-diagonal occupied and virtual
