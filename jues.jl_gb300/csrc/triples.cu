@@ -41,8 +41,9 @@ __device__ __forceinline__ double pt_warp_sum(double x) {
 
 // Work item: one (i, j, k) and one triple of 8-wide virtual tiles A >= B >= C.  The six orderings of
 // the tile triple are loaded as 8^3 cubes (64-byte runs of W's unit-stride index; a gather of the six
-// orderings per thread read 32-byte sectors for 8 bytes), so W is read once, and each thread takes two
-// (a >= b >= c).  FP64 issue bounds it (about 70 operations a point).
+// orderings per thread read 32-byte sectors for 8 bytes), so W is read once.  FP64 issue bounds it (about 70
+// operations a point), so tile triples on a diagonal go through lists of their a >= b >= c, which fill the
+// warps: 288 of 512 points with two equal tiles, 120 with three (o = 12, v = 48: 1.28 -> 0.97 ms).
 __global__ void __launch_bounds__(PT_THREADS) pt_energy_kernel(const double *__restrict__ W,
                                                                const PtItem *__restrict__ items, int nitems,
                                                                const int *__restrict__ tiles, int ntiles,
@@ -56,6 +57,15 @@ __global__ void __launch_bounds__(PT_THREADS) pt_energy_kernel(const double *__r
     const int tid = threadIdx.x;
     const long long total = (long long)nitems * ntiles;
     double acc = 0.0;
+    // the points a + 8 b + 64 c of tile triples A = B > C, A > B = C and A = B = C
+    constexpr int PAIR = PT_T * (PT_T + 1) / 2, CUBE = PT_T * (PT_T + 1) * (PT_T + 2) / 6;
+    __shared__ unsigned short points[2 * PT_T * PAIR + CUBE];
+    for (int e = tid; e < PT_T * PT_T * PT_T; e += PT_THREADS) {
+        const int a = e & 7, b = (e >> 3) & 7, c = e >> 6;
+        if (a >= b) points[c * PAIR + a * (a + 1) / 2 + b] = (unsigned short)e;
+        if (b >= c) points[PT_T * PAIR + (b * (b + 1) / 2 + c) * PT_T + a] = (unsigned short)e;
+        if (a >= b && b >= c) points[2 * PT_T * PAIR + a * (a + 1) * (a + 2) / 6 + b * (b + 1) / 2 + c] = (unsigned short)e;
+    }
     for (long long w = blockIdx.x; w < total; w += gridDim.x) {
         const PtItem it = items[w / ntiles];
         const int pk = tiles[w % ntiles];
@@ -88,12 +98,14 @@ __global__ void __launch_bounds__(PT_THREADS) pt_energy_kernel(const double *__r
         }
         __syncthreads();
         const double dij = fo[it.i] + fo[it.j] + fo[it.k], num = 2.0 - (it.i == it.j) - (it.j == it.k);
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const int e = tid + 256 * n;
+        const bool ab = org[0] == org[1], bc = org[1] == org[2];
+        const int count = ab && bc ? CUBE : ab || bc ? PT_T * PAIR : PT_T * PT_T * PT_T;
+        const unsigned short *list = points + (ab && bc ? 2 * PT_T * PAIR : bc ? PT_T * PAIR : 0);
+        for (int q = tid; q < count; q += PT_THREADS) {
+            const int e = ab || bc ? list[q] : q;
             const int a = e & 7, b = (e >> 3) & 7, c = e >> 6;
             const int ga = org[0] + a, gb = org[1] + b, gc = org[2] + c;
-            if (ga >= v || gb > ga || gc > gb) continue;
+            if (ga >= v) continue;   // a >= b >= c by the lists
             const int loc[3] = {a, b, c};
             double wv[6], vv[6];
 #pragma unroll
