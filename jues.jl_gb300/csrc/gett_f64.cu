@@ -438,6 +438,88 @@ __global__ void __launch_bounds__(256) gett_f64_small(GroupProblem g, int ll, in
     if ((L > 1 ? kl == 1 : true) && n1 != n0) put(n1, acc1);
 }
 
+// Small GEMM in tiles: a block stages tm rows of A and tn columns of B in shared memory, K in chunks of kc,
+// its tm tn outputs (<= 128) times groups of threads over K.  Latency and the operands' uncoalesced loads bound
+// such a product: a thread per part of an output loads every element of A once per column from L1 (100^3:
+// 38 loads a thread; here 7).
+constexpr int TILE_NT = 512, TILE_WORDS = 5120, TILE_KC = 384, TILE_SIDE = 16;
+__global__ void __launch_bounds__(TILE_NT) gett_f64_tile(GroupProblem g, int tm, int tn, int kc, int kfastA, int kfastB) {
+    __shared__ double buf[TILE_WORDS];
+    __shared__ long long ka[TILE_KC], kb[TILE_KC], ra[TILE_SIDE], rb[TILE_SIDE], rc[TILE_SIDE], cc[TILE_SIDE];
+    const int tid = threadIdx.x;
+    const int mt = (int)((g.M + tm - 1) / tm);
+    const long long m0 = (long long)(blockIdx.x % mt) * tm, n0 = (long long)(blockIdx.x / mt) * tn;
+    // rows and columns past the edge read the last one and are not stored
+    if (tid < tm) {
+        const long long m = min(m0 + tid, g.M - 1);
+        ra[tid] = mode_off(g.mA, m);
+        rc[tid] = mode_off(g.mC, m);
+    } else if (tid >= 32 && tid < 32 + tn) {
+        const long long n = min(n0 + tid - 32, g.N - 1);
+        rb[tid - 32] = mode_off(g.nB, n);
+        cc[tid - 32] = mode_off(g.nC, n);
+    }
+    const int P = tm * tn, G = TILE_NT / P, kg = tid / P, q = tid - kg * P, r = q % tm, c = q / tm;
+    double acc = 0.0;
+    for (long long k0 = 0; k0 < g.K; k0 += kc) {
+        const int kn = (int)min((long long)kc, g.K - k0);
+        __syncthreads();
+        for (int k = tid; k < kn; k += TILE_NT) {
+            ka[k] = mode_off(g.kA, k0 + k);
+            kb[k] = mode_off(g.kB, k0 + k);
+        }
+        __syncthreads();
+        double *As = buf, *Bs = buf + tm * kn;   // [k][row], [k][column]
+        const int na = tm * kn, nb = tn * kn;
+#pragma unroll 4
+        for (int e = tid; e < na; e += TILE_NT) {
+            const int k = kfastA ? e % kn : e / tm, i = kfastA ? e / kn : e % tm;
+            As[k * tm + i] = __ldg(g.A + ra[i] + ka[k]);
+        }
+#pragma unroll 4
+        for (int e = tid; e < nb; e += TILE_NT) {
+            const int k = kfastB ? e % kn : e / tn, i = kfastB ? e / kn : e % tn;
+            Bs[k * tn + i] = __ldg(g.B + rb[i] + kb[k]);
+        }
+        __syncthreads();
+        if (kg < G) {
+#pragma unroll 4
+            for (int k = kg; k < kn; k += G) acc = fma(As[k * tm + r], Bs[k * tn + c], acc);
+        }
+    }
+    __syncthreads();
+    for (int w = G; w > 1;) {
+        const int h = (w + 1) / 2;
+        if (kg >= h && kg < w) buf[tid] = acc;
+        __syncthreads();
+        if (kg + h < w) acc += buf[tid + h * P];
+        w = h;
+    }
+    if (tid >= P || m0 + r >= g.M || n0 + c >= g.N) return;
+    const long long off = rc[r] + cc[c];
+    double v = g.alpha * acc;
+    if (g.beta != 0.0) v = fma(g.beta, g.Cin[off], v);
+    g.C[off] = v;
+}
+
+// tile of a small GEMM: the least rounds of 152 blocks times the clocks of one (FP64 issue, its loads, the
+// latency of a chunk of K)
+void small_tile(long long M, long long N, long long K, int &tm, int &tn, int &kc) {
+    constexpr int SIDES[] = {2, 4, 5, 6, 7, 8, 10, 12, 14, 16};
+    double best = 1e300;
+    for (int x : SIDES)
+        for (int y : SIDES) {
+            const int P = x * y, G = TILE_NT / P;
+            if (P > 128 || P < 16) continue;
+            const long long tiles = ((M + x - 1) / x) * ((N + y - 1) / y);
+            const int ch = (int)std::min<long long>(std::min(TILE_KC, TILE_WORDS / (x + y)), K);
+            const double clk = 0.47 * TILE_NT * (double)((K + G - 1) / G) + 0.75 * (x + y) * (double)K +
+                               1500.0 * (double)((K + ch - 1) / ch) + 1500.0;
+            const double t = (double)((tiles + 151) / 152) * clk;
+            if (t < best) { best = t; tm = x; tn = y; kc = ch; }
+        }
+}
+
 }  // namespace
 
 GroupProblem to_problem(const GettArgs &a) {
@@ -471,6 +553,19 @@ void gett_f64(Ctx *ctx, const GettArgs &a, const char *name) {
     if (a.N > 8 && a.M * a.N <= 4096 && a.K <= 8192) {
         Ctx::Scope s(ctx, name);
         gett_f64_dots<<<(unsigned)((a.M * a.N * 32 + 255) / 256), 256, 0, ctx->stream>>>(g);
+        JUES_CHECK_CUDA(cudaGetLastError());
+        return;
+    }
+    // Tiles beyond that up to 32768 outputs (us against two outputs to a task: 100 x 100 x 100 13.9 / 11.5; 25 x
+    // 400 x 400 30 / 26; 150 x 150 x 150 24.5 / 18.4; 25 x 400 x 25 10.7 / 9.1); more outputs fill the GPU either
+    // way (250 x 250 x 100 27 / 25, 250 x 250 x 16 11.5 / 14).
+    if (a.N > 8 && a.M * a.N <= (1LL << 15) && a.K >= 16 && a.K <= 8192) {
+        int tm = 8, tn = 8, kc = 1;
+        small_tile(a.M, a.N, a.K, tm, tn, kc);
+        const long long tiles = ((a.M + tm - 1) / tm) * ((a.N + tn - 1) / tn);
+        Ctx::Scope s(ctx, name);
+        gett_f64_tile<<<(unsigned)tiles, TILE_NT, 0, ctx->stream>>>(g, tm, tn, kc, a.kA.s0 == 1 && a.kA.d0 > 1,
+                                                                   a.kB.s0 == 1 && a.kB.d0 > 1);
         JUES_CHECK_CUDA(cudaGetLastError());
         return;
     }

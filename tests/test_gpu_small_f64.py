@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 # dispatch (N = 8 / 9, K = 128 / 129, 4096 and 65536 outputs, K = 8192), K shorter than the lanes
 SIZES = [(1, 2, 1), (33, 3, 7), (257, 5, 128), (257, 5, 129), (700, 8, 31), (70000, 2, 3),
          (9, 9, 1), (64, 64, 33), (64, 65, 33), (65, 64, 511), (65, 65, 512), (65, 65, 513),
-         (256, 256, 16), (256, 257, 16), (455, 9, 8192), (456, 9, 8192)]
+         (256, 256, 16), (256, 257, 16), (455, 9, 8192), (456, 9, 8192),
+         # staged tiles: K = 15 / 16, one and several chunks of K, 32768 outputs and one more row, thin tiles
+         (100, 100, 15), (100, 100, 16), (90, 50, 385), (25, 400, 400), (128, 256, 20), (129, 256, 20), (3640, 9, 17)]
 
 
 @pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
