@@ -520,9 +520,29 @@ __global__ void __launch_bounds__(THREADS, 1)
     }
 }
 
-// K parts: one block per tile adds the parts' 64-bit sums (exact, so their number does not matter)
+// K parts, many of them: adds each group of PART_FOLD parts into its first one, an element a thread.  Latency
+// bounds the parts' pass: a tile's block took 1 us for each of up to 64 parts (100 x 50 x 4000, two tiles: 66
+// us, with this launch 16).
+constexpr int PART_FOLD = 8;
+__global__ void __launch_bounds__(256) e64_fold_kernel(longlong2 *__restrict__ part, int ksplit, long long n) {
+    const long long i = blockIdx.x * 256LL + threadIdx.x;
+    const int s0 = blockIdx.y * PART_FOLD;
+    if (i >= n) return;
+    longlong2 x[PART_FOLD];
+#pragma unroll
+    for (int s = 0; s < PART_FOLD; ++s)
+        x[s] = s0 + s < ksplit ? part[(s0 + s) * n + i] : make_longlong2(0, 0);
+#pragma unroll
+    for (int s = 1; s < PART_FOLD; ++s) {
+        x[0].x += x[s].x;
+        x[0].y += x[s].y;
+    }
+    part[s0 * n + i] = x[0];
+}
+
+// K parts: one block per tile adds every step-th part's 64-bit sums (exact, so their number does not matter)
 // and finishes the tile as the main kernel does
-__global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
+__global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g, int step) {
     __shared__ long long coloff[BN];
     __shared__ int colE[BN];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -540,7 +560,8 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g) {
     long long hi[HB], lo[HB];
 #pragma unroll
     for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
-    for (int s = 0; s < g.ksplit; ++s) {
+#pragma unroll 2
+    for (int s = 0; s < g.ksplit; s += step) {
         const longlong2 *src = g.part + (((long long)s * tiles + tile) * BN + eighth * HB) * BM + quarter * 32 + lane;
 #pragma unroll
         for (int j = 0; j < HB; ++j) {
@@ -985,7 +1006,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         // K parts of a grid too small for the GPU (chunks of 64 K); exact whatever their number
         const long long panel_tiles = prow / BM * ntiles;
         // rounds of the 152 SMs times (chunks a part + about two for the tile's epilogue), plus the
-        // parts' own pass
+        // parts' own pass (its time in chunks of 1.45 us)
         auto time = [&](int ks) {
             const long long rounds = (panel_tiles * ks + 151) / 152;
             return (double)rounds * ((chunks + ks - 1) / ks + 2) + (ks > 1 ? 4.0 + 0.02 * (double)(panel_tiles * ks) / 152 : 0.0);
@@ -1071,7 +1092,16 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         if (ksplit > 1) {
             const std::string nm = std::string(name) + ".reduce";
             Ctx::Scope s(ctx, nm.c_str());
-            e64_parts_kernel<<<(unsigned)(g.mtiles * g.ntiles), DRAIN, 0, ctx->stream>>>(g);
+            const long long n = (long long)g.mtiles * g.ntiles * BM * BN;
+            int step = 1;
+            if (ksplit > PART_FOLD) {
+                step = PART_FOLD;
+                e64_fold_kernel<<<dim3((unsigned)(n / 256), (unsigned)((ksplit + step - 1) / step)), 256, 0,
+                                  ctx->stream>>>(part, ksplit, n);
+                ctx->count_launch();
+                JUES_CHECK_CUDA(cudaGetLastError());
+            }
+            e64_parts_kernel<<<(unsigned)(g.mtiles * g.ntiles), DRAIN, 0, ctx->stream>>>(g, step);
             JUES_CHECK_CUDA(cudaGetLastError());
         }
     }

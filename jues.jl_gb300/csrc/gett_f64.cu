@@ -191,29 +191,6 @@ __global__ void __launch_bounds__(NT) gett_f64_grouped(const GroupProblem *__res
     }
 }
 
-// the tiles the tensor-core form left out (gett_e64.cu): an entry is a 128 x 16 tile of one problem.  The
-// list is nearly always empty; a short one is spread as 16 x 16 tiles (one block walking a 64 x 16 tile's K of
-// 2500 takes a millisecond), a long one as 64 x 16.
-__global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(const GroupProblem one,
-                                                            const GroupProblem *__restrict__ probs,
-                                                            const int *__restrict__ list) {
-    __shared__ TileSmem<64, 16> sm;
-    const int n = list[0];
-    const int sub = n <= 512 ? 8 : 2, rows = 128 / sub;
-    for (int x = blockIdx.x; x < n * sub; x += gridDim.x) {
-        const int e = x / sub;
-        GroupProblem g = probs ? probs[list[1 + 2 * e]] : one;
-        const long long t = list[2 + 2 * e], mt128 = (g.M + 127) / 128;
-        const long long mt = sub * (t % mt128) + x % sub;
-        g.mtiles = (g.M + rows - 1) / rows;
-        if (mt >= g.mtiles) continue;
-        if (sub == 8)
-            gett_tile<16, 16>(g, mt + g.mtiles * (t / mt128), reinterpret_cast<TileSmem<16, 16> &>(sm), 0, g.K);
-        else
-            gett_tile<64, 16>(g, mt + g.mtiles * (t / mt128), sm, 0, g.K);
-    }
-}
-
 // Offset of a mode index that advances by a fixed step: the division-free successor of
 // mode_off (the carries replace the divisions), so a K loop costs a few integer adds per
 // element instead of 32- or 64-bit divisions.
@@ -256,6 +233,66 @@ struct ModeIter {
         }
     }
 };
+
+// The tiles the tensor-core form left out (gett_e64.cu): an entry is a 128 x 16 tile of one problem.  The
+// list is nearly always empty; a long one runs as 64 x 16 tiles, a shorter one as 16 x 16, and one of up to 16
+// entries with a warp to two outputs: FP64 issue bounds a block's 16 x 16 K products, and eight such blocks leave
+// the other SMs idle (K = 3240, one, four and sixteen entries: 455, 450 and 467 us as 16 x 16, now 82, 147 and 299).
+__global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(const GroupProblem one,
+                                                            const GroupProblem *__restrict__ probs,
+                                                            const int *__restrict__ list) {
+    __shared__ TileSmem<64, 16> sm;
+    const int n = list[0];
+    if (n <= 16) {
+        const int lane = threadIdx.x & 31;
+        for (int w = (blockIdx.x * NT + threadIdx.x) >> 5; w < n * 1024; w += gridDim.x * (NT / 32)) {
+            const int e = w >> 10;
+            const GroupProblem &g = probs ? probs[list[1 + 2 * e]] : one;
+            const long long t = list[2 + 2 * e], mt128 = (g.M + 127) / 128;
+            const long long m = t % mt128 * 128 + (w & 127), n0 = t / mt128 * 16 + 2 * (w >> 7 & 7);
+            if (m >= g.M || n0 >= g.N) continue;
+            const long long n1 = n0 + 1 < g.N ? n0 + 1 : n0;
+            const double *pa = g.A + mode_off(g.mA, m);
+            const double *p0 = g.B + mode_off(g.nB, n0), *p1 = g.B + mode_off(g.nB, n1);
+            ModeIter ia, ib;
+            ia.init(g.kA, lane);
+            ib.init(g.kB, lane);
+            double acc0 = 0.0, acc1 = 0.0;
+#pragma unroll 4
+            for (long long k = lane; k < g.K; k += 32) {
+                const double x = __ldg(pa + ia.off);
+                acc0 = fma(x, __ldg(p0 + ib.off), acc0);
+                acc1 = fma(x, __ldg(p1 + ib.off), acc1);
+                ia.step(g.kA, 32);
+                ib.step(g.kB, 32);
+            }
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                acc0 += __shfl_xor_sync(0xffffffffu, acc0, d);
+                acc1 += __shfl_xor_sync(0xffffffffu, acc1, d);
+            }
+            if (lane > 1 || (lane == 1 && n1 == n0)) continue;
+            const long long off = mode_off(g.mC, m) + mode_off(g.nC, lane ? n1 : n0);
+            double v = g.alpha * (lane ? acc1 : acc0);
+            if (g.beta != 0.0) v = fma(g.beta, g.Cin[off], v);
+            g.C[off] = v;
+        }
+        return;
+    }
+    const int sub = n <= 512 ? 8 : 2, rows = 128 / sub;
+    for (int x = blockIdx.x; x < n * sub; x += gridDim.x) {
+        const int e = x / sub;
+        GroupProblem g = probs ? probs[list[1 + 2 * e]] : one;
+        const long long t = list[2 + 2 * e], mt128 = (g.M + 127) / 128;
+        const long long mt = sub * (t % mt128) + x % sub;
+        g.mtiles = (g.M + rows - 1) / rows;
+        if (mt >= g.mtiles) continue;
+        if (sub == 8)
+            gett_tile<16, 16>(g, mt + g.mtiles * (t / mt128), reinterpret_cast<TileSmem<16, 16> &>(sm), 0, g.K);
+        else
+            gett_tile<64, 16>(g, mt + g.mtiles * (t / mt128), sm, 0, g.K);
+    }
+}
 
 // skinny GEMM (N <= NN <= 8): one warp per output row, lanes split K
 template <int NN>
