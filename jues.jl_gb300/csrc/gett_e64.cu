@@ -19,7 +19,7 @@
 // (K = 100) to 8.4e-16 (640^3).
 //
 // Speed (packs included): 6400^3 10.6 ms = 49 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.25 against
-// 8.1 ms, 500000 x 100 x 100 0.93 against 11.8 ms.  At long K the MMAs paced by shared memory take about
+// 8.1 ms, 500000 x 100 x 100 0.77 against 11.8 ms.  At long K the MMAs paced by shared memory take about
 // four fifths of the time; at K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about
 // 8000 clocks a tile) does.
 //
