@@ -89,6 +89,13 @@ class WorkerPool {
 
 constexpr size_t kSlot = size_t(64) << 20;
 constexpr int kSlots = 3;
+// Page-locking a slot takes about 15 ms, and results alone need two buffers in turn: until an upload has made the
+// slots, results go through a pair of 16 MB (RCCD nbf=200 from device integrals, 328 MB of amplitudes, a context's
+// first call: 190 ms through the slots, 173 here).  Results of 512 MB and more keep the
+// slots: the MP2 gradient at nbf=120, 1.66 GB, takes 46.8 ms a call with them and 48.7 with the pair.
+constexpr size_t kSmall = size_t(16) << 20;
+constexpr int kSmalls = 2;
+constexpr size_t kLarge = size_t(512) << 20;
 constexpr size_t kTask = size_t(1) << 20;   // host copy granule
 
 // one slot's worth of ranges: stage[i] in the slot <-> host[i] / dev[i]
@@ -103,15 +110,15 @@ struct Fill {
     size_t used = 0;
 };
 
-// cut the ranges into slot-sized fills, in order
-std::vector<Fill> plan_fills(const std::vector<HostSeg> &segs) {
+// cut the ranges into fills of at most cap bytes, in order
+std::vector<Fill> plan_fills(const std::vector<HostSeg> &segs, size_t cap) {
     std::vector<Fill> fills(1);
     for (const HostSeg &s : segs) {
         size_t off = 0;
         while (off < s.bytes) {
-            if (fills.back().used == kSlot) fills.emplace_back();
+            if (fills.back().used == cap) fills.emplace_back();
             Fill &f = fills.back();
-            const size_t take = std::min(s.bytes - off, kSlot - f.used);
+            const size_t take = std::min(s.bytes - off, cap - f.used);
             f.pcs.push_back({f.used, static_cast<const char *>(s.src) + off, static_cast<char *>(s.dst) + off, take});
             f.used += take;
             off += take;
@@ -124,7 +131,8 @@ std::vector<Fill> plan_fills(const std::vector<HostSeg> &segs) {
 }  // namespace
 
 struct Staging {
-    char *host[kSlots] = {};   // kSlot bytes each, page-locked when first used (about 15 ms)
+    char *host[kSlots] = {};     // kSlot bytes each, page-locked when first used
+    char *small[kSmalls] = {};   // kSmall bytes each, likewise
     cudaEvent_t done[kSlots] = {};
     bool busy[kSlots] = {};
     WorkerPool *pool = nullptr;
@@ -140,18 +148,19 @@ static Staging *staging_of(Ctx *ctx) {
     return st;
 }
 
-static char *slot_of(Staging *st, int k) {
-    if (!st->host[k])
-        JUES_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&st->host[k]), kSlot, cudaHostAllocDefault));
-    return st->host[k];
+static char *locked(char *&p, size_t bytes) {
+    if (!p) JUES_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p), bytes, cudaHostAllocDefault));
+    return p;
 }
+static char *slot_of(Staging *st, int k) { return locked(st->host[k], kSlot); }
 
-// host side of one fill: copy the pieces' bytes between the slot and the caller's arrays in 1 MB
-// tasks over the workers (to_slot: caller -> slot)
+// host side of one fill: copy the pieces' bytes between the slot and the caller's arrays in tasks of
+// 1 MB (256 KB in a fill of 16 MB or less) over the workers (to_slot: caller -> slot)
 static void host_copy(Staging *st, const Fill &f, char *slot, bool to_slot) {
-    const int ntask = (int)((f.used + kTask - 1) / kTask);
+    const size_t task = f.used > kSmall ? kTask : kTask / 4;
+    const int ntask = (int)((f.used + task - 1) / task);
     st->pool->parallel_for(ntask, [&](int k) {
-        const size_t lo = (size_t)k * kTask, hi = std::min(f.used, lo + kTask);
+        const size_t lo = (size_t)k * task, hi = std::min(f.used, lo + task);
         // pieces are in slot order: start at the last one beginning at or before lo
         auto it = std::upper_bound(f.pcs.begin(), f.pcs.end(), lo,
                                    [](size_t x, const Fill::Piece &p) { return x < p.at; });
@@ -167,7 +176,7 @@ static void host_copy(Staging *st, const Fill &f, char *slot, bool to_slot) {
 }
 
 void staged_h2d(Ctx *ctx, const std::vector<HostSeg> &segs) {
-    const std::vector<Fill> fills = plan_fills(segs);
+    const std::vector<Fill> fills = plan_fills(segs, kSlot);
     if (fills.empty()) return;
     Staging *st = staging_of(ctx);
     for (size_t i = 0; i < fills.size(); ++i) {
@@ -183,14 +192,19 @@ void staged_h2d(Ctx *ctx, const std::vector<HostSeg> &segs) {
 }
 
 void staged_d2h(Ctx *ctx, const std::vector<HostSeg> &segs) {
-    const std::vector<Fill> fills = plan_fills(segs);
-    if (fills.empty()) return;
     Staging *st = staging_of(ctx);
-    // the link fills slot i while the host empties slot i - 1
+    size_t bytes = 0;
+    for (const HostSeg &s : segs) bytes += s.bytes;
+    const bool small = !st->host[0] && bytes < kLarge;   // slot 0 is the first that an upload takes
+    const std::vector<Fill> fills = plan_fills(segs, small ? kSmall : kSlot);
+    if (fills.empty()) return;
+    const int slots = small ? kSmalls : kSlots;
+    auto slot_at = [&](int k) { return small ? locked(st->small[k], kSmall) : slot_of(st, k); };
+    // the link fills slot i + 1 while the host empties slot i
     auto issue = [&](size_t i) {
-        const int k = (int)(i % kSlots);
+        const int k = (int)(i % slots);
         if (st->busy[k]) JUES_CHECK_CUDA(cudaEventSynchronize(st->done[k]));
-        char *slot = slot_of(st, k);
+        char *slot = slot_at(k);
         for (const Fill::Piece &p : fills[i].pcs)
             JUES_CHECK_CUDA(cudaMemcpyAsync(slot + p.at, p.src, p.bytes, cudaMemcpyDeviceToHost, ctx->stream));
         JUES_CHECK_CUDA(cudaEventRecord(st->done[k], ctx->stream));
@@ -199,9 +213,9 @@ void staged_d2h(Ctx *ctx, const std::vector<HostSeg> &segs) {
     issue(0);
     for (size_t i = 0; i < fills.size(); ++i) {
         if (i + 1 < fills.size()) issue(i + 1);
-        const int k = (int)(i % kSlots);
+        const int k = (int)(i % slots);
         JUES_CHECK_CUDA(cudaEventSynchronize(st->done[k]));
-        host_copy(st, fills[i], slot_of(st, k), false);
+        host_copy(st, fills[i], slot_at(k), false);
     }
 }
 
@@ -235,6 +249,8 @@ void staging_destroy(Staging *st) {
             cudaEventDestroy(st->done[k]);
         }
     for (char *h : st->host)
+        if (h) cudaFreeHost(h);
+    for (char *h : st->small)
         if (h) cudaFreeHost(h);
     delete st->pool;
     delete st;
