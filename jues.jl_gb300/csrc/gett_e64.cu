@@ -12,29 +12,32 @@
 // for j <= 3, so the FP32 accumulators hold these sums exactly whatever the data; S_4, S_5 and S_6
 // (2^-36 to 2^-54 of the product) could pass 2^24 only for a chunk of equal-signed maximal digits and
 // then lose one unit in 2^24.  After each chunk the sums are added into 64-bit integers (S_0..S_2 and
-// S_3..S_6 combined), so the accumulation over K is exact: the whole error is the rounding of the
-// inputs to 2^-63 of their row's maximum, the dropped products and one final rounding, below
-// 2^-61 |a|_2 |b|_2 + 2^-53 |a.b|, where an FP64 FMA loop also rounds each of its K sums.  Against exact
-// products, relative Frobenius error for normal entries: 4.7e-17 at every size, the FMA kernels 1.3e-16
-// (K = 100) to 8.4e-16 (640^3).
+// S_3..S_6 combined), so the accumulation over K is exact.  Cutting operands into slices whose products are
+// exact is the method of Ozaki, Ogita, Oishi and Rump (Numer. Algorithms 59, 2012).
 //
-// Speed (packs included): 6400^3 10.6 ms = 49 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.25 against
-// 8.1 ms, 500000 x 100 x 100 0.77 against 11.8 ms.  At long K the MMAs paced by shared memory take about
-// four fifths of the time; at K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about
-// 8000 clocks a tile) does.
+// Error: rounding the inputs to 2^-63 of their row's maximum and the six products of j = 7 left out are at most
+// 8.1 x 2^-63 max|a| max|b| for each k whose a_k and b_k are both nonzero, and the result is rounded once.  That is far
+// below an FMA loop's K 2^-53 sum |a_k b_k| unless the large elements of a row meet only small ones (or zeros) of
+// the column.  So every element is judged by the magnitude it is made of: a further plane holds |x| cut to E5M2,
+// whose products, a narrow 8-bit MMA for every 32 K values, sum to P <= sum |a_k b_k|; an element is taken only
+// where P >= 2^-7 max|a| max|b| (and 1/16 more), which bounds its error by K 2^-53 sum |a_k b_k| + 2^-53 |a.b|
+// whatever the operands are.  A half tile (16 columns) with an element below that, or with a
+// row or column that holds a non-finite, subnormal-only or extreme (beyond 2^+-400) maximum, is not stored but
+// listed, and gett_f64_tiles recomputes the listed ones on the FP64 pipe, with the same special values as ever.
+// Cancellation alone lists nothing.  Against exact products, relative Frobenius error for normal entries:
+// 4.7e-17 at every size, the FMA kernels 1.3e-16 (K = 100) to 8.4e-16 (640^3).
 //
-// That bound is relative to |a|_2 |b|_2, not to sum |a_k b_k|: rows whose large elements meet only
-// small ones of the other side (an operand graded along K) would lose relative accuracy that an
-// FMA loop keeps.  So every output tile is checked before it is stored: a tile with a row or a
-// column whose results all fall below 2^-5 / sqrt(K) of its bound, or with a row that holds a non-finite,
-// subnormal-only or extreme (beyond 2^+-400) maximum, is not stored but listed (by halves), and
-// gett_f64_tiles recomputes the listed tiles on the FP64 pipe, with the same special values as ever.
+// Speed (packs included): 6400^3 11.2 ms = 47 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.26 against
+// 8.1 ms, 500000 x 100 x 100 0.80 against 11.8 ms.  The magnitudes cost 7 % of that at long K (as a second
+// FP16 plane they cost 15 %).  At K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about 8000
+// clocks a tile) bounds it.
 //
-// The tile is 128 x 32: TMEM holds two buffers of 7 x 32 FP32 columns, so the drain of one chunk
-// overlaps the MMAs of the next.  With N = 32 per plane an instruction reads 4 KB of A and up to 7
-// KB of B from shared memory for 16 to 112 clocks of MMA, so a K = 16 step takes about 496 clocks
-// (448 at the dense rate); a wider tile would need TMEM that is not there.  A's planes arrive one by
-// one (64 K values x 128 rows, 16 KB, 128-byte swizzle) in a ring of ten, B's seven together.
+// The tile is 128 x 32: TMEM holds two buffers of 8 x 32 FP32 columns (seven digit sums and the magnitudes), so
+// the drain of one chunk overlaps the MMAs of the next; a wider tile would need TMEM that is not there.  At long K
+// shared memory paces: a chunk's MMAs read 240 KB of it (with N = 32 per plane an instruction takes 4 KB of A
+// and 1 to 7 KB of B for 16 to 112 clocks) and TMA writes 154 KB, 3070 clocks at 128 bytes a clock (measured 3040),
+// against 1820 clocks of MMA at the dense rate.  A's planes arrive one by one (64 K values x 128 rows, 16 KB,
+// 128-byte swizzle; the magnitudes 8 KB, 64-byte swizzle) in a ring of nine, B's together.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -55,11 +58,17 @@ namespace {
 constexpr int NP = E64_NP;            // digit planes of the FP64 form (the kernels take 3 too)
 constexpr int BM = 128, BN = 32;      // output tile
 constexpr int CK = 64;                // K per chunk: 128 bytes of FP16, one swizzle row
-constexpr int SLOTS = 10;             // ring of A planes
+constexpr int SLOTS = 9;              // ring of A planes
 constexpr int A_BYTES = BM * CK * 2;  // one A plane, 16 KB
-constexpr int b_bytes(int np) { return np * BN * CK * 2; }   // all of B: 28 KB for seven planes
+constexpr int b_bytes(int np) { return np * BN * CK * 2 + BN * CK; }   // all of B: 30 KB for seven digits
+// an operand's planes in FP16 words: np digits for each of its rows x kpad elements, then the magnitudes, bytes in
+// rows of whole 32-byte sectors
+constexpr long long mag_pitch(long long kpad) { return (kpad + 31) / 32 * 32; }
+constexpr size_t plane_halves(int np, long long rows, long long kpad) {
+    return (size_t)np * rows * kpad + (size_t)rows * mag_pitch(kpad) / 2;
+}
 constexpr int ring_bytes(int np) { return SLOTS * A_BYTES + 2 * b_bytes(np); }
-constexpr uint32_t TMEM_COLS = 512;   // two chunk buffers of np x 32 columns
+constexpr uint32_t TMEM_COLS = 512;   // two chunk buffers of (np + 1) x 32 columns
 // sixteen drain warps: the drain and the epilogue are chains of short integer operations, and with
 // two warps per scheduler (eight in all) they issued one instruction in three clocks
 constexpr int THREADS = 576, DRAIN = 512;
@@ -74,11 +83,16 @@ struct Tables {
 };
 constexpr int smem_bytes(int np) { return ring_bytes(np) + BAR_BYTES + ITEMS * 16 + 6 * (int)sizeof(Tables) + 1024; }
 constexpr int E_MIN = 1023 - 400, E_MAX = 1023 + 400;   // biased exponents of regular row maxima
+// least sum of magnitudes of a stored result: 17/16 2^-7 of max|a| max|b|, the codes' products being in units of 2^-30
+constexpr float MAG_MIN = 8912896.0f;
 
 // instruction descriptor: FP32 accumulate, FP16 A and B, both K-major, M = 128, N = n
 __host__ __device__ constexpr uint32_t idesc(int n) {
     return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
+
+// the magnitudes': E5M2 A and B, N = 32
+__host__ __device__ constexpr uint32_t idesc_mag() { return idesc(BN) | (1u << 7) | (1u << 10); }
 
 __host__ __device__ __forceinline__ long long e64_items(const E64Args &g) {
     return (long long)g.mtiles * g.ntiles * g.ksplit;
@@ -110,47 +124,31 @@ __device__ __forceinline__ long long e64_join(long long hi, long long lo, int &u
 }
 
 // One thread's row of a tile (8 columns): its sums become FP64 values (hi[j] is overwritten with
-// the bits), and the checks above run.  ea: the row's biased exponent (0 outside M or a zero row);
-// colE: the columns' (shared memory).  V's exponent before scaling compares a result with 2^-weak of its
-// bound 2^(ea + eb) whatever the exponents are.  Returns whether this thread saw a reason to leave the
-// tile to the FP64 pipe.
+// the bits), and the checks above run.  mag: the elements' sums of magnitudes; ea: the row's biased exponent (0
+// outside M or a zero row); colE: the columns' (shared memory).  Returns whether this thread saw a reason to
+// leave the tile to the FP64 pipe.
 template <bool LOW, class E>
-__device__ __forceinline__ bool e64_finish(const E64Out &g, long long (&hi)[HB], const long long (&lo)[HB], int ea,
-                                           const E *colE) {
+__device__ __forceinline__ bool e64_finish(const E64Out &g, long long (&hi)[HB], const long long (&lo)[HB],
+                                           const float (&mag)[HB], int ea, const E *colE) {
     const bool live = ea != 0;
     bool bad = live && (ea < E_MIN || ea > E_MAX);
-    int eb[HB];
-    unsigned cols = 0;   // columns that are not zero
-#pragma unroll
-    for (int j = 0; j < HB; ++j) {
-        eb[j] = colE[j];
-        if (eb[j]) cols |= 1u << j;
-        bad |= eb[j] != 0 && (unsigned)(eb[j] - E_MIN) > (unsigned)(E_MAX - E_MIN);
-    }
-    // one or two results of a row (column) may cancel further by chance, so they get more room
-    const int few = min(__popc(cols), __popc(__ballot_sync(0xffffffffu, live)));
-    // |V 2^-36| >= 2^(34 - weak) in the exponent field
-    const unsigned thr = (unsigned)(1023 + 34 - g.weak - (few >= 3 ? 0 : (few == 2 ? 4 : 8))) << 20;
     const int neg = g.alpha_neg ? (int)0x80000000 : 0;
     const int sc0 = ea - 2 * 1022 - 70 + 36 + g.alpha_k;
-    unsigned strong = 0;
 #pragma unroll
     for (int j = 0; j < HB; ++j) {
+        const int eb = colE[j];
+        bad |= eb != 0 && ((unsigned)(eb - E_MIN) > (unsigned)(E_MAX - E_MIN) || (live && mag[j] < MAG_MIN));
         int up = 0;
         const double v = __ll2double_rn(LOW ? e64_join(hi[j], lo[j], up) : hi[j]);   // 0 for a zero row or column
         const int vh = __double2hiint(v);
-        const unsigned mag = (unsigned)vh & 0x7FFFFFFFu;
-        if (mag >= thr + (up << 20)) strong |= 1u << j;
-        const int sc = mag ? (sc0 + eb[j] - up) << 20 : 0;
+        const int sc = (vh & 0x7FFFFFFF) ? (sc0 + eb - up) << 20 : 0;
         hi[j] = __double_as_longlong(__hiloint2double((vh + sc) ^ neg, __double2loint(v)));
     }
     if (!g.alpha_pow2) {
 #pragma unroll
         for (int j = 0; j < HB; ++j) hi[j] = __double_as_longlong(g.alpha * __longlong_as_double(hi[j]));
     }
-    if (live) bad |= cols && !(strong & cols);
-    const unsigned any = __reduce_or_sync(0xffffffffu, live ? strong | 1u << 31 : 0u);
-    return bad || (any && (cols & ~any));
+    return bad;
 }
 
 // store one thread's row through the output modes (co: column offsets, -1 past N)
@@ -213,13 +211,14 @@ __device__ __forceinline__ void add_sum(long long &acc, uint32_t x) {
 // quarter, 8 columns each).  Every wait is bounded; on expiry the CTA raises FLAG_TIMEOUT, skips its
 // stores, waits for its own copies, frees TMEM and returns.
 // GROUPED: the launch covers ngp problems (gp, in order of item0) whose operand rows lie in shared planes;
-// item w belongs to the last problem with item0 <= w.  PL planes: 7 (FP64), or 3 = 27 bits with the six
-// products of j < 3 (split precision).
+// item w belongs to the last problem with item0 <= w.  PL digit planes: 7 (FP64), or 3 = 27 bits with the six
+// products of j < 3 (split precision); plane PL holds the magnitudes.
 template <int PL, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
     gett_e64_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                    const __grid_constant__ CUtensorMap magA, const __grid_constant__ CUtensorMap magB,
                     const __grid_constant__ E64Args g0, const E64Args *__restrict__ gp, int ngp, int nitems) {
-    constexpr int B_BYTES = b_bytes(PL), RING_BYTES = ring_bytes(PL), BUF_COLS = PL * BN;
+    constexpr int B_BYTES = b_bytes(PL), RING_BYTES = ring_bytes(PL), BUF_COLS = (PL + 1) * BN;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *ringB = smem + SLOTS * A_BYTES;
@@ -316,11 +315,12 @@ __global__ void __launch_bounds__(THREADS, 1)
                     if (c > c0 && !wait(&bempty[b], ((gc >> 1) & 1u) ^ 1u)) break;
                     mbar_expect_tx(&bfull[b], B_BYTES);
                     tma_load_3d(ringB + b * B_BYTES, &mapB, &bfull[b], c * CK, n0, 0);
-                    for (int p = 0; p < PL; ++p, ++it) {
+                    tma_load_3d(ringB + b * B_BYTES + PL * BN * CK * 2, &magB, &bfull[b], c * CK, n0, 0);
+                    for (int p = 0; p <= PL; ++p, ++it) {
                         const unsigned s = it % SLOTS;
                         if (!wait(&aempty[s], ((it / SLOTS) & 1u) ^ 1u)) break;
-                        mbar_expect_tx(&afull[s], A_BYTES);
-                        tma_load_3d(smem + s * A_BYTES, &mapA, &afull[s], c * CK, m0, p);
+                        mbar_expect_tx(&afull[s], p < PL ? A_BYTES : BM * CK);
+                        tma_load_3d(smem + s * A_BYTES, p < PL ? &mapA : &magA, &afull[s], c * CK, m0, p < PL ? p : 0);
                     }
                 }
             }
@@ -358,14 +358,18 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t dbuf = tm + b * BUF_COLS;
                 const int steps = min(4, k16 - 4 * c);
 #pragma unroll
-                for (int p = 0; p < PL; ++p) {
+                for (int p = 0; p <= PL; ++p) {
                     if (!mbar_wait_warp(&afull[s], ph, abort_flag, flags)) {
                         stop = true;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t a0 = sw128_lo(smem + s * A_BYTES);
-                    if (steps == 4) {
+                    if (p == PL) {   // the magnitudes: 32 bytes per K = 32 step
+                        const uint32_t bm = b0 + (PL * BN * CK * 2 >> 4);
+                        umma_warp_f8(dbuf + (uint32_t)(PL * BN), a0, bm, idesc_mag(), 0u);
+                        if (steps > 2) umma_warp_f8(dbuf + (uint32_t)(PL * BN), a0 + 2, bm + 2, idesc_mag(), 1u);
+                    } else if (steps == 4) {
                         umma_warp_x4(dbuf + (uint32_t)(p * BN), a0, b0, idesc((PL - p) * BN), p == 0 ? 0u : 1u);
                     } else {
                         for (int kk = 0; kk < steps; ++kk)   // 32 bytes per K = 16 step
@@ -394,7 +398,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // that vote and list by themselves, so that the halves drift apart and one's conversions overlap
         // the other's waits.  The vote is the only barrier: the tables of tile w + 1 are written before the
         // vote of tile w, and a thread still storing tile w - 1 reads others (three sets).  A failed wait
-        // makes the warp skip TMEM from then on but keep voting (its tiles count as weak), so no thread is
+        // makes the warp skip TMEM from then on but keep voting (its tiles are not stored), so no thread is
         // left waiting at a barrier.
         const int quarter = warp & 3, eighth = (warp - 2) >> 2, half = eighth >> 1, sub = (eighth & 1) * HB;
         const int dt = (threadIdx.x - 64) & 255;   // within the half: warps 2-9 are half 0, 10-17 half 1
@@ -438,12 +442,17 @@ __global__ void __launch_bounds__(THREADS, 1)
         int4 I = make_int4(0, 0, 0, 0);
         if ((int)blockIdx.x < nitems) I = open(0);
         vote_any(half, false);
+        const int row = quarter * 32 + lane;
         for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
             const Tables &T = mine[set];
             const E64Out &g = GROUPED ? T.g : static_cast<const E64Out &>(g0);
             long long hi[HB], lo[HB];
+            float mag[HB];
 #pragma unroll
-            for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
+            for (int j = 0; j < HB; ++j) {
+                hi[j] = lo[j] = 0;
+                mag[j] = 0.0f;
+            }
             for (int c = 0; c < I.z; ++c, ++gc) {
                 const unsigned buf = gc & 1u;
                 if (!bad) {
@@ -458,10 +467,11 @@ __global__ void __launch_bounds__(THREADS, 1)
                 tc_fence_after();
                 const uint32_t base =
                     tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * BUF_COLS + eighth * HB);
-                uint32_t r0[HB], r1[HB], r2[HB];
+                uint32_t r0[HB], r1[HB], r2[HB], rm[HB];
                 tmem_ld8(base, r0);
                 tmem_ld8(base + BN, r1);
                 tmem_ld8(base + 2 * BN, r2);
+                tmem_ld8(base + PL * BN, rm);
                 tmem_ld_wait();
                 if constexpr (PL == 3) {
                     tc_fence_before();
@@ -472,6 +482,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     add_sum<18>(hi[j], r0[j]);
                     add_sum<9>(hi[j], r1[j]);
                     add_sum<0>(hi[j], r2[j]);
+                    mag[j] += __uint_as_float(rm[j]);
                 }
                 if constexpr (PL > 3) {
                     uint32_t r3[HB];
@@ -495,14 +506,16 @@ __global__ void __launch_bounds__(THREADS, 1)
             set = set == 2 ? 0 : set + 1;
             if (w + (int)gridDim.x < nitems) I = open(set);
             if (!GROUPED && g0.ksplit > 1) {
-                longlong2 *dst = g0.part + ((long long)at * BN + eighth * HB) * BM + quarter * 32 + lane;
+                const long long at0 = ((long long)at * BN + eighth * HB) * BM + row;
 #pragma unroll
-                for (int j = 0; j < HB; ++j) dst[(long long)j * BM] = make_longlong2(hi[j], lo[j]);
+                for (int j = 0; j < HB; ++j) {
+                    g0.part[at0 + j * BM] = make_longlong2(hi[j], lo[j]);
+                    g0.pmag[at0 + j * BM] = mag[j];
+                }
                 continue;
             }
-            const int row = quarter * 32 + lane;
-            const bool weak = e64_finish<(PL > 3)>(g, hi, lo, T.rowE[row], T.colE + sub);
-            if (vote_any(half, weak || bad)) {
+            const bool left = e64_finish<(PL > 3)>(g, hi, lo, mag, T.rowE[row], T.colE + sub);
+            if (vote_any(half, left || bad)) {
                 // after a failed wait nothing is listed: the host reports the time-out
                 if (dt == 0 && *abort_flag == 0 && n0 < g.N) e64_list_tile(g, GROUPED ? at : 0, m0, n0);
             } else if (T.rowoff[row] >= 0) {
@@ -524,20 +537,26 @@ __global__ void __launch_bounds__(THREADS, 1)
 // bounds the parts' pass: a tile's block took 1 us for each of up to 64 parts (100 x 50 x 4000, two tiles: 66
 // us, with this launch 16).
 constexpr int PART_FOLD = 8;
-__global__ void __launch_bounds__(256) e64_fold_kernel(longlong2 *__restrict__ part, int ksplit, long long n) {
+__global__ void __launch_bounds__(256) e64_fold_kernel(longlong2 *__restrict__ part, float *__restrict__ pmag,
+                                                       int ksplit, long long n) {
     const long long i = blockIdx.x * 256LL + threadIdx.x;
     const int s0 = blockIdx.y * PART_FOLD;
     if (i >= n) return;
     longlong2 x[PART_FOLD];
+    float m[PART_FOLD];
 #pragma unroll
-    for (int s = 0; s < PART_FOLD; ++s)
+    for (int s = 0; s < PART_FOLD; ++s) {
         x[s] = s0 + s < ksplit ? part[(s0 + s) * n + i] : make_longlong2(0, 0);
+        m[s] = s0 + s < ksplit ? pmag[(s0 + s) * n + i] : 0.0f;
+    }
 #pragma unroll
     for (int s = 1; s < PART_FOLD; ++s) {
         x[0].x += x[s].x;
         x[0].y += x[s].y;
+        m[0] += m[s];
     }
     part[s0 * n + i] = x[0];
+    pmag[s0 * n + i] = m[0];
 }
 
 // K parts: one block per tile adds every step-th part's 64-bit sums (exact, so their number does not matter)
@@ -558,21 +577,26 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g, int s
     const long long mrow = (long long)m0 + quarter * 32 + lane;
     const int ea = mrow < g.M ? __ldg(g.expA + mrow) : 0;
     long long hi[HB], lo[HB];
+    float mag[HB];
 #pragma unroll
-    for (int j = 0; j < HB; ++j) hi[j] = lo[j] = 0;
+    for (int j = 0; j < HB; ++j) {
+        hi[j] = lo[j] = 0;
+        mag[j] = 0.0f;
+    }
 #pragma unroll 2
     for (int s = 0; s < g.ksplit; s += step) {
-        const longlong2 *src = g.part + (((long long)s * tiles + tile) * BN + eighth * HB) * BM + quarter * 32 + lane;
+        const long long at = (((long long)s * tiles + tile) * BN + eighth * HB) * BM + quarter * 32 + lane;
 #pragma unroll
         for (int j = 0; j < HB; ++j) {
-            const longlong2 p = src[(long long)j * BM];
+            const longlong2 p = g.part[at + j * BM];
             hi[j] += p.x;
             lo[j] += p.y;
+            mag[j] += g.pmag[at + j * BM];
         }
     }
     __syncthreads();
-    const bool weak = e64_finish<true>(g, hi, lo, ea, colE + eighth * HB);
-    if (vote_any(half, weak)) {
+    const bool left = e64_finish<true>(g, hi, lo, mag, ea, colE + eighth * HB);
+    if (vote_any(half, left)) {
         if ((threadIdx.x & 255) == 0 && n0 + half * VN < g.N) e64_list_tile(g, 0, m0, n0 + half * VN);
     } else if (mrow < g.M) {
         e64_store(g, hi, coloff + eighth * HB, mode_off(g.mC, g.row0 + mrow));
@@ -587,14 +611,15 @@ constexpr int PK = 128;
 constexpr int pack_rows(long long kpad) { return kpad <= 64 ? 32 : 16; }
 constexpr int pack_k(long long kpad) { return kpad <= 64 ? 64 : 128; }
 
-// one operand of a pack launch: rows [row0, row0 + R) of src into digit planes [NP][Rpad][Kpad] and
-// the rows' exponents
+// one operand of a pack launch: rows [row0, row0 + R) of src into digit planes [NP][Rpad][Kpad], magnitudes
+// [Rpad][mag_pitch] and the rows' exponents
 struct PackArgs {
     const double *src;
     Mode rm, km;
     long long row0, R, K, Rpad, Kpad;
     int *exps;
     __half *dst;
+    uint8_t *mag;
     unsigned blocks;   // of this operand in the launch
     int kfast;         // K (else the row index) is the source's unit-stride index
     int kseg;          // row-maximum pass: K chunks per block
@@ -638,10 +663,18 @@ __device__ __forceinline__ uint32_t digit_pair(unsigned long long s0, unsigned l
     return *reinterpret_cast<const uint32_t *>(&h);
 }
 
+// |x| in units of 2^-15 of its row's power of two as E5M2, cut below 2^-29 of it: the exponent field is 29 for
+// elements of the maximum's binade, the mantissa's two leading bits follow
+__device__ __forceinline__ uint32_t mag_code(double x, int E) {
+    const int c = (int)(((unsigned)__double2hiint(x) & 0x7FFFFFFFu) >> 18) - ((E - 29) << 2);
+    return c < 4 ? 0u : (uint32_t)c;
+}
+
 template <int PL, int KW>
 struct PackSmem {
     static constexpr int PR = 2048 / KW;
     uint32_t outp[PL][PR][KW / 2 + 4];   // pitch: 16-byte pieces, the pair stores of both layouts free of conflicts
+    uint16_t mag[PR][KW / 2 + 4];        // pairs of magnitudes, 8-byte pieces
     long long roff[PR], koff[KW];
     unsigned rowE[PR];                   // the rows' exponents; LOCALMAX: their largest magnitudes
 };
@@ -700,10 +733,11 @@ __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, 
     for (int i = 0; i < 4; ++i) {
         const int r = row_of(i), c = pair_of(i);
         if (c >= pairs) continue;
-        const int base = shift_base<PL>(LOCALMAX ? exp_of(sm.rowE[r]) : (int)sm.rowE[r]);
+        const int E = LOCALMAX ? exp_of(sm.rowE[r]) : (int)sm.rowE[r], base = shift_base<PL>(E);
         const unsigned long long s0 = fixed_point<PL>(x[i][0], base), s1 = fixed_point<PL>(x[i][1], base);
 #pragma unroll
         for (int p = 0; p < PL; ++p) sm.outp[p][r][c] = digit_pair<PL>(s0, s1, p);
+        sm.mag[r][c] = (uint16_t)(E ? mag_code(x[i][0], E) | mag_code(x[i][1], E) << 8 : 0u);
     }
     __syncthreads();
     // one piece of eight halves of each plane to a thread
@@ -714,6 +748,8 @@ __device__ __forceinline__ void e64_pack_block(const PackArgs &a, long long r0, 
 #pragma unroll
     for (int p = 0; p < PL; ++p, dst += plane)
         *reinterpret_cast<uint4 *>(dst) = *reinterpret_cast<const uint4 *>(&sm.outp[p][row][4 * seg]);
+    *reinterpret_cast<uint2 *>(a.mag + (size_t)(r0 + row) * mag_pitch(a.Kpad) + k0 + 8 * seg) =
+        *reinterpret_cast<const uint2 *>(&sm.mag[row][4 * seg]);
 }
 
 // both operands of a GEMM in one launch: blocks [0, a.blocks) pack a, the rest b
@@ -826,27 +862,41 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
 }
 
-// digit planes [NP][rows][kpad]; one box = 64 K values (past kpad: zeros) x box_rows rows x box_planes
-CUtensorMap plane_map(const __half *base, long long rows, long long kpad, int np, int box_rows, int box_planes) {
+// [np][rows][kpad] elements, rows pitch bytes apart
+CUtensorMap tensor_map(CUtensorMapDataType type, CUtensorMapSwizzle swizzle, long long pitch, const void *base,
+                       long long kpad, long long rows, int np, int box_rows, int box_planes) {
     CUtensorMap m;
     std::memset(&m, 0, sizeof(m));
     cuuint64_t dims[3] = {(cuuint64_t)kpad, (cuuint64_t)rows, (cuuint64_t)np};
-    cuuint64_t strides[2] = {(cuuint64_t)kpad * 2, (cuuint64_t)rows * kpad * 2};
+    cuuint64_t strides[2] = {(cuuint64_t)pitch, (cuuint64_t)(rows * pitch)};
     cuuint32_t box[3] = {(cuuint32_t)CK, (cuuint32_t)box_rows, (cuuint32_t)box_planes};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = encode_fn()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<__half *>(base), dims, strides, box,
-                             estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = encode_fn()(&m, type, 3, const_cast<void *>(base), dims, strides, box, estr,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw Error(JUES_ECUDA, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
     return m;
 }
+// digit planes [np][rows][kpad]; one box = 64 K values (past kpad: zeros) x box_rows rows x box_planes
+CUtensorMap plane_map(const __half *planes, long long rows, long long kpad, int np, int box_rows, int box_planes) {
+    return tensor_map(CU_TENSOR_MAP_DATA_TYPE_FLOAT16, CU_TENSOR_MAP_SWIZZLE_128B, 2 * kpad, planes, kpad, rows, np, box_rows,
+                      box_planes);
+}
+// the magnitudes behind them, [rows][mag_pitch] bytes
+uint8_t *mag_at(const __half *planes, int np, long long rows, long long kpad) {
+    return reinterpret_cast<uint8_t *>(const_cast<__half *>(planes) + (size_t)np * rows * kpad);
+}
+CUtensorMap mag_map(const __half *planes, long long rows, long long kpad, int np, int box_rows) {
+    return tensor_map(CU_TENSOR_MAP_DATA_TYPE_UINT8, CU_TENSOR_MAP_SWIZZLE_64B, mag_pitch(kpad),
+                      mag_at(planes, np, rows, kpad), kpad, rows, 1, box_rows, 1);
+}
 
 PackArgs pack_args(const double *src, const Mode &rm, const Mode &km, long long row0, long long R, long long K,
-                   long long Rpad, long long Kpad, int *exps, __half *dst) {
+                   long long Rpad, long long Kpad, int *exps, __half *dst, uint8_t *mag) {
     PackArgs p;
     p.src = src; p.rm = rm; p.km = km;
     p.row0 = row0; p.R = R; p.K = K; p.Rpad = Rpad; p.Kpad = Kpad;
-    p.exps = exps; p.dst = dst;
+    p.exps = exps; p.dst = dst; p.mag = mag;
     p.blocks = (unsigned)((Rpad / pack_rows(Kpad)) * ((Kpad + pack_k(Kpad) - 1) / pack_k(Kpad)));
     p.kfast = km.s0 == 1 && km.d0 > 1;
     // about 16 blocks per SM in the row-maximum pass, at most 16 chunks a block
@@ -906,13 +956,6 @@ void allow_smem(Ctx *ctx) {
     JUES_CHECK_CUDA(cudaFuncSetAttribute(gett_e64_kernel<PL, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          smem_bytes(PL)));
     set.fetch_or(bit);
-}
-
-// an FMA loop's own error grows as sqrt(K): 2^-weak keeps 2^-61 2^weak at its level
-int weak_level(long long K) {
-    int kl = 0;
-    while ((1LL << kl) < K) ++kl;
-    return 5 + kl / 2;
 }
 
 void set_scaling(E64Args &g, double alpha, double beta, bool in_place) {
@@ -990,7 +1033,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     if (mtiles_all * ntiles >= (1LL << 30) || (Nall / PR) * ((Kpad + PK - 1) / PK) >= (1LL << 31)) return false;
     if (!ctx->pack) ctx->pack = new PackCache();
     PackCache &pc = *ctx->pack;
-    const size_t hA = (size_t)NP * Mall * Kpad, hB = (size_t)NP * Nall * Kpad;
+    const size_t hA = plane_halves(NP, Mall, Kpad), hB = plane_halves(NP, Nall, Kpad);
     const bool keepA = keep_planes(a.a_const, a.K, hA), keepB = keep_planes(a.b_const, a.K, hB);
     PackEntry *eA = keepA ? find_entry(pc, a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad) : nullptr;
     PackEntry *eB = keepB ? find_entry(pc, a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad) : nullptr;
@@ -1001,7 +1044,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     longlong2 *part = nullptr;
     for (size_t panel = PANEL_MAX;; panel /= 2) {
         if (!keepA && hA > panel)
-            prow = std::max<long long>(BM, (long long)(panel / ((size_t)NP * Kpad)) / BM * BM);
+            prow = std::max<long long>(BM, (long long)(panel / plane_halves(NP, 2, Kpad) * 2) / BM * BM);
         if ((prow / PR) * ((Kpad + PK - 1) / PK) >= (1LL << 31)) return false;
         // K parts of a grid too small for the GPU (chunks of 64 K); exact whatever their number
         const long long panel_tiles = prow / BM * ntiles;
@@ -1025,7 +1068,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
                 newB.reset(new PackEntry{a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad, NP, take_buffer(ctx, pc.free_planes, hB),
                                          take_buffer(ctx, pc.free_exps, (size_t)Nall)});
             if (!keepA) {
-                grow(ctx, pc.e64_planes[0], (size_t)NP * prow * Kpad);
+                grow(ctx, pc.e64_planes[0], plane_halves(NP, prow, Kpad));
                 grow(ctx, pc.e64_exps[0], (size_t)prow);
             }
             if (!keepB) {
@@ -1033,9 +1076,9 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
                 grow(ctx, pc.e64_exps[1], (size_t)Nall);
             }
             grow(ctx, pc.e64_list, (size_t)(4 * mtiles_all * ntiles + 1));
-            if (ksplit > 1)
-                part = static_cast<longlong2 *>(
-                    ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN * sizeof(longlong2)));
+            if (ksplit > 1)   // the parts' sums, then their magnitudes
+                part = static_cast<longlong2 *>(ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN *
+                                                                    (sizeof(longlong2) + sizeof(float))));
             break;
         } catch (const Error &e) {
             if (e.code != JUES_ENOMEM) throw;
@@ -1062,9 +1105,11 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         __half *planesA = eA ? eA->buf.p : newA ? newA->buf.p : pc.e64_planes[0].p;
         int *expsA = eA ? eA->exps.p : newA ? newA->exps.p : pc.e64_exps[0].p;
         const bool packB = r0 == 0 && !eB;
-        const PackArgs pb = pack_args(a.B, a.nB, a.kB, 0, a.N, a.K, Nall, Kpad, expsB, planesB);
+        const PackArgs pb = pack_args(a.B, a.nB, a.kB, 0, a.N, a.K, Nall, Kpad, expsB, planesB,
+                                      mag_at(planesB, NP, Nall, Kpad));
         if (!eA)
-            run_pack<NP>(ctx, pack_args(a.A, a.mA, a.kA, r0, R, a.K, Rpad, Kpad, expsA, planesA), packB ? &pb : nullptr);
+            run_pack<NP>(ctx, pack_args(a.A, a.mA, a.kA, r0, R, a.K, Rpad, Kpad, expsA, planesA, mag_at(planesA, NP, Rpad, Kpad)),
+                         packB ? &pb : nullptr);
         else if (packB)
             run_pack<NP>(ctx, pb, nullptr);
         E64Args g;
@@ -1079,14 +1124,15 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         g.flags = ctx->d_flags;
         g.ksplit = ksplit; g.kper = kper;
         g.part = part;
+        g.pmag = reinterpret_cast<float *>(part + (size_t)ksplit * g.mtiles * g.ntiles * BM * BN);
         g.list = pc.e64_list.p;
-        g.weak = weak_level(a.K);
-        const CUtensorMap ma = plane_map(planesA, Rpad, Kpad, NP, BM, 1), mb = plane_map(planesB, Nall, Kpad, NP, BN, NP);
+        const CUtensorMap ma = plane_map(planesA, Rpad, Kpad, NP, BM, 1), mb = plane_map(planesB, Nall, Kpad, NP, BN, NP),
+                          xa = mag_map(planesA, Rpad, Kpad, NP, BM), xb = mag_map(planesB, Nall, Kpad, NP, BN);
         const long long items = e64_items(g);
         {
             Ctx::Scope s(ctx, name);
             gett_e64_kernel<NP, false><<<(unsigned)std::min<long long>(items, 152), THREADS, smem_bytes(NP),
-                                         ctx->stream>>>(ma, mb, g, nullptr, 0, (int)items);
+                                         ctx->stream>>>(ma, mb, xa, xb, g, nullptr, 0, (int)items);
             JUES_CHECK_CUDA(cudaGetLastError());
         }
         if (ksplit > 1) {
@@ -1097,7 +1143,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
             if (ksplit > PART_FOLD) {
                 step = PART_FOLD;
                 e64_fold_kernel<<<dim3((unsigned)(n / 256), (unsigned)((ksplit + step - 1) / step)), 256, 0,
-                                  ctx->stream>>>(part, ksplit, n);
+                                  ctx->stream>>>(part, g.pmag, ksplit, n);
                 ctx->count_launch();
                 JUES_CHECK_CUDA(cudaGetLastError());
             }
@@ -1122,13 +1168,14 @@ void e64_alloc(Ctx *ctx, E64Planes &P, long long rows, long long K, int np) {
     P.K = K;
     P.Kpad = roundup(K, 16);
     JUES_REQUIRE(P.rows < (1LL << 31) && (P.rows / PR) * ((P.Kpad + PK - 1) / PK) < (1LL << 31), "too many operand rows");
-    P.planes = DBuf<__half>(ctx, (size_t)np * P.rows * P.Kpad);
+    P.planes = DBuf<__half>(ctx, plane_halves(np, P.rows, P.Kpad));
     P.exps = DBuf<int>(ctx, (size_t)P.rows);
 }
 
 void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const Mode &km, long long R) {
     JUES_REQUIRE(R <= P.rows, "operand does not fit its planes");
-    const PackArgs a = pack_args(src, rm, km, 0, R, P.K, P.rows, P.Kpad, P.exps.p, P.planes.p);
+    const PackArgs a = pack_args(src, rm, km, 0, R, P.K, P.rows, P.Kpad, P.exps.p, P.planes.p,
+                                 mag_at(P.planes.p, P.np, P.rows, P.Kpad));
     if (P.np == 3)
         run_pack<3>(ctx, a, nullptr);
     else
@@ -1150,8 +1197,8 @@ E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long 
     g.flags = ctx->d_flags;
     g.ksplit = 1; g.kper = (g.k16 + 3) / 4;
     g.part = nullptr;
+    g.pmag = nullptr;
     g.list = list;
-    g.weak = weak_level(K);
     return g;
 }
 
@@ -1160,7 +1207,9 @@ void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Ar
     if (n <= 0 || items <= 0) return;
     JUES_REQUIRE(A.np == B.np && A.Kpad == B.Kpad && items < (1LL << 31), "mismatched planes");
     const CUtensorMap ma = plane_map(A.planes.p, A.rows, A.Kpad, A.np, BM, 1),
-                      mb = plane_map(B.planes.p, B.rows, B.Kpad, B.np, BN, B.np);
+                      mb = plane_map(B.planes.p, B.rows, B.Kpad, B.np, BN, B.np),
+                      xa = mag_map(A.planes.p, A.rows, A.Kpad, A.np, BM),
+                      xb = mag_map(B.planes.p, B.rows, B.Kpad, B.np, BN);
     JUES_CHECK_CUDA(cudaMemsetAsync(list, 0, sizeof(int), ctx->stream));
     E64Args g{};
     g.flags = ctx->d_flags;
@@ -1169,10 +1218,10 @@ void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Ar
         Ctx::Scope s(ctx, name);
         if (A.np == 3) {
             allow_smem<3, true>(ctx);
-            gett_e64_kernel<3, true><<<grid, THREADS, smem_bytes(3), ctx->stream>>>(ma, mb, g, probs, n, (int)items);
+            gett_e64_kernel<3, true><<<grid, THREADS, smem_bytes(3), ctx->stream>>>(ma, mb, xa, xb, g, probs, n, (int)items);
         } else {
             allow_smem<NP, true>(ctx);
-            gett_e64_kernel<NP, true><<<grid, THREADS, smem_bytes(NP), ctx->stream>>>(ma, mb, g, probs, n, (int)items);
+            gett_e64_kernel<NP, true><<<grid, THREADS, smem_bytes(NP), ctx->stream>>>(ma, mb, xa, xb, g, probs, n, (int)items);
         }
         JUES_CHECK_CUDA(cudaGetLastError());
     }
@@ -1235,7 +1284,8 @@ E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const char 
         long long ra = 0, rb = 0, at = 0;
         auto pack = [&](const E64Planes &P, long long row, const double *src, const Mode &rm, const Mode &km, long long R,
                         long long K) {
-            PackArgs p = pack_args(src, rm, km, 0, R, K, P.rows, P.Kpad, P.exps.p + row, P.planes.p + row * P.Kpad);
+            PackArgs p = pack_args(src, rm, km, 0, R, K, P.rows, P.Kpad, P.exps.p + row, P.planes.p + row * P.Kpad,
+                                   mag_at(P.planes.p, P.np, P.rows, P.Kpad) + row * mag_pitch(P.Kpad));
             first.push_back(g->blocks);
             g->blocks += (unsigned)(roundup(R, pr) / pr);
             ops.push_back(p);

@@ -22,8 +22,6 @@ struct E64Out {
     long long N;                // columns
     int alpha_pow2, alpha_k, alpha_neg;
     int beta_mode;              // 0: C = v; 1: C += v in place; 2: C = Cin + v; 3: C = beta Cin + v
-    int weak;                   // a row or column is weak when no result reaches 2^-weak max|a| max|b|
-    int pad;
 };
 // one contraction as the kernels see it
 struct E64Args : E64Out {
@@ -37,16 +35,18 @@ struct E64Args : E64Out {
     unsigned *flags;
     int ksplit, kper;           // K parts of kper chunks each
     longlong2 *part;            // ksplit > 1: [part][tile][BN][BM] pairs of 64-bit sums
+    float *pmag;                // and their sums of magnitudes
 };
 
-// digit planes [np][rows][Kpad] of one operand (or of several with the same K, rows concatenated)
+// digit planes and the magnitude plane, [np + 1][rows][Kpad], of one operand (or of several with the same K, rows
+// concatenated)
 struct E64Planes {
     DBuf<__half> planes;
     DBuf<int> exps;
     long long rows = 0, K = 0, Kpad = 0;
     int np = 0;
 };
-// np = 7 planes (FP64) or 3 (27 bits: split precision)
+// np = 7 digit planes (FP64) or 3 (27 bits: split precision)
 void e64_alloc(Ctx *ctx, E64Planes &P, long long rows, long long K, int np);
 void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const Mode &km, long long R);
 // C[mC(m) + nC(n)] = alpha sum_k A[rowA + m, k] B[rowB + n, k] + beta C, beta 0 or 1; item0: the items of

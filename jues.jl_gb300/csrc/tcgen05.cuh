@@ -157,6 +157,18 @@ __device__ __forceinline__ void umma_warp_x4(uint32_t tmem_d, uint32_t alo, uint
         "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// one K = 32 step of 8-bit floats; both tiles 64 bytes a row in TMA's 64-byte swizzle (8-row groups of 512 bytes)
+__device__ __forceinline__ void umma_warp_f8(uint32_t tmem_d, uint32_t alo, uint32_t blo, uint32_t idesc,
+                                             uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 a, b;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 a, {%1, 0x80004020};\n\tmov.b64 b, {%2, 0x80004020};\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], a, b, %3, p;\n\t}\n" ::"r"(tmem_d),
+        "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit_warp(uint64_t *bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"
