@@ -966,7 +966,8 @@ void allow_smem(Ctx *ctx) {
 void set_scaling(E64Args &g, double alpha, double beta, bool in_place) {
     g.alpha = alpha; g.beta = beta;
     int ak = 0;
-    g.alpha_pow2 = std::frexp(std::fabs(alpha), &ak) == 0.5 && ak - 1 >= -8 && ak - 1 <= 8;
+    // operands within 2^+-400 and sums from 2^-70 on: with 2^+-100 more a result is still a normal number
+    g.alpha_pow2 = std::frexp(std::fabs(alpha), &ak) == 0.5 && ak - 1 >= -100 && ak - 1 <= 100;
     g.alpha_k = g.alpha_pow2 ? ak - 1 : 0;
     g.alpha_neg = g.alpha_pow2 && alpha < 0;
     g.beta_mode = beta == 0.0 ? 0 : (beta == 1.0 ? (in_place ? 1 : 2) : 3);

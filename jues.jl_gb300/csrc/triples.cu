@@ -11,9 +11,15 @@
 // W[a,b,c,k] through the output modes, and one kernel forms V = W + the three (vo|vo) T1 terms on the
 // fly and sums the reference's weighted energy expression over a >= b >= c (:117-131).  The twelve
 // contractions per pair took 48 launches with their packs; at o = 12, v = 48 the call took 31 ms.
+// A row of R and a column of Q each hold integrals beside amplitudes under one scale of the digits, so the
+// amplitudes enter both as sigma T2, sigma the power of two that brings their largest element to the integrals'
+// (a factor of sigma on W, taken off with alpha): with amplitudes far smaller than the integrals the digits of
+// half of each row would else be lost and its contractions redone on the FP64 pipe (T2 2^-10 of the size that it
+// has beside these integrals, o = 12, v = 48: 34 ms, with sigma 4.0).
 // Partial sums go to fixed per-block slots that are added in a fixed order, and the six additions
 // to W are ordered by their launches, so the result is deterministic.
 #include <algorithm>
+#include <cmath>
 #include <vector>
 
 #include "gett_e64.cuh"
@@ -247,11 +253,54 @@ void pair_w(Ctx *ctx, int prec, int i, int j, const double *T2, const View4 &Vv,
          plain(O0[3]), mode2(v, O0[0], O0[1]), 1.0, w, ab, ck, "pt_w", true);
 }
 
+// out = max(out, bits of |x|) over the four-index array a of extents d0..d3
+__global__ void __launch_bounds__(256) pt_absmax_kernel(View4 a, int d0, int d1, int d2, long long n,
+                                                        unsigned long long *out) {
+    unsigned long long m = 0;
+    for (long long t = blockIdx.x * 256LL + threadIdx.x; t < n; t += 256LL * gridDim.x) {
+        const long long t1 = t / d0, t2 = t1 / d1;
+        const double x = a.p[t % d0 * a.s[0] + t1 % d1 * a.s[1] + t2 % d2 * a.s[2] + t2 / d2 * a.s[3]];
+        m = max(m, (unsigned long long)__double_as_longlong(fabs(x)));
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, d));
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
+// log2 of sigma: the power of two nearest sqrt(max|Vvvvo| max|Vvooo|) / max|T2|; 0 where one of them is zero or
+// not finite
+int amplitude_scale(Ctx *ctx, const double *T2, const View4 &Vv, const View4 &Vo, int o, int v) {
+    auto *bits = reinterpret_cast<unsigned long long *>(ctx->d_red);
+    JUES_CHECK_CUDA(cudaMemsetAsync(bits, 0, 3 * sizeof(*bits), ctx->stream));
+    {
+        Ctx::Scope s(ctx, "pt_absmax");
+        auto run = [&](const View4 &a, int d0, int d1, int d2, int d3, int k) {
+            const long long n = (long long)d0 * d1 * d2 * d3;
+            pt_absmax_kernel<<<(unsigned)std::min<long long>((n + 1023) / 1024, 152 * 8), 256, 0, ctx->stream>>>(
+                a, d0, d1, d2, n, bits + k);
+            JUES_CHECK_CUDA(cudaGetLastError());
+        };
+        run(col_major(T2, o, o, v), o, o, v, v, 0);
+        run(Vv, v, v, v, o, 1);
+        run(Vo, v, o, o, o, 2);
+        ctx->count_launch();
+        ctx->count_launch();
+    }
+    double x[3];
+    JUES_CHECK_CUDA(cudaMemcpyAsync(x, bits, sizeof(x), cudaMemcpyDeviceToHost, ctx->stream));
+    ctx->sync();
+    for (double y : x)
+        if (!(y > 0.0) || !std::isfinite(y)) return 0;
+    const double l = 0.5 * (std::log2(x[1]) + std::log2(x[2])) - std::log2(x[0]);
+    return (int)std::lrint(std::max(-90.0, std::min(90.0, l)));
+}
+
 // rows R and columns Q, dense and as digit planes; throws JUES_ENOMEM where they do not fit
 struct PtStacks {
     DBuf<double> R, Q;
     E64Planes pr, pq;
     long long rowsR, rowsQ, K;
+    double unscale;   // 1 / sigma
     PtStacks(Ctx *ctx, int np, const double *T2, const View4 &Vv, const View4 &Vo, int o, int v) {
         const long long oo = (long long)o * o, oov = oo * v, v2 = (long long)v * v;
         K = v + o;
@@ -261,15 +310,18 @@ struct PtStacks {
         Q = DBuf<double>(ctx, (size_t)(rowsQ * K));
         e64_alloc(ctx, pr, rowsR, K, np);
         e64_alloc(ctx, pq, rowsQ, K, np);
+        const int ls = amplitude_scale(ctx, T2, Vv, Vo, o, v);
+        const double sigma = std::ldexp(1.0, ls);
+        unscale = std::ldexp(1.0, -ls);
         const long long *V0 = Vv.s, *O0 = Vo.s;
-        // R[x + v y + v^2 p, d] = Vvvvo[y,d,x,p];  R[.., v + l] = -T2[p,l,x,y]
+        // R[x + v y + v^2 p, d] = Vvvvo[y,d,x,p];  R[.., v + l] = -sigma T2[p,l,x,y]
         permute4(ctx, Perm4{{v, v, o, v}, {V0[2], V0[0], V0[3], V0[1]}, {1, v, v2, rowsR}}, 1.0, Vv.p, 0.0, R.p);
-        permute4(ctx, Perm4{{v, v, o, o}, {oo, oov, 1, o}, {1, v, v2, rowsR}}, -1.0, T2, 0.0, R.p + rowsR * v);
+        permute4(ctx, Perm4{{v, v, o, o}, {oo, oov, 1, o}, {1, v, v2, rowsR}}, -sigma, T2, 0.0, R.p + rowsR * v);
         for (int h = 0; h < 2; ++h) {
-            // Q[u + v r + v o q, d] = T2[r,q,u,d];  Q[.., v + l] = Vvooo[u,r,q,l]; second half: r and q traded
+            // Q[u + v r + v o q, d] = sigma T2[r,q,u,d];  Q[.., v + l] = Vvooo[u,r,q,l]; second half: r and q traded
             double *q = Q.p + h * v * oo;
             const long long sr = h ? (long long)v * o : v, sq = h ? v : (long long)v * o;
-            permute4(ctx, Perm4{{v, o, o, v}, {oo, 1, o, oov}, {1, sr, sq, rowsQ}}, 1.0, T2, 0.0, q);
+            permute4(ctx, Perm4{{v, o, o, v}, {oo, 1, o, oov}, {1, sr, sq, rowsQ}}, sigma, T2, 0.0, q);
             permute4(ctx, Perm4{{v, o, o, o}, {O0[0], O0[1], O0[2], O0[3]}, {1, sr, sq, rowsQ}}, 1.0, Vo.p, 0.0,
                      q + rowsQ * v);
         }
@@ -363,11 +415,11 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
                     long long w0 = 0;
                     for (int p = 0; p < b.npair; ++p) {
                         const PtTerm m = pt_term(t, i, j, o, v);
-                        args.push_back(e64_problem(ctx, st->pr, st->pq, st->K, m.rowA, m.M, m.rowB, m.N, 1.0, t ? 1.0 : 0.0,
+                        args.push_back(e64_problem(ctx, st->pr, st->pq, st->K, m.rowA, m.M, m.rowB, m.N, st->unscale, t ? 1.0 : 0.0,
                                                    W.p + w0, m.mC, m.nC, (int)n, lp));
                         GettArgs g;
                         g.M = m.M; g.N = m.N; g.K = st->K;
-                        g.alpha = 1.0; g.beta = t ? 1.0 : 0.0;
+                        g.alpha = st->unscale; g.beta = t ? 1.0 : 0.0;
                         g.A = st->R.p + m.rowA; g.mA = plain(1); g.kA = plain(st->rowsR);
                         g.B = st->Q.p + m.rowB; g.kB = plain(st->rowsQ); g.nB = plain(1);
                         g.C = W.p + w0; g.mC = m.mC; g.nC = m.nC;
