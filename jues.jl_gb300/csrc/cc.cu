@@ -595,7 +595,7 @@ static std::unique_ptr<CCState> cc_begin(Ctx *ctx, int method, int n, int o, int
     JUES_REQUIRE(valid_precision(opts.precision), "unknown precision");
     JUES_REQUIRE(opts.guess >= 0 && opts.guess <= 2, "unknown guess");
     std::unique_ptr<CCState> s(new CCState());
-    s->ctx = ctx;
+    s->ctx = s->idle.ctx = ctx;
     s->method = method;
     s->n = n; s->o = o; s->v = v;
     s->opts = opts;

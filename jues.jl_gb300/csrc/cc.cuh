@@ -5,8 +5,17 @@
 
 namespace jues {
 
+// Frees the idle packs of a context; a state's first member, so it runs when the buffers are gone
+struct IdlePacks {
+    Ctx *ctx = nullptr;
+    ~IdlePacks() {
+        if (ctx) pack_cache_reclaim(ctx, false);
+    }
+};
+
 // Device-resident closed-shell CC problem (CCD or CCSD).
 struct CCState {
+    IdlePacks idle;
     Ctx *ctx = nullptr;
     int method = 0;   // 0 CCD, 1 CCSD
     int n = 0, o = 0, v = 0;

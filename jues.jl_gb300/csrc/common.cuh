@@ -249,7 +249,8 @@ void gett_tc_noalloc(Ctx *ctx, const GettArgs &g);
 void expired_wait(Ctx *ctx);
 size_t gett_tc_noalloc_limit();
 void pack_cache_clear(Ctx *ctx);
-bool pack_cache_reclaim(Ctx *ctx);   // frees the FP64 digit planes; whether anything was freed
+// memory wanted elsewhere: frees the buffers of dropped packs, and with all set the FP64 digit planes too
+void pack_cache_reclaim(Ctx *ctx, bool all);
 void pack_cache_destroy(PackCache *p);
 void batch_cache_destroy(BatchCache *p);
 void batch_rmp2(Ctx *ctx, int nsys, const jues_mp2_system *sys, int precision, double e_bar, double *e_out,

@@ -42,7 +42,17 @@ Ctx::~Ctx() {
 
 void *Ctx::alloc(size_t bytes) {
     if (bytes == 0) return nullptr;
-    if (mem_limit && mem_used + bytes > mem_limit) pack_cache_reclaim(this);
+    // idle packs first, then the digit planes and the scratch of K parts (its users launch before they allocate)
+    auto reclaim = [&](bool all) {
+        pack_cache_reclaim(this, all);
+        if (all) {
+            free(splitk_ws, splitk_bytes);
+            splitk_ws = nullptr;
+            splitk_bytes = 0;
+        }
+    };
+    for (bool all : {false, true})
+        if (mem_limit && mem_used + bytes > mem_limit) reclaim(all);
     if (mem_limit && mem_used + bytes > mem_limit)
         throw Error(JUES_ENOMEM, "device allocation of " + std::to_string(bytes) +
                                      " bytes exceeds the context memory limit (" +
@@ -65,10 +75,11 @@ void *Ctx::alloc(size_t bytes) {
     }
     void *p = nullptr;
     cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
-    if (e != cudaSuccess) {
+    for (bool all : {false, true}) {
+        if (e == cudaSuccess) break;
         // give the pool's idle blocks back and try once more (fragmentation)
         cudaGetLastError();
-        pack_cache_reclaim(this);
+        reclaim(all);
         cudaStreamSynchronize(stream);
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);

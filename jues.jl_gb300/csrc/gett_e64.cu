@@ -973,10 +973,18 @@ void set_scaling(E64Args &g, double alpha, double beta, bool in_place) {
     g.beta_mode = beta == 0.0 ? 0 : (beta == 1.0 ? (in_place ? 1 : 2) : 3);
 }
 
+// the allocations of one product: its planes are not reclaimed for one another
 struct Busy {
     PackCache &c;
-    explicit Busy(PackCache &x) : c(x) { c.busy = true; }
-    ~Busy() { c.busy = false; }
+    Busy(PackCache &x, const PackEntry *a, const PackEntry *b) : c(x) {
+        c.busy = c.e64_active = true;
+        c.in_use[0] = a;
+        c.in_use[1] = b;
+    }
+    ~Busy() {
+        c.busy = c.e64_active = false;
+        c.in_use[0] = c.in_use[1] = nullptr;
+    }
 };
 
 PackEntry *find_entry(PackCache &pc, const double *src, const Mode &rm, const Mode &km, long long R, long long K,
@@ -1040,7 +1048,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     if (!ctx->pack) ctx->pack = new PackCache();
     PackCache &pc = *ctx->pack;
     const size_t hA = plane_halves(NP, Mall, Kpad), hB = plane_halves(NP, Nall, Kpad);
-    const bool keepA = keep_planes(a.a_const, a.K, hA), keepB = keep_planes(a.b_const, a.K, hB);
+    bool keepA = keep_planes(a.a_const, a.K, hA), keepB = keep_planes(a.b_const, a.K, hB);
     PackEntry *eA = keepA ? find_entry(pc, a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad) : nullptr;
     PackEntry *eB = keepB ? find_entry(pc, a.B, a.nB, a.kB, a.N, a.K, Nall, Kpad) : nullptr;
     std::unique_ptr<PackEntry> newA, newB;
@@ -1066,7 +1074,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         kper = (chunks + ksplit - 1) / ksplit;
         ksplit = (chunks + kper - 1) / kper;
         try {
-            Busy busy(pc);
+            Busy busy(pc, eA, eB);
             if (keepA && !eA && !newA)
                 newA.reset(new PackEntry{a.A, a.mA, a.kA, a.M, a.K, Mall, Kpad, NP, take_buffer(ctx, pc.free_planes, hA),
                                          take_buffer(ctx, pc.free_exps, (size_t)Mall)});
@@ -1088,6 +1096,14 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
             break;
         } catch (const Error &e) {
             if (e.code != JUES_ENOMEM) throw;
+            if ((keepA && !eA) || (keepB && !eB)) {   // no room to keep new planes: transient ones, in panels
+                newA.reset();
+                newB.reset();
+                keepA = eA != nullptr;
+                keepB = eB != nullptr;
+                panel = 2 * PANEL_MAX;
+                continue;
+            }
             if (keepA || hA <= PANEL_MIN || panel <= PANEL_MIN) return false;   // the FP64 pipe needs no planes
         }
     }

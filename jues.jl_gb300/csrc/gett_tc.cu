@@ -842,27 +842,27 @@ void pack_cache_clear(Ctx *ctx) {
         ctx->pack->busy = false;
     }
 }
-// Device memory wanted elsewhere: give back what the FP64 digit planes hold (they are formed again, or
-// the FP64 pipe runs instead).  Frees are stream-ordered, so queued readers are safe.
-bool pack_cache_reclaim(Ctx *ctx) {
-    if (!ctx->pack || ctx->pack->busy) return false;
+// Device memory wanted elsewhere: give back the buffers of dropped entries and, with all set, what the FP64 digit
+// planes hold (they are formed again, or the FP64 pipe runs instead), except those that a digit product in its
+// allocations uses.  Frees are stream-ordered, so queued readers are safe.
+void pack_cache_reclaim(Ctx *ctx, bool all) {
+    if (!ctx->pack) return;
     PackCache &pc = *ctx->pack;
+    const bool was_busy = pc.busy;
     pc.busy = true;
-    bool any = false;
-    auto e64 = [](const std::unique_ptr<PackEntry> &x) { return x->np == E64_NP; };
-    const size_t before = pc.cached.size();
-    pc.cached.erase(std::remove_if(pc.cached.begin(), pc.cached.end(), e64), pc.cached.end());
-    any = pc.cached.size() != before;
-    for (auto *b : {&pc.e64_planes[0], &pc.e64_planes[1]}) {
-        any = any || b->p;
-        b->reset();
+    pc.free_planes.clear();
+    pc.free_exps.clear();
+    if (all) {
+        auto idle = [&](const std::unique_ptr<PackEntry> &x) {
+            return x->np == E64_NP && x.get() != pc.in_use[0] && x.get() != pc.in_use[1];
+        };
+        pc.cached.erase(std::remove_if(pc.cached.begin(), pc.cached.end(), idle), pc.cached.end());
+        if (!pc.e64_active) {
+            for (auto *b : {&pc.e64_planes[0], &pc.e64_planes[1]}) b->reset();
+            for (auto *b : {&pc.e64_exps[0], &pc.e64_exps[1], &pc.e64_list}) b->reset();
+        }
     }
-    for (auto *b : {&pc.e64_exps[0], &pc.e64_exps[1], &pc.e64_list}) {
-        any = any || b->p;
-        b->reset();
-    }
-    pc.busy = false;
-    return any;
+    pc.busy = was_busy;
 }
 // Entries are keyed by their source address.  Device memory is reused quickly (the context's
 // pool hands freed blocks out again), so every free of device memory forgets the entries whose

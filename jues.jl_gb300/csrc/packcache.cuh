@@ -19,6 +19,9 @@ struct PackEntry {
 };
 struct PackCache {
     bool busy = false;   // inside a cache operation: frees of the cache's own buffers are not lookups
+    // a digit product being set up: its kept operands, and whether the transient planes are its own
+    const PackEntry *in_use[2] = {nullptr, nullptr};
+    bool e64_active = false;
     std::vector<std::unique_ptr<PackEntry>> cached;
     DBuf<__half> scratch[2];
     DBuf<int> scratch_exp[2];
