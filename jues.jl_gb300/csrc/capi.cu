@@ -491,6 +491,7 @@ int jues_rmp2_adjoint(jues_ctx *ctx, const double *gao, int n, const double *C, 
         cudaSetDevice(c.device);
         DBuf<double> gbuf;
         const double *gp = ao_operand(c, gao, (size_t)n * n * n * n, precision, gbuf);
+        const PackScope packs(&c, gp);
         DBuf<double> dC = h2d(c, C, (size_t)n * n);
         DBuf<double> de = h2d(c, eps, (size_t)n);
         const double *Co = dC.p, *Cv = dC.p + (size_t)n * o;
@@ -547,7 +548,6 @@ int jues_rmp2_adjoint(jues_ctx *ctx, const double *gao, int n, const double *C, 
             }
             d2h(c, C_bar, cb.p, cb.n);
         }
-        pack_cache_drop(&c, gp);
         c.check_flags();
     });
 }

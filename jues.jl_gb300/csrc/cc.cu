@@ -711,6 +711,7 @@ static CCState *cc_finish(std::unique_ptr<CCState> s) {
 CCState *cc_create(Ctx *ctx, int method, const double *g, int n, const double *Cocc, int o,
                    const double *Cvir, int v, const double *eps_dev, const jues_cc_opts &opts) {
     std::unique_ptr<CCState> s = cc_begin(ctx, method, n, o, v, eps_dev, opts);
+    const PackScope packs(ctx, g);   // g may be the caller's own device array
     const long long oo = (long long)o * o, vv = (long long)v * v, ov = (long long)o * v;
     const size_t t2n = (size_t)(oo * vv);
     // integral blocks (mRCCD.jl:120-127, mRCCSD.jl:102-110), physicists' notation

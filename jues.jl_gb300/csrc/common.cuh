@@ -257,6 +257,15 @@ void batch_rmp2(Ctx *ctx, int nsys, const jues_mp2_system *sys, int precision, d
                 double **gao_bar, double **C_bar, jues_batch_info *info);
 void pack_cache_drop(Ctx *ctx, const void *ptr);
 void pack_cache_forget(Ctx *ctx, const void *p, size_t bytes);   // on every free of device memory
+// the packs of an array whose values may change once the scope is left, also by an error
+struct PackScope {
+    Ctx *ctx;
+    const void *p;
+    PackScope(Ctx *c, const void *src) : ctx(c), p(src) {}
+    PackScope(const PackScope &) = delete;
+    PackScope &operator=(const PackScope &) = delete;
+    ~PackScope() { pack_cache_drop(ctx, p); }
+};
 
 // ---------------------------------------------------------------------------------------
 // bandwidth kernels (kernels.cu)

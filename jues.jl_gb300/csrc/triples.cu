@@ -20,6 +20,7 @@
 // to W are ordered by their launches, so the result is deterministic.
 #include <algorithm>
 #include <cmath>
+#include <memory>
 #include <vector>
 
 #include "gett_e64.cuh"
@@ -465,6 +466,9 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
         for (auto &x : hitems) x.w0 = v3 * x.k;
         JUES_CHECK_CUDA(cudaMemcpyAsync(items.p, hitems.data(), hitems.size() * sizeof(PtItem), cudaMemcpyHostToDevice,
                                         ctx->stream));
+        std::vector<std::unique_ptr<PackScope>> kept;   // the slices of the operands that pair_w declares constant
+        for (int i = 0; i < o; ++i)
+            for (const double *p : {Vv.p + i * Vv.s[3], T2 + i}) kept.emplace_back(new PackScope(ctx, p));
         long long at = 0;
         for (int i = 0; i < o; ++i)
             for (int j = 0; j <= i; ++j) {
@@ -472,10 +476,6 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
                 energy(ctx, W.p, items.p + at, j + 1, tiles, T1, Vvovo, fo, fv, o, v, slots.p);
                 at += j + 1;
             }
-        for (int i = 0; i < o; ++i) {   // the kept slices
-            pack_cache_drop(ctx, Vv.p + i * Vv.s[3]);
-            pack_cache_drop(ctx, T2 + i);
-        }
     }
     pt_sum_slots<<<1, 1024, 0, ctx->stream>>>(slots.p, PT_BLOCKS, slots.p + PT_BLOCKS);
     JUES_CHECK_CUDA(cudaGetLastError());
