@@ -211,7 +211,7 @@ static void pair_l(CCState *s, const char *name) {
 // ladders and the folds together 970 -> 510).
 // Taken from o^2 v^4 = 3.5e9 on, where the unfolded ladder's 170 us outweigh the folds' and the second sign's
 // launches, and only where the folded weights (half of vvvv's size) leave room for everything the solver may
-// still allocate: the DIIS vectors and the digit planes.  A split solve's few closing sweeps do not repay the
+// still allocate: the DIIS vectors and the digit planes (those held now, of whatever ran before, can be had back).  A split solve's few closing sweeps do not repay the
 // folding of vvvv (nbf = 90, two of them: 14.18 ms, folded 14.20) and stay unfolded.
 // ---------------------------------------------------------------------------------------
 static bool fold64_ready(CCState *s) {
@@ -224,7 +224,8 @@ static bool fold64_ready(CCState *s) {
     const double words = 2.0 * nq * nq + 2.0 * oo * nq + 7.0 * np * nq + 2.0 * np * np + 2.0 * oo * np;
     const double later = 2.0 * std::max(1, s->opts.diis_size) * oo * vv + 4.0 * vv * vv + 16.0 * oo * vv;
     const double need = 8.0 * (words + later);
-    if (ctx->mem_limit && (double)ctx->mem_used + need > (double)ctx->mem_limit) return false;
+    const size_t held = pack_cache_reclaimable(ctx);
+    if (ctx->mem_limit && (double)(ctx->mem_used - held) + need > (double)ctx->mem_limit) return false;
     size_t avail = 0, total = 0;
     JUES_CHECK_CUDA(cudaMemGetInfo(&avail, &total));
     if (ctx->pool) {
@@ -233,15 +234,17 @@ static bool fold64_ready(CCState *s) {
         JUES_CHECK_CUDA(cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used));
         avail += (size_t)(reserved - std::min(used, reserved));
     }
-    if (need > (double)avail) return false;
+    if (need > (double)(avail + held)) return false;
+    const bool had_arrays = s->invF.p;   // a session that ran split sweeps before
     try {
         s->Bpm = DBuf<double>(ctx, (size_t)(2 * nq * nq));
         s->Xw64 = DBuf<double>(ctx, (size_t)(2 * oo * nq));
         pair_arrays(s);
     } catch (const Error &e) {
         if (e.code != JUES_ENOMEM) throw;
-        s->Bpm.reset();
-        s->Xw64.reset();
+        for (DBuf<double> *b : {&s->Bpm, &s->Xw64}) b->reset();
+        if (!had_arrays)
+            for (DBuf<double> *b : {&s->Opm, &s->Apm, &s->Lpm, &s->Cpm, &s->Xpm, &s->invF}) b->reset();
         return false;
     }
     pair_fold(ctx, s->vvvv.p, nq, true, 0, 1, v, (int)v, vv, vv * v, 0.5, true, s->Bpm.p);

@@ -251,6 +251,7 @@ size_t gett_tc_noalloc_limit();
 void pack_cache_clear(Ctx *ctx);
 // memory wanted elsewhere: frees the buffers of dropped packs, and with all set the FP64 digit planes too
 void pack_cache_reclaim(Ctx *ctx, bool all);
+size_t pack_cache_reclaimable(Ctx *ctx);   // bytes that it would free
 void pack_cache_destroy(PackCache *p);
 void batch_cache_destroy(BatchCache *p);
 void batch_rmp2(Ctx *ctx, int nsys, const jues_mp2_system *sys, int precision, double e_bar, double *e_out,

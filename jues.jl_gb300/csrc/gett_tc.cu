@@ -864,6 +864,18 @@ void pack_cache_reclaim(Ctx *ctx, bool all) {
     }
     pc.busy = was_busy;
 }
+size_t pack_cache_reclaimable(Ctx *ctx) {
+    size_t bytes = ctx->splitk_bytes;
+    if (!ctx->pack) return bytes;
+    const PackCache &pc = *ctx->pack;
+    for (auto &b : pc.free_planes) bytes += b.n * sizeof(__half);
+    for (auto &b : pc.free_exps) bytes += b.n * sizeof(int);
+    for (auto &x : pc.cached)
+        if (x->np == E64_NP) bytes += x->buf.n * sizeof(__half) + x->exps.n * sizeof(int);
+    for (auto *b : {&pc.e64_planes[0], &pc.e64_planes[1]}) bytes += b->n * sizeof(__half);
+    for (auto *b : {&pc.e64_exps[0], &pc.e64_exps[1], &pc.e64_list}) bytes += b->n * sizeof(int);
+    return bytes;
+}
 // Entries are keyed by their source address.  Device memory is reused quickly (the context's
 // pool hands freed blocks out again), so every free of device memory forgets the entries whose
 // source lay in the freed range: a later array at the same address can never hit a stale pack.

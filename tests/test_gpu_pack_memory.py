@@ -105,3 +105,46 @@ def test_planes_that_cannot_be_kept_are_formed_again():
     finally:
         free.close()
         tight.close()
+
+
+def test_folded_ladders_do_not_depend_on_planes_held_before():
+    # the smallest limit after the set-up under which the first sweep still folds the ladders, told by the last
+    # bits of the amplitudes; with 250 MB more of another product's planes than the set-up leaves it folds under the same limit
+    from juesgpu import _lib
+    from juesgpu.CoupledCluster import CCSession
+    n, o = 78, 18
+    sy = make_system(n, o, 3 * n, seed=3)
+    g = np.asfortranarray(sy.ao_eri())
+    rng = np.random.default_rng(2)
+    A, B = np.asfortranarray(rng.normal(size=(130000, 400))), np.asfortranarray(rng.normal(size=(400, 32)))
+
+    def sweep(limit, product=False):
+        ctx = _lib.Context(0)
+        try:
+            with mock.patch.object(_lib, "context", lambda device=0: ctx):
+                s = CCSession(0, gao=g, Cocc=np.asfortranarray(sy.C[:, :o]), Cvir=np.asfortranarray(sy.C[:, o:]),
+                              eps=sy.eps, maxit=2, r_conv=0.0, precision="fp64")
+            try:
+                if product:
+                    assert gemm(ctx, A, B, 0)
+                ctx.set_mem_limit(limit * MB)
+                s.iterate(1)
+                ctx.set_mem_limit(0)
+                return s.amplitudes()[1]
+            except _lib.JuESError as e:
+                assert e.code == _lib.ENOMEM
+                return None
+            finally:
+                s.close()
+        finally:
+            ctx.close()
+
+    want = sweep(0)
+    lo, hi = 1, 8192
+    while hi - lo > 8:
+        mid = (lo + hi) // 2
+        got = sweep(mid)
+        lo, hi = (lo, mid) if got is not None and np.array_equal(got, want) else (mid, hi)
+    got = sweep(hi - 16)
+    assert got is None or not np.array_equal(got, want)   # below the line the bits do differ
+    assert np.array_equal(sweep(hi + 8, product=True), want)
