@@ -10,6 +10,7 @@
 #include <cstring>
 #include <functional>
 #include <mutex>
+#include <system_error>
 #include <thread>
 
 #include "staging.cuh"
@@ -22,7 +23,11 @@ namespace {
 class WorkerPool {
   public:
     explicit WorkerPool(int workers) {
-        for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { run(); });
+        try {
+            for (int i = 0; i < workers; ++i) threads_.emplace_back([this] { run(); });
+        } catch (const std::system_error &) {
+            // fewer threads, or the caller alone, do the same work
+        }
     }
     ~WorkerPool() {
         {
@@ -148,11 +153,19 @@ static Staging *staging_of(Ctx *ctx) {
     return st;
 }
 
+// a slot's memory, null where page-locked memory is refused
 static char *locked(char *&p, size_t bytes) {
-    if (!p) JUES_CHECK_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&p), bytes, cudaHostAllocDefault));
+    if (!p && cudaHostAlloc(reinterpret_cast<void **>(&p), bytes, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        p = nullptr;
+    }
     return p;
 }
-static char *slot_of(Staging *st, int k) { return locked(st->host[k], kSlot); }
+static char *slot_of(Staging *st, int k) {
+    char *p = locked(st->host[k], kSlot);
+    if (!p) throw Error(JUES_ECUDA, "page-locked memory for the upload ring was refused");
+    return p;
+}
 
 // host side of one fill: copy the pieces' bytes between the slot and the caller's arrays in tasks of
 // 1 MB (256 KB in a fill of 16 MB or less) over the workers (to_slot: caller -> slot)
@@ -198,8 +211,17 @@ void staged_d2h(Ctx *ctx, const std::vector<HostSeg> &segs) {
     const bool small = !st->host[0] && bytes < kLarge;   // slot 0 is the first that an upload takes
     const std::vector<Fill> fills = plan_fills(segs, small ? kSmall : kSlot);
     if (fills.empty()) return;
-    const int slots = small ? kSmalls : kSlots;
-    auto slot_at = [&](int k) { return small ? locked(st->small[k], kSmall) : slot_of(st, k); };
+    auto slot_at = [&](int k) { return small ? locked(st->small[k], kSmall) : locked(st->host[k], kSlot); };
+    // two buffers in turn are enough; without them the driver copies into the caller's arrays
+    const int most = (int)std::min<size_t>(small ? kSmalls : kSlots, fills.size());
+    int slots = 0;
+    while (slots < most && slot_at(slots)) ++slots;
+    if (slots < std::min(most, 2)) {
+        for (const HostSeg &s : segs)
+            JUES_CHECK_CUDA(cudaMemcpyAsync(s.dst, s.src, s.bytes, cudaMemcpyDeviceToHost, ctx->stream));
+        ctx->sync();
+        return;
+    }
     // the link fills slot i + 1 while the host empties slot i
     auto issue = [&](size_t i) {
         const int k = (int)(i % slots);

@@ -21,7 +21,7 @@ struct HostSeg {
 void staged_h2d(Ctx *ctx, const std::vector<HostSeg> &segs);
 
 // Device -> host (src device, dst host) after the work queued on ctx->stream; returns with the
-// data in the caller's arrays.
+// data in the caller's arrays.  Where page-locked memory is refused it copies them directly.
 void staged_d2h(Ctx *ctx, const std::vector<HostSeg> &segs);
 
 // releases the ring and its threads (context destruction)
