@@ -170,6 +170,7 @@ struct BatchPlan {
     DBuf<double> arena;
     std::vector<size_t> off_g, off_C, off_eps, off_gb, off_cb;
     std::vector<int> n, o;
+    E64Shared e64;                  // digit planes, one set for all stages
     std::vector<Stage> stages;      // grouped GETT stages in order; energy runs after stage 4
     DBuf<SysDesc> sys;
     DBuf<double> energies, epart;
@@ -186,9 +187,15 @@ struct BatchPlan {
 
 struct BatchCache {
     std::map<std::string, std::unique_ptr<BatchPlan>> plans;
+    bool busy = false;   // inside a batched call
 };
 
 void batch_cache_destroy(BatchCache *c) { delete c; }
+
+// memory wanted elsewhere: the idle plan, its arena and planes (built again by the next batched call)
+void batch_cache_reclaim(Ctx *ctx) {
+    if (ctx->batch && !ctx->batch->busy) ctx->batch->plans.clear();
+}
 
 static void run_stage(Ctx *ctx, Stage &st) {
     if (st.shape == kShapeE64) {
@@ -473,7 +480,12 @@ static std::unique_ptr<BatchPlan> make_plan(Ctx *ctx, const std::string &key, in
     if (split)
         for (Stage &st : bp->stages) st.tc = tc_group_build(ctx, st.args, (st.name + "_tc").c_str());
     else if (ctx->batch_form != 1)
-        for (Stage &st : bp->stages) st.e64 = e64_group_build(ctx, st.args, (st.name + "_e64").c_str());
+    {
+        std::vector<const std::vector<GettArgs> *> all;
+        for (const Stage &st : bp->stages) all.push_back(&st.args);
+        e64_shared_reserve(ctx, bp->e64, all);
+        for (Stage &st : bp->stages) st.e64 = e64_group_build(ctx, st.args, bp->e64, (st.name + "_e64").c_str());
+    }
     for (Stage &st : bp->stages)
         if (!st.e64) split_long_k(ctx, st);
     return bp;
@@ -502,6 +514,11 @@ void batch_rmp2(Ctx *ctx, int nsys, const jues_mp2_system *sys, int precision, d
         want_cb = want_cb || (C_bar && C_bar[s]);
     }
     if (!ctx->batch) ctx->batch = new BatchCache();
+    struct Busy {
+        BatchCache *c;
+        explicit Busy(BatchCache *x) : c(x) { c->busy = true; }
+        ~Busy() { c->busy = false; }
+    } busy(ctx->batch);
     const std::string key = signature(nsys, sys, e_bar, want_gb, want_cb, split, ctx->batch_form);
     auto it = ctx->batch->plans.find(key);
     bool fresh = false;

@@ -254,6 +254,7 @@ void pack_cache_reclaim(Ctx *ctx, bool all);
 size_t pack_cache_reclaimable(Ctx *ctx);   // bytes that it would free
 void pack_cache_destroy(PackCache *p);
 void batch_cache_destroy(BatchCache *p);
+void batch_cache_reclaim(Ctx *ctx);   // frees the plan that no call is using
 void batch_rmp2(Ctx *ctx, int nsys, const jues_mp2_system *sys, int precision, double e_bar, double *e_out,
                 double **gao_bar, double **C_bar, jues_batch_info *info);
 void pack_cache_drop(Ctx *ctx, const void *ptr);

@@ -42,17 +42,19 @@ Ctx::~Ctx() {
 
 void *Ctx::alloc(size_t bytes) {
     if (bytes == 0) return nullptr;
-    // idle packs first, then the digit planes and the scratch of K parts (its users launch before they allocate)
-    auto reclaim = [&](bool all) {
-        pack_cache_reclaim(this, all);
-        if (all) {
+    // idle packs first, then the digit planes and the scratch of K parts (its users launch before they allocate),
+    // then an idle batch plan
+    auto reclaim = [&](int level) {
+        if (level < 2) pack_cache_reclaim(this, level == 1);
+        if (level == 1) {
             free(splitk_ws, splitk_bytes);
             splitk_ws = nullptr;
             splitk_bytes = 0;
         }
+        if (level == 2) batch_cache_reclaim(this);
     };
-    for (bool all : {false, true})
-        if (mem_limit && mem_used + bytes > mem_limit) reclaim(all);
+    for (int level = 0; level < 3; ++level)
+        if (mem_limit && mem_used + bytes > mem_limit) reclaim(level);
     if (mem_limit && mem_used + bytes > mem_limit)
         throw Error(JUES_ENOMEM, "device allocation of " + std::to_string(bytes) +
                                      " bytes exceeds the context memory limit (" +
@@ -75,11 +77,10 @@ void *Ctx::alloc(size_t bytes) {
     }
     void *p = nullptr;
     cudaError_t e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);
-    for (bool all : {false, true}) {
-        if (e == cudaSuccess) break;
+    for (int level = 0; level < 3 && e != cudaSuccess; ++level) {
         // give the pool's idle blocks back and try once more (fragmentation)
         cudaGetLastError();
-        reclaim(all);
+        reclaim(level);
         cudaStreamSynchronize(stream);
         cudaMemPoolTrimTo(pool, 0);
         e = cudaMallocFromPoolAsync(&p, bytes, pool, stream);

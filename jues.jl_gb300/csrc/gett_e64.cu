@@ -1256,49 +1256,114 @@ void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Ar
 // ---------------------------------------------------------------------------------------------
 struct E64Group {
     std::string name;
-    E64Planes A, B;
+    E64Planes A, B;             // views of the shared planes
     DBuf<E64Args> args;
     DBuf<GroupProblem> f64;
     DBuf<PackArgs> ops;
     DBuf<unsigned> first;
-    DBuf<int> list;
+    int *list = nullptr;
     int nprob = 0, nops = 0;
     unsigned blocks = 0;
     long long items = 0;
 };
 
-E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const char *name) {
-    // Measured on 24 systems of nbf 10 to 60: the eleven K <= 64 stages took 22 ms on the FP64 tiles and take
-    // 3 ms here; a stage below 1e8 flop in all costs its four launches more than that
-    double flops = 0.0;
-    long long kmax = 0;
+namespace {
+
+// the stage's contractions as the kernels take them, and the planes that they need
+struct StageShape {
     std::vector<GettArgs> ps;
+    long long kmax = 0, kpad = 0, pr = 0, rows[2] = {0, 0}, items = 0;
+    size_t halves(int side) const { return plane_halves(NP, rows[side], kpad); }
+    size_t bytes() const {
+        return (halves(0) + halves(1)) * sizeof(__half) + (size_t)(rows[0] + rows[1] + 4 * items + 1) * sizeof(int);
+    }
+};
+
+// A stage below 1e8 flop in all costs its four launches more than the FP64 tiles take (24 systems of nbf 10 to
+// 60: the eleven K <= 64 stages took 22 ms on the FP64 tiles and take 3 ms here).
+bool stage_shape(const std::vector<GettArgs> &in, StageShape &s) {
+    double flops = 0.0;
     for (const GettArgs &a : in) {
         if (a.M <= 0 || a.N <= 0) continue;
         if (a.K < 1 || a.K > PK || (a.beta != 0.0 && a.beta != 1.0) || (a.beta == 1.0 && a.Cin && a.Cin != a.C))
-            return nullptr;
+            return false;
         flops += 2.0 * (double)a.M * (double)a.N * (double)a.K;
-        kmax = std::max(kmax, a.K);
-        ps.push_back(orient(a));
+        s.kmax = std::max(s.kmax, a.K);
+        s.ps.push_back(orient(a));
+        s.items += e64_tiles(s.ps.back().M, s.ps.back().N);
     }
-    if (flops < 1e8) return nullptr;
+    if (flops < 1e8) return false;
+    s.kpad = roundup(s.kmax, 16);
+    s.pr = pack_rows(s.kpad);
+    for (const GettArgs &a : s.ps) {
+        s.rows[0] += roundup(a.M, s.pr);
+        s.rows[1] += roundup(a.N, s.pr);
+    }
+    for (long long &r : s.rows) r = roundup(r, BM);
+    return s.rows[0] < (1LL << 30) && s.rows[1] < (1LL << 30) && s.items < (1LL << 28);
+}
+
+template <class T>
+DBuf<T> view_of(const DBuf<T> &b) {
+    DBuf<T> v;   // no context: never freed through it
+    v.p = b.p;
+    v.n = b.n;
+    return v;
+}
+
+}  // namespace
+
+void e64_shared_reserve(Ctx *ctx, E64Shared &sh, const std::vector<const std::vector<GettArgs> *> &stages) {
+    std::vector<StageShape> fit;
+    for (const std::vector<GettArgs> *st : stages) {
+        StageShape s;
+        if (stage_shape(*st, s)) fit.push_back(std::move(s));
+    }
+    std::sort(fit.begin(), fit.end(), [](const StageShape &a, const StageShape &b) { return a.bytes() < b.bytes(); });
+    for (; !fit.empty(); fit.pop_back()) {   // without its largest stage where that does not fit
+        size_t halves[2] = {0, 0}, rows[2] = {0, 0}, items = 0;
+        for (const StageShape &s : fit) {
+            for (int k = 0; k < 2; ++k) {
+                halves[k] = std::max(halves[k], s.halves(k));
+                rows[k] = std::max(rows[k], (size_t)s.rows[k]);
+            }
+            items = std::max(items, (size_t)s.items);
+        }
+        try {
+            for (int k = 0; k < 2; ++k) {
+                grow(ctx, sh.planes[k], halves[k]);
+                grow(ctx, sh.exps[k], rows[k]);
+            }
+            grow(ctx, sh.list, 4 * items + 1);
+            return;
+        } catch (const Error &e) {
+            if (e.code != JUES_ENOMEM) throw;   // the FP64 tiles need no planes
+            sh = E64Shared();
+        }
+    }
+}
+
+E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const E64Shared &sh, const char *name) {
+    StageShape s;
+    if (!stage_shape(in, s)) return nullptr;
+    for (int k = 0; k < 2; ++k)
+        if (sh.planes[k].n < s.halves(k) || sh.exps[k].n < (size_t)s.rows[k]) return nullptr;
+    if (sh.list.n < (size_t)(4 * s.items + 1)) return nullptr;
     try {
         std::unique_ptr<E64Group> g(new E64Group());
         g->name = name;
-        long long rowsA = 0, rowsB = 0;
-        const long long pr = pack_rows(roundup(kmax, 16));
-        for (const GettArgs &a : ps) {
-            rowsA += roundup(a.M, pr);
-            rowsB += roundup(a.N, pr);
+        g->items = s.items;
+        g->list = sh.list.p;
+        const long long pr = s.pr;
+        for (int k = 0; k < 2; ++k) {
+            E64Planes &P = k ? g->B : g->A;
+            P.np = NP;
+            P.rows = s.rows[k];
+            P.K = s.kmax;
+            P.Kpad = s.kpad;
+            P.planes = view_of(sh.planes[k]);
+            P.exps = view_of(sh.exps[k]);
         }
-        if (rowsA >= (1LL << 30) || rowsB >= (1LL << 30)) return nullptr;
-        e64_alloc(ctx, g->A, rowsA, kmax, NP);
-        e64_alloc(ctx, g->B, rowsB, kmax, NP);
-        long long items = 0;
-        for (const GettArgs &a : ps) items += e64_tiles(a.M, a.N);
-        if (items >= (1LL << 28)) return nullptr;
-        g->items = items;
-        g->list = DBuf<int>(ctx, (size_t)(4 * items + 1));
         std::vector<E64Args> args;
         std::vector<GroupProblem> f64;
         std::vector<PackArgs> ops;
@@ -1312,11 +1377,11 @@ E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const char 
             g->blocks += (unsigned)(roundup(R, pr) / pr);
             ops.push_back(p);
         };
-        for (const GettArgs &a : ps) {
+        for (const GettArgs &a : s.ps) {
             pack(g->A, ra, a.A, a.mA, a.kA, a.M, a.K);
             pack(g->B, rb, a.B, a.nB, a.kB, a.N, a.K);
             args.push_back(e64_problem(ctx, g->A, g->B, a.K, ra, a.M, rb, a.N, a.alpha, a.beta, a.C, a.mC, a.nC, (int)at,
-                                       g->list.p));
+                                       g->list));
             f64.push_back(to_problem(a));
             ra += roundup(a.M, pr);
             rb += roundup(a.N, pr);
@@ -1352,7 +1417,7 @@ void e64_group_exec(Ctx *ctx, E64Group *g) {
             e64_pack_grouped_kernel<NP, 128><<<g->blocks, 256, 0, ctx->stream>>>(g->ops.p, g->first.p, g->nops);
         JUES_CHECK_CUDA(cudaGetLastError());
     }
-    e64_group_run(ctx, g->A, g->B, g->args.p, g->f64.p, g->nprob, g->items, g->list.p, g->name.c_str());
+    e64_group_run(ctx, g->A, g->B, g->args.p, g->f64.p, g->nprob, g->items, g->list, g->name.c_str());
 }
 
 void e64_group_destroy(E64Group *g) { delete g; }

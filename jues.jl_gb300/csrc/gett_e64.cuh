@@ -60,9 +60,16 @@ inline long long e64_tiles(long long M, long long N) { return ((M + 127) / 128) 
 void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Args *probs, const GroupProblem *f64,
                    int n, long long items, int *list, const char *name);
 
-// a stage of a batch (K <= 128 throughout): null when the sizes or the memory left do not suit it
+// A stage of a batch (K <= 128 throughout).  Stages run one after another, so their operands go through one
+// set of planes: reserve sizes it for the largest of the stages that suit it and fit the memory left; build gives
+// null for the others
 struct E64Group;
-E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &probs, const char *name);
+struct E64Shared {
+    DBuf<__half> planes[2];
+    DBuf<int> exps[2], list;
+};
+void e64_shared_reserve(Ctx *ctx, E64Shared &sh, const std::vector<const std::vector<GettArgs> *> &stages);
+E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &probs, const E64Shared &sh, const char *name);
 void e64_group_exec(Ctx *ctx, E64Group *g);
 void e64_group_destroy(E64Group *g);
 
