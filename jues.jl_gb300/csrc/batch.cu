@@ -296,27 +296,31 @@ static void upload_stage(Ctx *ctx, Stage &st) {
                                     cudaMemcpyHostToDevice, ctx->stream));
 }
 
-// time each tile shape on the real stage (inputs already in the arena) and keep the fastest
+// Time each form on the real stage (inputs already in the arena) and keep the fastest.  The digit form is timed
+// first: where it beats what the FP64 pipe needs at best for 32 x 32 tiles (2 FP64 FMAs a clock and SM, 1.26 TFLOP/s
+// at 2070 MHz), no tile shape can be faster and none is timed (500 systems of nbf 10 to 20 with adjoints, first call: 131 ms, with
+// every shape of every stage timed 218).
 static void autotune(Ctx *ctx, BatchPlan &bp) {
     cudaEvent_t e0, e1;
     JUES_CHECK_CUDA(cudaEventCreate(&e0));
     JUES_CHECK_CUDA(cudaEventCreate(&e1));
     for (size_t k = 0; k < bp.stages.size(); ++k) {
         Stage &st = bp.stages[k];
-        if (st.e64) {   // by its sizes, not by timing
-            st.shape = kShapeE64;
-            run_stage(ctx, st);
-            if ((int)k + 1 == bp.n_forward) run_gamma(ctx, bp);
-            continue;
-        }
+        double flops = 0.0;
+        for (const GettArgs &a : st.args)
+            flops += 2.0 * (double)((a.M + 31) / 32 * 32) * (double)((a.N + 31) / 32 * 32) * (double)a.K;
         float best = -1.f;
         int best_shape = 0;
-        // the FP64 tile shapes, and the grouped tcgen05 form where it was built
-        const int first = (ctx->batch_form == 2 && st.tc) ? kShapeTC : 0;
-        const int last = (st.tc && ctx->batch_form != 1) ? kShapeTC : kNumTileShapes - 1;
-        for (int sh = first; sh <= last; ++sh) {
+        // the grouped tensor-core form where it was built, and the FP64 tile shapes
+        std::vector<int> shapes;
+        if (st.e64) shapes.push_back(kShapeE64);
+        if (st.tc && ctx->batch_form != 1) shapes.push_back(kShapeTC);
+        if (shapes.empty() || ctx->batch_form != 2)
+            for (int sh = 0; sh < kNumTileShapes; ++sh) shapes.push_back(sh);
+        for (int sh : shapes) {
+            if (sh < kNumTileShapes && best_shape == kShapeE64 && best > 0.f && best <= flops / 1.26e9) break;
             st.shape = sh;
-            if (sh != kShapeTC) upload_stage(ctx, st);
+            if (sh < kNumTileShapes) upload_stage(ctx, st);
             // warm once, then time
             run_stage(ctx, st);
             JUES_CHECK_CUDA(cudaEventRecord(e0, ctx->stream));
@@ -328,7 +332,11 @@ static void autotune(Ctx *ctx, BatchPlan &bp) {
             if (best < 0 || ms < best) { best = ms; best_shape = sh; }
         }
         st.shape = best_shape;
-        if (st.shape != kShapeTC) upload_stage(ctx, st);
+        if (st.shape < kNumTileShapes) upload_stage(ctx, st);
+        if (st.e64 && st.shape != kShapeE64) {
+            e64_group_destroy(st.e64);
+            st.e64 = nullptr;
+        }
         // stages read what earlier stages wrote: run this one for real before tuning the next
         run_stage(ctx, st);
         if ((int)k + 1 == bp.n_forward) run_gamma(ctx, bp);
