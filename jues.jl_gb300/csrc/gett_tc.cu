@@ -19,7 +19,7 @@
 // accumulation as L2 reductions).  The grid is persistent (one CTA per SM); a ragged last round
 // has its tiles split over K, their parts summed by tail_reduce_kernel.  Operand tiles
 // arrive by TMA (128-byte swizzle) into a STAGES-deep shared-memory ring guarded by mbarriers;
-// one thread issues the TMA loads and one the MMAs.  Every mbarrier wait is bounded by
+// one thread issues the TMA loads and one warp, in step, the MMAs.  Every mbarrier wait is bounded by
 // %globaltimer; on expiry the CTA raises FLAG_TIMEOUT, skips its stores, frees its TMEM and
 // returns.
 #include <cuda.h>

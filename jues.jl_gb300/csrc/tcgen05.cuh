@@ -102,22 +102,10 @@ __device__ __forceinline__ void tmem_relinquish() {
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// D[tmem] (+)= A[smem desc] . B[smem desc]^T, 16-bit inputs, FP32 accumulation
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                     smem_u32(bar))
-                 : "memory");
-}
-// The same issued by a whole warp in step (one elected lane issues).  With warp-uniform loops and
+// D[tmem] (+)= A[smem] . B[smem]^T, 16-bit inputs, FP32 accumulation, issued by a whole warp in step (one
+// elected lane issues).  Both tiles are K-major as TMA writes them with 128-byte swizzle: the shared-memory
+// descriptor has the start address >> 4, LBO unused (1), SBO = 1024 bytes between 8-row groups, version 1 and layout
+// type 2 (SWIZZLE_128B).  With warp-uniform loops and
 // operands an MMA costs a few issue slots; a loop that one lane runs alone takes about 100 clocks per
 // MMA, more than a narrow MMA itself.  alo, blo: low words of sw128 descriptors (sw128_lo); the
 // high word is constant.
@@ -220,13 +208,6 @@ __device__ __forceinline__ void red_add_f64(double *p, double v) {
     asm volatile("red.global.add.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
 }
 
-// UMMA shared-memory descriptor of a K-major tile written by TMA with 128-byte swizzle:
-// start address >> 4, LBO unused (1), SBO = 1024 bytes between 8-row groups, version 1,
-// layout type 2 = SWIZZLE_128B.
-__device__ __forceinline__ uint64_t sw128_desc(const void *smem) {
-    const uint64_t a = smem_u32(smem);
-    return ((a & 0x3FFFFull) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
 __device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
