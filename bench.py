@@ -588,7 +588,8 @@ def run_gpu(args):
         t_e2e, nsw, e2e_kernels, e2e_host, e_e2e = runs[len(runs) // 2]
         h2d = gao.nbytes + system.C.nbytes + eps.nbytes
         e2e = {"value": t_e2e / nsw, "unit": "s/iter", "h2d_bytes_per_step": int(h2d / nsw),
-               "d2h_bytes_per_step": int(8 / nsw), "sweeps": nsw, "converged": nsw < args.e2e_maxit,
+               "d2h_bytes_per_step": 8,   # every sweep's energy is read back (the call's log)
+               "sweeps": nsw, "converged": nsw < args.e2e_maxit,
                "wall_s": t_e2e, "energy": e_e2e,
                "energy_error_eh": (e_e2e - e_gold) if e_gold is not None else None,
                "config": "precision=split (three-plane integrals, two-plane sweeps), MP2 guess, DIIS 6, "
