@@ -21,9 +21,10 @@
 // the column.  So every element is judged by the magnitude it is made of: a further plane holds |x| cut to E5M2,
 // whose products, a narrow 8-bit MMA for every 32 K values, sum to P <= sum |a_k b_k|; an element is taken only
 // where P >= 2^-7 max|a| max|b| (and 1/16 more), which bounds its error by K 2^-53 sum |a_k b_k| + 2^-53 |a.b|
-// whatever the operands are.  A half tile (16 columns) with an element below that, or with a
-// row or column that holds a non-finite, subnormal-only or extreme (beyond 2^+-400) maximum, is not stored but
-// listed, and gett_f64_tiles recomputes the listed ones on the FP64 pipe, with the same special values as ever.
+// whatever the operands are.  Elements below that, and those of rows and columns that hold a non-finite,
+// subnormal-only or extreme (beyond 2^+-400) maximum, are not stored but listed, and gett_f64_tiles recomputes them
+// on the FP64 pipe, with the same special values as ever: one by one where up to a quarter of the pieces (eight
+// columns of a row) of a half tile have any, else the half tile (16 columns).
 // Cancellation alone lists nothing, and neither do zeros of symmetry: P = 0 where a row and a column have no
 // nonzero element in common, and the result is exactly 0.  Against exact products, relative Frobenius error for normal entries:
 // 4.7e-17 at every size, the FMA kernels 1.3e-16 (K = 100) to 8.4e-16 (640^3).
@@ -126,20 +127,20 @@ __device__ __forceinline__ long long e64_join(long long hi, long long lo, int &u
 
 // One thread's row of a tile (8 columns): its sums become FP64 values (hi[j] is overwritten with
 // the bits), and the checks above run.  mag: the elements' sums of magnitudes; ea: the row's biased exponent (0
-// outside M or a zero row); colE: the columns' (shared memory).  Returns whether this thread saw a reason to
-// leave the tile to the FP64 pipe.
+// outside M or a zero row); colE: the columns' (shared memory).  Returns the columns left to the FP64 pipe.
 template <bool LOW, class E>
-__device__ __forceinline__ bool e64_finish(const E64Out &g, long long (&hi)[HB], const long long (&lo)[HB],
+__device__ __forceinline__ unsigned e64_finish(const E64Out &g, long long (&hi)[HB], const long long (&lo)[HB],
                                            const float (&mag)[HB], int ea, const E *colE) {
     const bool live = ea != 0;
-    bool bad = live && (ea < E_MIN || ea > E_MAX);
+    unsigned left = live && (ea < E_MIN || ea > E_MAX) ? (1u << HB) - 1 : 0u;
     const int neg = g.alpha_neg ? (int)0x80000000 : 0;
     const int sc0 = ea - 2 * 1022 - 70 + 36 + g.alpha_k;
 #pragma unroll
     for (int j = 0; j < HB; ++j) {
         const int eb = colE[j];
-        bad |= eb != 0 && ((unsigned)(eb - E_MIN) > (unsigned)(E_MAX - E_MIN) ||
-                           (live && mag[j] > 0.0f && mag[j] < MAG_MIN));
+        if (eb != 0 && ((unsigned)(eb - E_MIN) > (unsigned)(E_MAX - E_MIN) ||
+                        (live && mag[j] > 0.0f && mag[j] < MAG_MIN)))
+            left |= 1u << j;
         int up = 0;
         const double v = __ll2double_rn(LOW ? e64_join(hi[j], lo[j], up) : hi[j]);   // 0 for a zero row or column
         const int vh = __double2hiint(v);
@@ -150,13 +151,30 @@ __device__ __forceinline__ bool e64_finish(const E64Out &g, long long (&hi)[HB],
 #pragma unroll
         for (int j = 0; j < HB; ++j) hi[j] = __double_as_longlong(g.alpha * __longlong_as_double(hi[j]));
     }
-    return bad;
+    return left;
 }
 
-// store one thread's row through the output modes (co: column offsets, -1 past N)
+// store one thread's row through the output modes (co: column offsets, -1 past N), without the columns left out
+template <bool LEFT>
 __device__ __forceinline__ void e64_store(const E64Out &g, const long long (&val)[HB], const long long *co,
-                                          long long rowoff) {
+                                          long long rowoff, unsigned left) {
     double *out = g.C + rowoff;
+    if constexpr (LEFT) {
+        for (int j = 0; j < HB; ++j) {
+            if (co[j] < 0 || (left >> j & 1)) continue;
+            long long x = val[0];   // no dynamic index into registers
+#pragma unroll
+            for (int i = 1; i < HB; ++i) x = i == j ? val[i] : x;
+            const double v = __longlong_as_double(x);
+            if (g.beta_mode == 0)
+                out[co[j]] = v;
+            else if (g.beta_mode == 1)
+                red_add_f64(out + co[j], v);
+            else
+                out[co[j]] = g.beta_mode == 2 ? g.Cin[rowoff + co[j]] + v : fma(g.beta, g.Cin[rowoff + co[j]], v);
+        }
+        return;
+    }
     if (g.beta_mode == 0) {
 #pragma unroll
         for (int j = 0; j < HB; ++j)
@@ -180,15 +198,18 @@ __device__ __forceinline__ void e64_store(const E64Out &g, const long long (&val
     }
 }
 
-// tiles are listed by halves (16 columns), the unit of a vote
-__device__ __forceinline__ void e64_list_tile(const E64Out &g, int prob, int m0, int n0) {
-    const long long t = (g.row0 + m0) / BM + g.mtiles_all * (n0 / VN);
-    const int at = atomicAdd(g.list, 1);
-    g.list[1 + 2 * at] = prob;
-    g.list[2 + 2 * at] = (int)t;
+// barrier over the 256 drain threads of one half (named barrier 1 or 2) that counts, or ORs, a predicate over them
+__device__ __forceinline__ unsigned vote_count(int half, bool pred) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.u32 p, %1, 0;\n\t"
+        "bar.red.popc.u32 %0, %3, %2, p;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)pred), "n"(DRAIN / 2), "r"(half + 1)
+        : "memory");
+    return r;
 }
-
-// barrier over the 256 drain threads of one half (named barrier 1 or 2) that ORs a predicate over them
 __device__ __forceinline__ bool vote_any(int half, bool pred) {
     uint32_t r;
     asm volatile(
@@ -200,6 +221,46 @@ __device__ __forceinline__ bool vote_any(int half, bool pred) {
         : "r"((uint32_t)pred), "n"(DRAIN / 2), "r"(half + 1)
         : "memory");
     return r != 0;
+}
+
+// A half tile (16 columns, the unit of a vote) of which n > 0 threads left columns out: listed whole, or where they
+// are few, piece by piece; the caller stores the rest of a half tile listed by pieces (true).  lost: a thread's
+// sums are not there (a failed wait): nothing of the half tile is listed or stored, the host reports the time-out.
+// slot: two ints of shared memory of the half's own, free again at its next vote.
+__device__ __forceinline__ bool e64_list_half(const E64Out &g, int prob, int m0, int n0, int half, unsigned n, unsigned left,
+                                              bool lost, int row, int group, bool first, int *slot) {
+    const int t = (int)((g.row0 + m0) / BM + g.mtiles_all * (n0 / VN));
+    if (n > E64_FINE) {
+        if (!vote_any(half, lost) && first && n0 < g.N) {
+            const int at = atomicAdd(g.list, 1);
+            g.list[2 + 2 * (long long)at] = prob;
+            g.list[3 + 2 * (long long)at] = t;
+        }
+        return false;
+    }
+    if (first) {
+        slot[0] = atomicAdd(g.list + 1, 1);
+        slot[1] = 0;
+    }
+    __syncwarp();
+    const bool none = vote_any(half, lost);
+    int *f = g.fine + (long long)slot[0] * E64_FINE_INTS;
+    if (first) {
+        f[0] = prob;
+        f[1] = t;
+        f[2] = none ? 0 : (int)n;
+    }
+    __syncwarp();
+    if (none) return false;
+    const unsigned who = __ballot_sync(0xffffffffu, left != 0);
+    if (who) {
+        const int lane = threadIdx.x & 31, lead = __ffs(who) - 1;
+        int at = 0;
+        if (lane == lead) at = atomicAdd(slot + 1, __popc(who));
+        at = __shfl_sync(0xffffffffu, at, lead) + __popc(who & ((1u << lane) - 1));
+        if (left) reinterpret_cast<uint16_t *>(f + 3)[at] = (uint16_t)(row | group << 7 | left << 8);
+    }
+    return true;
 }
 
 // acc += integer(x) 2^sh, x the bits of an integer-valued FP32 sum
@@ -234,6 +295,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint64_t *ifull = fin + 1;           // [ITEMS] an item's place is in the queue
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ifull + ITEMS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    int *slots = reinterpret_cast<int *>(tmem_slot + 2);   // two ints per half (e64_list_half)
     int4 *queue = reinterpret_cast<int4 *>(smem + RING_BYTES + BAR_BYTES);   // [ITEMS] m0, n0, chunks, problem | part
     Tables *tabs = reinterpret_cast<Tables *>(queue + ITEMS);                // three sets per half
 
@@ -516,12 +578,14 @@ __global__ void __launch_bounds__(THREADS, 1)
                 }
                 continue;
             }
-            const bool left = e64_finish<(PL > 3)>(g, hi, lo, mag, T.rowE[row], T.colE + sub);
-            if (vote_any(half, left || bad)) {
-                // after a failed wait nothing is listed: the host reports the time-out
-                if (dt == 0 && *abort_flag == 0 && n0 < g.N) e64_list_tile(g, GROUPED ? at : 0, m0, n0);
-            } else if (T.rowoff[row] >= 0) {
-                e64_store(g, hi, T.coloff + sub, T.rowoff[row]);
+            const unsigned left = e64_finish<(PL > 3)>(g, hi, lo, mag, T.rowE[row], T.colE + sub);
+            const unsigned n = vote_count(half, left || bad);
+            if (n == 0) {
+                if (T.rowoff[row] >= 0) e64_store<false>(g, hi, T.coloff + sub, T.rowoff[row], 0u);
+            } else if (e64_list_half(g, GROUPED ? at : 0, m0, n0, half, n, left, bad, row, sub / HB, dt == 0,
+                                     slots + 2 * half) &&
+                       T.rowoff[row] >= 0) {
+                e64_store<true>(g, hi, T.coloff + sub, T.rowoff[row], left);
             }
         }
         const bool ok = !bad;
@@ -565,7 +629,7 @@ __global__ void __launch_bounds__(256) e64_fold_kernel(longlong2 *__restrict__ p
 // and finishes the tile as the main kernel does
 __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g, int step) {
     __shared__ long long coloff[BN];
-    __shared__ int colE[BN];
+    __shared__ int colE[BN], slots[4];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int quarter = warp & 3, eighth = warp >> 2, half = eighth >> 1;
     const int tile = blockIdx.x, tiles = g.mtiles * g.ntiles;
@@ -597,11 +661,14 @@ __global__ void __launch_bounds__(DRAIN) e64_parts_kernel(const E64Args g, int s
         }
     }
     __syncthreads();
-    const bool left = e64_finish<true>(g, hi, lo, mag, ea, colE + eighth * HB);
-    if (vote_any(half, left)) {
-        if ((threadIdx.x & 255) == 0 && n0 + half * VN < g.N) e64_list_tile(g, 0, m0, n0 + half * VN);
-    } else if (mrow < g.M) {
-        e64_store(g, hi, coloff + eighth * HB, mode_off(g.mC, g.row0 + mrow));
+    const unsigned left = e64_finish<true>(g, hi, lo, mag, ea, colE + eighth * HB);
+    const unsigned n = vote_count(half, left != 0);
+    if (n == 0) {
+        if (mrow < g.M) e64_store<false>(g, hi, coloff + eighth * HB, mode_off(g.mC, g.row0 + mrow), 0u);
+    } else if (e64_list_half(g, 0, m0, n0 + half * VN, half, n, left, false, quarter * 32 + lane, eighth & 1,
+                             (threadIdx.x & 255) == 0, slots + 2 * half) &&
+               mrow < g.M) {
+        e64_store<true>(g, hi, coloff + eighth * HB, mode_off(g.mC, g.row0 + mrow), left);
     }
 }
 
@@ -1089,7 +1156,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
                 grow(ctx, pc.e64_planes[1], hB);
                 grow(ctx, pc.e64_exps[1], (size_t)Nall);
             }
-            grow(ctx, pc.e64_list, (size_t)(4 * mtiles_all * ntiles + 1));
+            grow(ctx, pc.e64_list, e64_list_ints(mtiles_all * ntiles));
             if (ksplit > 1)   // the parts' sums, then their magnitudes
                 part = static_cast<longlong2 *>(ctx->splitk_scratch((size_t)ksplit * panel_tiles * BM * BN *
                                                                     (sizeof(longlong2) + sizeof(float))));
@@ -1121,7 +1188,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
 
     __half *planesB = eB ? eB->buf.p : newB ? newB->buf.p : pc.e64_planes[1].p;
     int *expsB = eB ? eB->exps.p : newB ? newB->exps.p : pc.e64_exps[1].p;
-    JUES_CHECK_CUDA(cudaMemsetAsync(pc.e64_list.p, 0, sizeof(int), ctx->stream));
+    JUES_CHECK_CUDA(cudaMemsetAsync(pc.e64_list.p, 0, 2 * sizeof(int), ctx->stream));
     for (long long r0 = 0; r0 < a.M; r0 += prow) {
         const long long R = std::min(prow, a.M - r0), Rpad = roundup(R, BM);
         __half *planesA = eA ? eA->buf.p : newA ? newA->buf.p : pc.e64_planes[0].p;
@@ -1148,6 +1215,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
         g.part = part;
         g.pmag = reinterpret_cast<float *>(part + (size_t)ksplit * g.mtiles * g.ntiles * BM * BN);
         g.list = pc.e64_list.p;
+        g.fine = g.list + 2 + 4 * mtiles_all * ntiles;
         const CUtensorMap ma = plane_map(planesA, Rpad, Kpad, NP, BM, 1), mb = plane_map(planesB, Nall, Kpad, NP, BN, NP),
                           xa = mag_map(planesA, Rpad, Kpad, NP, BM), xb = mag_map(planesB, Nall, Kpad, NP, BN);
         const long long items = e64_items(g);
@@ -1175,7 +1243,7 @@ bool gett_e64(Ctx *ctx, const GettArgs &a0, const char *name) {
     }
     if (newA) pc.cached.push_back(std::move(newA));
     if (newB) pc.cached.push_back(std::move(newB));
-    gett_f64_tiles(ctx, &a, nullptr, pc.e64_list.p, name);
+    gett_f64_tiles(ctx, &a, nullptr, pc.e64_list.p, mtiles_all * ntiles, name);
     return true;
 }
 
@@ -1206,7 +1274,7 @@ void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const M
 
 E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long K, long long rowA, long long M,
                     long long rowB, long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
-                    int *list) {
+                    int *list, long long list_tiles) {
     E64Args g{};
     g.M = M; g.N = N; g.row0 = 0;
     g.rowA = (int)rowA; g.rowB = (int)rowB; g.item0 = item0;
@@ -1221,18 +1289,19 @@ E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long 
     g.part = nullptr;
     g.pmag = nullptr;
     g.list = list;
+    g.fine = list ? list + 2 + 4 * list_tiles : nullptr;
     return g;
 }
 
 void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Args *probs, const GroupProblem *f64,
-                   int n, long long items, int *list, const char *name) {
+                   int n, long long items, int *list, long long list_tiles, const char *name) {
     if (n <= 0 || items <= 0) return;
     JUES_REQUIRE(A.np == B.np && A.Kpad == B.Kpad && items < (1LL << 31), "mismatched planes");
     const CUtensorMap ma = plane_map(A.planes.p, A.rows, A.Kpad, A.np, BM, 1),
                       mb = plane_map(B.planes.p, B.rows, B.Kpad, B.np, BN, B.np),
                       xa = mag_map(A.planes.p, A.rows, A.Kpad, A.np, BM),
                       xb = mag_map(B.planes.p, B.rows, B.Kpad, B.np, BN);
-    JUES_CHECK_CUDA(cudaMemsetAsync(list, 0, sizeof(int), ctx->stream));
+    JUES_CHECK_CUDA(cudaMemsetAsync(list, 0, 2 * sizeof(int), ctx->stream));
     E64Args g{};
     g.flags = ctx->d_flags;
     const unsigned grid = (unsigned)std::min<long long>(items, 152);
@@ -1247,7 +1316,7 @@ void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Ar
         }
         JUES_CHECK_CUDA(cudaGetLastError());
     }
-    gett_f64_tiles(ctx, nullptr, f64, list, name);
+    gett_f64_tiles(ctx, nullptr, f64, list, list_tiles, name);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1262,6 +1331,7 @@ struct E64Group {
     DBuf<PackArgs> ops;
     DBuf<unsigned> first;
     int *list = nullptr;
+    long long list_tiles = 0;
     int nprob = 0, nops = 0;
     unsigned blocks = 0;
     long long items = 0;
@@ -1275,7 +1345,8 @@ struct StageShape {
     long long kmax = 0, kpad = 0, pr = 0, rows[2] = {0, 0}, items = 0;
     size_t halves(int side) const { return plane_halves(NP, rows[side], kpad); }
     size_t bytes() const {
-        return (halves(0) + halves(1)) * sizeof(__half) + (size_t)(rows[0] + rows[1] + 4 * items + 1) * sizeof(int);
+        return (halves(0) + halves(1)) * sizeof(__half) +
+               ((size_t)(rows[0] + rows[1]) + e64_list_ints(items)) * sizeof(int);
     }
 };
 
@@ -1321,20 +1392,22 @@ void e64_shared_reserve(Ctx *ctx, E64Shared &sh, const std::vector<const std::ve
     }
     std::sort(fit.begin(), fit.end(), [](const StageShape &a, const StageShape &b) { return a.bytes() < b.bytes(); });
     for (; !fit.empty(); fit.pop_back()) {   // without its largest stage where that does not fit
-        size_t halves[2] = {0, 0}, rows[2] = {0, 0}, items = 0;
+        size_t halves[2] = {0, 0}, rows[2] = {0, 0};
+        long long items = 0;
         for (const StageShape &s : fit) {
             for (int k = 0; k < 2; ++k) {
                 halves[k] = std::max(halves[k], s.halves(k));
                 rows[k] = std::max(rows[k], (size_t)s.rows[k]);
             }
-            items = std::max(items, (size_t)s.items);
+            items = std::max(items, s.items);
         }
         try {
             for (int k = 0; k < 2; ++k) {
                 grow(ctx, sh.planes[k], halves[k]);
                 grow(ctx, sh.exps[k], rows[k]);
             }
-            grow(ctx, sh.list, 4 * items + 1);
+            grow(ctx, sh.list, e64_list_ints(items));
+            sh.list_tiles = items;
             return;
         } catch (const Error &e) {
             if (e.code != JUES_ENOMEM) throw;   // the FP64 tiles need no planes
@@ -1348,12 +1421,13 @@ E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const E64Sh
     if (!stage_shape(in, s)) return nullptr;
     for (int k = 0; k < 2; ++k)
         if (sh.planes[k].n < s.halves(k) || sh.exps[k].n < (size_t)s.rows[k]) return nullptr;
-    if (sh.list.n < (size_t)(4 * s.items + 1)) return nullptr;
+    if (sh.list_tiles < s.items) return nullptr;
     try {
         std::unique_ptr<E64Group> g(new E64Group());
         g->name = name;
         g->items = s.items;
         g->list = sh.list.p;
+        g->list_tiles = sh.list_tiles;
         const long long pr = s.pr;
         for (int k = 0; k < 2; ++k) {
             E64Planes &P = k ? g->B : g->A;
@@ -1381,7 +1455,7 @@ E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &in, const E64Sh
             pack(g->A, ra, a.A, a.mA, a.kA, a.M, a.K);
             pack(g->B, rb, a.B, a.nB, a.kB, a.N, a.K);
             args.push_back(e64_problem(ctx, g->A, g->B, a.K, ra, a.M, rb, a.N, a.alpha, a.beta, a.C, a.mC, a.nC, (int)at,
-                                       g->list));
+                                       g->list, g->list_tiles));
             f64.push_back(to_problem(a));
             ra += roundup(a.M, pr);
             rb += roundup(a.N, pr);
@@ -1417,7 +1491,7 @@ void e64_group_exec(Ctx *ctx, E64Group *g) {
             e64_pack_grouped_kernel<NP, 128><<<g->blocks, 256, 0, ctx->stream>>>(g->ops.p, g->first.p, g->nops);
         JUES_CHECK_CUDA(cudaGetLastError());
     }
-    e64_group_run(ctx, g->A, g->B, g->args.p, g->f64.p, g->nprob, g->items, g->list, g->name.c_str());
+    e64_group_run(ctx, g->A, g->B, g->args.p, g->f64.p, g->nprob, g->items, g->list, g->list_tiles, g->name.c_str());
 }
 
 void e64_group_destroy(E64Group *g) { delete g; }

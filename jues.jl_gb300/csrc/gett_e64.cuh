@@ -11,12 +11,18 @@ namespace jues {
 // the memory left do not suit it and the FP64 pipe should run the contraction
 bool gett_e64(Ctx *ctx, const GettArgs &a, const char *name);
 
+// Results left to the FP64 pipe, in ints: the counts of whole half tiles (128 x 16) and of half tiles with few
+// elements left out, (problem, tile) pairs of the first, then E64_FINE_INTS for each of the second: problem, tile,
+// count of pieces, and the pieces, a row's eight columns each: row | column group << 7 | left-out columns << 8
+constexpr int E64_FINE = 64, E64_FINE_INTS = 3 + E64_FINE / 2;
+inline size_t e64_list_ints(long long tiles) { return 2 + 2 * (size_t)tiles * (2 + E64_FINE_INTS); }   // of 128 x 32
+
 // where and how the results of one contraction are stored
 struct E64Out {
     double alpha, beta;
     double *C;
     const double *Cin;
-    int *list;                  // tiles left to the FP64 pipe: count, then (problem, tile) pairs
+    int *list, *fine;           // results left to the FP64 pipe; the half tiles with few of them
     long long row0;             // first row of the panel in the whole output
     long long mtiles_all;       // row tiles of the whole output (tile numbers in the list)
     long long N;                // columns
@@ -53,12 +59,12 @@ void e64_pack(Ctx *ctx, E64Planes &P, const double *src, const Mode &rm, const M
 // the problems before it in the launch (e64_tiles each)
 E64Args e64_problem(Ctx *ctx, const E64Planes &A, const E64Planes &B, long long K, long long rowA, long long M,
                     long long rowB, long long N, double alpha, double beta, double *C, const Mode &mC, const Mode &nC, int item0,
-                    int *list);
+                    int *list, long long list_tiles);
 inline long long e64_tiles(long long M, long long N) { return ((M + 127) / 128) * ((N + 31) / 32); }
 // one launch over n problems (device tables: probs, and f64 the same contractions for the FP64 pipe);
-// list holds 4 items + 1 ints
+// list has room for list_tiles >= items tiles (as the problems were told)
 void e64_group_run(Ctx *ctx, const E64Planes &A, const E64Planes &B, const E64Args *probs, const GroupProblem *f64,
-                   int n, long long items, int *list, const char *name);
+                   int n, long long items, int *list, long long list_tiles, const char *name);
 
 // A stage of a batch (K <= 128 throughout).  Stages run one after another, so their operands go through one
 // set of planes: reserve sizes it for the largest of the stages that suit it and fit the memory left; build gives
@@ -67,15 +73,17 @@ struct E64Group;
 struct E64Shared {
     DBuf<__half> planes[2];
     DBuf<int> exps[2], list;
+    long long list_tiles = 0;
 };
 void e64_shared_reserve(Ctx *ctx, E64Shared &sh, const std::vector<const std::vector<GettArgs> *> &stages);
 E64Group *e64_group_build(Ctx *ctx, const std::vector<GettArgs> &probs, const E64Shared &sh, const char *name);
 void e64_group_exec(Ctx *ctx, E64Group *g);
 void e64_group_destroy(E64Group *g);
 
-// gett_f64.cu: recompute the listed output tiles on the FP64 pipe.  list[0] = count, then pairs
-// (problem, tile t): rows [128 (t % mt), + 128), columns [16 (t / mt), + 16) of the problem's output, mt =
-// its 128-row tiles; the problem is *one, or probs[problem] (device)
-void gett_f64_tiles(Ctx *ctx, const GettArgs *one, const GroupProblem *probs, const int *list, const char *name);
+// gett_f64.cu: recompute the listed results on the FP64 pipe.  Tile t of a problem is its rows
+// [128 (t % mt), + 128), columns [16 (t / mt), + 16), mt = its 128-row tiles; the problem is *one, or probs[problem]
+// (device)
+void gett_f64_tiles(Ctx *ctx, const GettArgs *one, const GroupProblem *probs, const int *list, long long list_tiles,
+                    const char *name);
 
 }  // namespace jues

@@ -234,21 +234,84 @@ struct ModeIter {
     }
 };
 
-// The tiles the tensor-core form left out (gett_e64.cu): an entry is a 128 x 16 tile of one problem.  The
-// list is nearly always empty; a long one runs as 64 x 16 tiles, a shorter one as 16 x 16, and one of up to 16
-// entries with a warp to two outputs: FP64 issue bounds a block's 16 x 16 K products, and eight such blocks leave
-// the other SMs idle (K = 3240, one, four and sixteen entries: 455, 450 and 467 us as 16 x 16, now 82, 147 and 299).
+// What the tensor-core form left out (gett_e64.cu).  Half tiles with few elements left out: a block each (several
+// where there are few of them), four lanes to an element.  An element costs 2.3 times what it does in a whole tile,
+// so half tiles go this way up to a quarter of their pieces (MP2 of s functions on a chain, nbf = 96, first quarter:
+// 4.21 -> 2.95 ms).  Whole ones, 128 x 16 of one problem: a long list runs as 64 x 16 tiles, a shorter one as
+// 16 x 16, and one of up to 16 entries with a warp to two outputs: FP64 issue bounds a block's 16 x 16 K
+// products, and eight such blocks leave the other SMs idle (K = 3240, one, four and sixteen entries: 455, 450 and 467
+// us as 16 x 16, now 82, 147 and 299).  Both lists are nearly always empty.
 __global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(const GroupProblem one,
                                                             const GroupProblem *__restrict__ probs,
-                                                            const int *__restrict__ list) {
+                                                            const int *__restrict__ list,
+                                                            const int *__restrict__ fine) {
     __shared__ TileSmem<64, 16> sm;
-    const int n = list[0];
+    const int n = list[0], nf = list[1];
+    // a block each, or as many as there are blocks for
+    const int shares = nf ? max(1, min(32, (int)gridDim.x / nf)) : 1;
+    for (long long x = blockIdx.x; x < (long long)nf * shares; x += gridDim.x) {
+        const long long d = x / shares;
+        const int share = (int)(x % shares);
+        __shared__ unsigned short elem[8 * E64_FINE];   // row | column << 7
+        __shared__ int sums[NT / 32];
+        const int *f = fine + d * E64_FINE_INTS;
+        const GroupProblem &g = probs ? probs[f[0]] : one;
+        const long long mt128 = (g.M + 127) / 128, m0 = f[1] % mt128 * 128, n0 = f[1] / mt128 * 16;
+        const int tid = threadIdx.x, lane = tid & 31;
+        __syncthreads();
+        // the pieces' elements, in the order of the list (every block that shares it takes others of them)
+        const unsigned piece = tid < f[2] ? reinterpret_cast<const unsigned short *>(f + 3)[tid] : 0u;
+        int at = __popc(piece >> 8), ne = 0;
+#pragma unroll
+        for (int i = 1; i < 32; i <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, at, i);
+            if (lane >= i) at += y;
+        }
+        if (lane == 31) sums[tid >> 5] = at;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < NT / 32; ++i) {
+            if (i == tid >> 5) at += ne;
+            ne += sums[i];
+        }
+        at -= __popc(piece >> 8);
+        for (int j = 0; j < 8; ++j)
+            if (piece >> (8 + j) & 1) elem[at++] = (unsigned short)((piece & 127) | ((piece >> 7 & 1) * 8 + j) << 7);
+        __syncthreads();
+        for (int e0 = share * (NT / 4) + (tid >> 5) * 8; e0 < ne; e0 += shares * (NT / 4)) {
+            const int e = min(e0 + (lane & 7), ne - 1), part = lane >> 3;
+            const long long m = m0 + (elem[e] & 127), c = n0 + (elem[e] >> 7);
+            const bool in = m < g.M && c < g.N;
+            double acc = 0.0;
+            if (in) {
+                const double *pa = g.A + mode_off(g.mA, m), *pb = g.B + mode_off(g.nB, c);
+                ModeIter ia, ib;
+                ia.init(g.kA, part);
+                ib.init(g.kB, part);
+#pragma unroll 4
+                for (long long k = part; k < g.K; k += 4) {
+                    acc = fma(__ldg(pa + ia.off), __ldg(pb + ib.off), acc);
+                    ia.step(g.kA, 4);
+                    ib.step(g.kB, 4);
+                }
+            }
+            __syncwarp();
+            acc += __shfl_xor_sync(0xffffffffu, acc, 8);
+            acc += __shfl_xor_sync(0xffffffffu, acc, 16);
+            if (part == 0 && in && e0 + lane < ne) {
+                const long long off = mode_off(g.mC, m) + mode_off(g.nC, c);
+                double v = g.alpha * acc;
+                if (g.beta != 0.0) v = fma(g.beta, g.Cin[off], v);
+                g.C[off] = v;
+            }
+        }
+    }
     if (n <= 16) {
         const int lane = threadIdx.x & 31;
         for (int w = (blockIdx.x * NT + threadIdx.x) >> 5; w < n * 1024; w += gridDim.x * (NT / 32)) {
             const int e = w >> 10;
-            const GroupProblem &g = probs ? probs[list[1 + 2 * e]] : one;
-            const long long t = list[2 + 2 * e], mt128 = (g.M + 127) / 128;
+            const GroupProblem &g = probs ? probs[list[2 + 2 * e]] : one;
+            const long long t = list[3 + 2 * e], mt128 = (g.M + 127) / 128;
             const long long m = t % mt128 * 128 + (w & 127), n0 = t / mt128 * 16 + 2 * (w >> 7 & 7);
             if (m >= g.M || n0 >= g.N) continue;
             const long long n1 = n0 + 1 < g.N ? n0 + 1 : n0;
@@ -282,8 +345,8 @@ __global__ void __launch_bounds__(NT) gett_f64_tiles_kernel(const GroupProblem o
     const int sub = n <= 512 ? 8 : 2, rows = 128 / sub;
     for (int x = blockIdx.x; x < n * sub; x += gridDim.x) {
         const int e = x / sub;
-        GroupProblem g = probs ? probs[list[1 + 2 * e]] : one;
-        const long long t = list[2 + 2 * e], mt128 = (g.M + 127) / 128;
+        GroupProblem g = probs ? probs[list[2 + 2 * e]] : one;
+        const long long t = list[3 + 2 * e], mt128 = (g.M + 127) / 128;
         const long long mt = sub * (t % mt128) + x % sub;
         g.mtiles = (g.M + rows - 1) / rows;
         if (mt >= g.mtiles) continue;
@@ -572,12 +635,13 @@ GroupProblem to_problem(const GettArgs &a) {
     return g;
 }
 
-void gett_f64_tiles(Ctx *ctx, const GettArgs *one, const GroupProblem *probs, const int *list, const char *name) {
+void gett_f64_tiles(Ctx *ctx, const GettArgs *one, const GroupProblem *probs, const int *list, long long list_tiles,
+                    const char *name) {
     GroupProblem g{};
     if (one) g = to_problem(*one);
     const std::string nm = std::string(name) + ".rest";
     Ctx::Scope s(ctx, nm.c_str());
-    gett_f64_tiles_kernel<<<152 * 4, NT, 0, ctx->stream>>>(g, probs, list);
+    gett_f64_tiles_kernel<<<152 * 4, NT, 0, ctx->stream>>>(g, probs, list, list + 2 + 4 * list_tiles);
     JUES_CHECK_CUDA(cudaGetLastError());
 }
 

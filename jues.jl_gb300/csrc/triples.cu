@@ -400,12 +400,12 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
     std::vector<E64Args> args;
     std::vector<GroupProblem> probs;
     std::vector<long long> nitem;   // GEMM items of each launch
+    long long most_items = 0;
     try {
         W = DBuf<double>(ctx, (size_t)(v3 * wmax));
         const int np = prec == JUES_PREC_SPLIT || prec == JUES_PREC_SPLIT2 ? 3 : 7;
         st.reset(new PtStacks(ctx, np, T2, Vv, Vo, o, v));
-        long long most_items = 0;
-        auto build = [&](int *lp) {
+        auto build = [&](int *lp, long long lt) {
             args.clear();
             probs.clear();
             nitem.clear();
@@ -417,7 +417,7 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
                     for (int p = 0; p < b.npair; ++p) {
                         const PtTerm m = pt_term(t, i, j, o, v);
                         args.push_back(e64_problem(ctx, st->pr, st->pq, st->K, m.rowA, m.M, m.rowB, m.N, st->unscale, t ? 1.0 : 0.0,
-                                                   W.p + w0, m.mC, m.nC, (int)n, lp));
+                                                   W.p + w0, m.mC, m.nC, (int)n, lp, lt));
                         GettArgs g;
                         g.M = m.M; g.N = m.N; g.K = st->K;
                         g.alpha = st->unscale; g.beta = t ? 1.0 : 0.0;
@@ -433,9 +433,9 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
                     most_items = std::max(most_items, n);
                 }
         };
-        build(nullptr);
-        list = DBuf<int>(ctx, (size_t)(4 * most_items + 1));
-        build(list.p);
+        build(nullptr, 0);
+        list = DBuf<int>(ctx, e64_list_ints(most_items));
+        build(list.p, most_items);
         dargs = DBuf<E64Args>(ctx, args.size());
         dprobs = DBuf<GroupProblem>(ctx, probs.size());
         JUES_CHECK_CUDA(cudaMemcpyAsync(dargs.p, args.data(), args.size() * sizeof(E64Args), cudaMemcpyHostToDevice,
@@ -454,7 +454,8 @@ double pT_energy(Ctx *ctx, int prec, const double *T1, const double *T2, const V
         size_t at = 0, launch = 0;
         for (const Batch &b : batches) {
             for (int t = 0; t < 6; ++t, ++launch) {
-                e64_group_run(ctx, st->pr, st->pq, dargs.p + at, dprobs.p + at, b.npair, nitem[launch], list.p, "pt_w");
+                e64_group_run(ctx, st->pr, st->pq, dargs.p + at, dprobs.p + at, b.npair, nitem[launch], list.p, most_items,
+                              "pt_w");
                 at += (size_t)b.npair;
             }
             energy(ctx, W.p, items.p + b.item0, b.nitems, tiles, T1, Vvovo, fo, fv, o, v, slots.p);

@@ -77,3 +77,25 @@ def test_every_tile_left_out():
     want[:, 1::2] = exact(x * 2.0 ** 40, B[30:, 1::2]) * np.longdouble(2.0 ** -40)
     got = _lib.gemm(A, B, precision="fp64")
     assert np.all(np.abs((got - want).astype(float)) <= 65 * U * (np.abs(A) @ np.abs(B)))
+
+
+# few elements of a half tile below the line (listed one by one), with every way of storing the others; 41 rows apart,
+# so that pieces of both column groups and of the last, short row and column tiles are among them
+@pytest.mark.parametrize("M,N,K", [(1300, 83, 100), (400, 150, 300), (200, 70, 6000)])
+@pytest.mark.parametrize("alpha,beta", [(1.0, 0.0), (-2.0, 1.0), (0.3, -0.7)])
+@pytest.mark.parametrize("transB", [False, True])
+def test_few_elements_left_out(M, N, K, alpha, beta, transB):
+    from juesgpu import _lib
+    rng = np.random.default_rng(M + N + K)
+    A, B, want = operands(M, N, K, 2.0 ** -40, 41, rng)
+    A[-1], want[-1] = 0.0, 0.0
+    C0 = rng.normal(size=(M, N))
+    got = _lib.gemm(A, np.asfortranarray(B.T) if transB else B, C=C0, alpha=alpha, beta=beta, transB=transB,
+                    precision="fp64")
+    full = np.longdouble(alpha) * want + np.longdouble(beta) * C0.astype(np.longdouble)
+    mag = abs(alpha) * (np.abs(A) @ np.abs(B)) + abs(beta) * np.abs(C0)
+    assert np.all(np.abs((got - full).astype(float)) <= (K + 5) * U * mag)
+    # and with beta = 0 the small elements keep their own bound beside the large ones
+    if beta == 0.0:
+        low = want[::41, 1::41]
+        assert np.all(np.abs((got[::41, 1::41] - alpha * low).astype(float)) <= (K + 5) * U * mag[::41, 1::41])
