@@ -57,7 +57,9 @@ extern "C" {
  * keep ~2^-24, the FP32 rounding of the chunk sums. */
 #define JUES_PREC_FP64 0       /* plain FP64 (the drop-in form): contractions of 3e6 flop and more run on the
                                   tensor cores as exact sums of 9-bit digit products, rounded once; the
-                                  others, and tiles whose operands do not suit that, as FP64 FMAs  */
+                                  others, and every element whose sum of magnitudes lies below 2^-7 of its
+                                  row's and column's largest, as FP64 FMAs.  Each element keeps an FMA loop's
+                                  bound, (K + 5) 2^-53 sum |a_k b_k| */
 #define JUES_PREC_SPLIT 1      /* the split form at <= 1 uEh: three planes for every contraction
                                   that produces integrals (four-index transforms, get_eri blocks,
                                   DF factors, the MP2 adjoint's back-transforms), two planes for
@@ -211,7 +213,7 @@ JUES_API int jues_rmp2_adjoint(jues_ctx *ctx, const double *gao, int n, const do
  * systems of uneven size.  All systems run in one CUDA graph of grouped persistent launches (one
  * per stage, 12 stages with the adjoint); the graph is cached for a repeated batch signature.
  * precision: JUES_PREC_FP64 runs every stage as a grouped FP64 GETT, on the tensor cores (exact
- * digit products) where the stage is large enough; the split forms add, for
+ * digit products) where that is faster on the batch at hand; the split forms add, for
  * every stage whose contractions all have K <= 64 (all but the final dE/dC stage when every
  * nbf <= 64), the grouped three-plane tcgen05 GEMM as a candidate.  On first use each stage's
  * form is chosen by timing the candidates (autotuning).  Host arrays; gao_bar / C_bar are arrays

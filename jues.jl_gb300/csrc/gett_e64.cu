@@ -29,17 +29,19 @@
 // nonzero element in common, and the result is exactly 0.  Against exact products, relative Frobenius error for normal entries:
 // 4.7e-17 at every size, the FMA kernels 1.3e-16 (K = 100) to 8.4e-16 (640^3).
 //
-// Speed (packs included): 6400^3 11.2 ms = 47 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.26 against
-// 8.1 ms, 500000 x 100 x 100 0.80 against 11.8 ms.  The magnitudes cost 7 % of that at long K (as a second
-// FP16 plane they cost 15 %).  At K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about 8000
-// clocks a tile) bounds it.
+// Speed (packs included): 6400^3 11.5 ms = 46 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.27 against
+// 8.1 ms, 500000 x 100 x 100 0.82 against 11.8 ms.  The magnitudes cost 8 to 12 % of that at long K (as an FP16 plane
+// they cost 15 % and more; leaving them out of a tile's later chunks once its elements have enough made the MMA
+// loop slower than the loads gained).  At K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about
+// 8000 clocks a tile) bounds it.
 //
 // The tile is 128 x 32: TMEM holds two buffers of 8 x 32 FP32 columns (seven digit sums and the magnitudes), so
 // the drain of one chunk overlaps the MMAs of the next; a wider tile would need TMEM that is not there.  At long K
-// shared memory paces: a chunk's MMAs read 240 KB of it (with N = 32 per plane an instruction takes 4 KB of A
-// and 1 to 7 KB of B for 16 to 112 clocks) and TMA writes 154 KB, 3070 clocks at 128 bytes a clock (measured 3040),
-// against 1820 clocks of MMA at the dense rate.  A's planes arrive one by one (64 K values x 128 rows, 16 KB,
-// 128-byte swizzle; the magnitudes 8 KB, 64-byte swizzle) in a ring of nine, B's together.
+// moving the operands paces: 150 KB a chunk from L2 (13.8 TB/s over all SMs), and shared memory, of which the chunk's
+// MMAs read 240 KB (with N = 32 per plane an instruction takes 4 KB of A and 1 to 7 KB of B for 16 to 112 clocks)
+// while TMA writes those 150, 3070 clocks at 128 bytes a clock against 1820 of MMA at the dense rate.  A's planes
+// arrive one by one (64 K values x 128 rows, 16 KB, 128-byte swizzle; the magnitudes 8 KB, 64-byte swizzle) in a
+// ring of nine, B's together.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -752,7 +754,7 @@ struct PackSmem {
 };
 
 // LOCALMAX: the block sees whole rows (K <= KW) and writes their exponents; else they are read.  Integer issue
-// and the block's three phases bound it: 22 bytes an element (8 read, 14 written) at 3.6 to 4.1 TB/s of 6.7.
+// and the block's three phases bound it: 23 bytes an element (8 read, 15 written) at 3.6 to 4.1 TB/s of 6.7.
 // The digits stay one 64-bit number until two of them are put into an FP16 pair, padded K is skipped, and a
 // thread writes one 16-byte piece of each plane (500000 x 100: 345 -> 305 us; 6400^2: 352 -> 306).
 template <int PL, int KW, bool KFAST, bool LOCALMAX>
