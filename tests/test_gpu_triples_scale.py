@@ -41,3 +41,21 @@ def test_pT_without_amplitudes_or_integrals():
         kw[name] = np.zeros_like(kw[name])
         e = {p: PerturbativeTriples.compute_pT(precision=p, **kw) for p in ("fp64", "split")}
         assert np.isfinite(e["fp64"]) and abs(e["split"] - e["fp64"]) <= 2.0 ** -18 * abs(e["fp64"])
+
+
+@pytest.mark.parametrize("every", [2, 5, 16])
+def test_pT_graded_amplitudes(every):
+    # amplitudes and integrals of some virtual orbitals 2^-14 and 2^-30 times the others': the grouped contractions leave
+    # out single elements and whole half tiles; bounds as at the edges (1e-11 FP64, 1e-6 split)
+    from juesgpu.CoupledCluster import PerturbativeTriples
+    from oracle import triples
+    o, v = 4, 37
+    kw = inputs(o, v, every)
+    d = np.where(np.arange(v) % every == 0, 2.0 ** -14, 1.0)
+    f = np.where(np.arange(v) % every == 1, 2.0 ** -30, 1.0)
+    kw["T1"] = np.asfortranarray(np.random.default_rng(1).normal(size=(o, v)) * 1e-2)
+    kw["T2"] = np.asfortranarray(kw["T2"] * d[:, None] * d)
+    kw["Vvvvo"] = np.asfortranarray(kw["Vvvvo"] * f[:, None, None, None] * f[:, None, None])
+    want = triples.compute_pT(**kw)
+    assert abs(PerturbativeTriples.compute_pT(**kw) - want) <= 1e-11 * abs(want)
+    assert abs(PerturbativeTriples.compute_pT(precision="split", **kw) - want) <= 1e-6 * abs(want)

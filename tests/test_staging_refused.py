@@ -71,7 +71,8 @@ def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("staging")
     src, so = d / "stand_ins.cpp", d / "libstaging.so"
     src.write_text(STAND_INS)
-    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-pthread", "-I", CSRC, "-I", inc, str(src), "-x",
+    # -Bsymbolic: its own stand-ins, also where the process has loaded the CUDA runtime
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-pthread", "-I", CSRC, "-I", inc, str(src), "-x",
                     "c++", os.path.join(CSRC, "staging.cu"), "-o", str(so)], check=True)
     lib = C.CDLL(str(so))
     lib.run.argtypes = [C.c_void_p, C.c_void_p, C.c_longlong, C.c_void_p, C.c_longlong, C.c_int, C.c_int]
