@@ -29,19 +29,19 @@
 // nonzero element in common, and the result is exactly 0.  Against exact products, relative Frobenius error for normal entries:
 // 4.7e-17 at every size, the FMA kernels 1.3e-16 (K = 100) to 8.4e-16 (640^3).
 //
-// Speed (packs included): 6400^3 11.5 ms = 46 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.27 against
-// 8.1 ms, 500000 x 100 x 100 0.82 against 11.8 ms.  The magnitudes cost 8 to 12 % of that at long K (as an FP16 plane
-// they cost 15 % and more; leaving them out of a tile's later chunks once its elements have enough made the MMA
-// loop slower than the loads gained).  At K <= 128 a tile's epilogue (integer issue of the sixteen drain warps, about
-// 8000 clocks a tile) bounds it.
+// Speed (packs included): 6400^3 10.8 ms = 49 TFLOP/s against 420 ms on the FP64 pipe, 1600^3 0.26 against
+// 8.1 ms, 500000 x 100 x 100 0.82 against 11.8 ms.  The magnitudes cost 4 to 7 % of that at long K: they come with B,
+// so the MMA loop has one wait for both (in the ring of A planes they cost 8 to 12 %, as an FP16 plane 15 %), and
+// a tile whose elements all have enough after two chunks loads no more of them (else 7 to 9 %).  At K <= 128 a tile's
+// epilogue (integer issue of the sixteen drain warps, about 8000 clocks a tile) bounds it.
 //
 // The tile is 128 x 32: TMEM holds two buffers of 8 x 32 FP32 columns (seven digit sums and the magnitudes), so
 // the drain of one chunk overlaps the MMAs of the next; a wider tile would need TMEM that is not there.  At long K
-// moving the operands paces: 150 KB a chunk from L2 (13.8 TB/s over all SMs), and shared memory, of which the chunk's
+// moving the operands paces: 140 KB a chunk from L2 (13.8 TB/s over all SMs), and shared memory, of which the chunk's
 // MMAs read 240 KB (with N = 32 per plane an instruction takes 4 KB of A and 1 to 7 KB of B for 16 to 112 clocks)
-// while TMA writes those 150, 3070 clocks at 128 bytes a clock against 1820 of MMA at the dense rate.  A's planes
-// arrive one by one (64 K values x 128 rows, 16 KB, 128-byte swizzle; the magnitudes 8 KB, 64-byte swizzle) in a
-// ring of nine, B's together.
+// while TMA writes those 140, 2990 clocks at 128 bytes a clock against 1820 of MMA at the dense rate.  A's planes
+// arrive one by one (64 K values x 128 rows, 16 KB, 128-byte swizzle) in a ring of eight, B's together with the
+// magnitudes of both (64-byte swizzle).
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -62,9 +62,10 @@ namespace {
 constexpr int NP = E64_NP;            // digit planes of the FP64 form (the kernels take 3 too)
 constexpr int BM = 128, BN = 32;      // output tile
 constexpr int CK = 64;                // K per chunk: 128 bytes of FP16, one swizzle row
-constexpr int SLOTS = 9;              // ring of A planes
+constexpr int SLOTS = 8;              // ring of A planes
 constexpr int A_BYTES = BM * CK * 2;  // one A plane, 16 KB
-constexpr int b_bytes(int np) { return np * BN * CK * 2 + BN * CK; }   // all of B: 30 KB for seven digits
+// all of B and the magnitudes of both: 28 + 2 + 8 KB for seven digits
+constexpr int b_bytes(int np) { return np * BN * CK * 2 + (BN + BM) * CK; }
 // an operand's planes in FP16 words: np digits for each of its rows x kpad elements, then the magnitudes, bytes in
 // rows of whole 32-byte sectors
 constexpr long long mag_pitch(long long kpad) { return (kpad + 31) / 32 * 32; }
@@ -79,6 +80,9 @@ constexpr int THREADS = 576, DRAIN = 512;
 constexpr int HB = BN / 4;            // columns per drain thread
 constexpr int VN = BN / 2;            // columns of a vote: eight drain warps
 constexpr int BAR_BYTES = 512, ITEMS = 8;
+// chunks of an item that load magnitudes whatever they are: the drain warps look at them once, after the second,
+// which they have left when the loads of the sixth begin
+constexpr int MAG_CHUNKS = 5;
 // what the drain warps of one half need of a tile
 struct Tables {
     long long rowoff[BM], coloff[VN];
@@ -298,6 +302,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ifull + ITEMS);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     int *slots = reinterpret_cast<int *>(tmem_slot + 2);   // two ints per half (e64_list_half)
+    int *judged = slots + 4;                               // [ITEMS] drain warps whose elements have enough magnitude
     int4 *queue = reinterpret_cast<int4 *>(smem + RING_BYTES + BAR_BYTES);   // [ITEMS] m0, n0, chunks, problem | part
     Tables *tabs = reinterpret_cast<Tables *>(queue + ITEMS);                // three sets per half
 
@@ -373,20 +378,30 @@ __global__ void __launch_bounds__(THREADS, 1)
                 // free once the MMAs of item ni - 2 are done, whose accumulators item ni - 4 has left.
                 if (!wait(&bempty[gc & 1u], ((gc >> 1) & 1u) ^ 1u)) break;
                 queue[ni % ITEMS] = make_int4(m0, n0, c1 - c0, GROUPED ? cur : part * tiles + tile);
+                judged[ni % ITEMS] = 0;
+                bool mags = true;
                 mbar_arrive(&ifull[ni % ITEMS]);
                 m0 += g.rowA;
                 n0 += g.rowB;
                 for (int c = c0; c < c1 && !stop; ++c, ++gc) {
                     const unsigned b = gc & 1u;
                     if (c > c0 && !wait(&bempty[b], ((gc >> 1) & 1u) ^ 1u)) break;
-                    mbar_expect_tx(&bfull[b], B_BYTES);
-                    tma_load_3d(ringB + b * B_BYTES, &mapB, &bfull[b], c * CK, n0, 0);
-                    tma_load_3d(ringB + b * B_BYTES + PL * BN * CK * 2, &magB, &bfull[b], c * CK, n0, 0);
-                    for (int p = 0; p <= PL; ++p, ++it) {
+                    // Where every element of the tile has enough magnitude the item's further chunks load no more (a
+                    // grouped launch's items are too short): their MMAs add those of an earlier chunk, which
+                    // change nothing.  Read without an order: it decides about time alone.
+                    if (!GROUPED && c == c0 + MAG_CHUNKS) mags = *(volatile int *)&judged[ni % ITEMS] < DRAIN / 32;
+                    uint8_t *const bb = ringB + b * B_BYTES, *const mb = bb + PL * BN * CK * 2;
+                    mbar_expect_tx(&bfull[b], mags ? B_BYTES : PL * BN * CK * 2);
+                    tma_load_3d(bb, &mapB, &bfull[b], c * CK, n0, 0);
+                    if (mags) {
+                        tma_load_3d(mb, &magB, &bfull[b], c * CK, n0, 0);
+                        tma_load_3d(mb + BN * CK, &magA, &bfull[b], c * CK, m0, 0);
+                    }
+                    for (int p = 0; p < PL; ++p, ++it) {
                         const unsigned s = it % SLOTS;
                         if (!wait(&aempty[s], ((it / SLOTS) & 1u) ^ 1u)) break;
-                        mbar_expect_tx(&afull[s], p < PL ? A_BYTES : BM * CK);
-                        tma_load_3d(smem + s * A_BYTES, p < PL ? &mapA : &magA, &afull[s], c * CK, m0, p < PL ? p : 0);
+                        mbar_expect_tx(&afull[s], A_BYTES);
+                        tma_load_3d(smem + s * A_BYTES, &mapA, &afull[s], c * CK, m0, p);
                     }
                 }
             }
@@ -424,18 +439,14 @@ __global__ void __launch_bounds__(THREADS, 1)
                 const uint32_t dbuf = tm + b * BUF_COLS;
                 const int steps = min(4, k16 - 4 * c);
 #pragma unroll
-                for (int p = 0; p <= PL; ++p) {
+                for (int p = 0; p < PL; ++p) {
                     if (!mbar_wait_warp(&afull[s], ph, abort_flag, flags)) {
                         stop = true;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t a0 = sw128_lo(smem + s * A_BYTES);
-                    if (p == PL) {   // the magnitudes: 32 bytes per K = 32 step
-                        const uint32_t bm = b0 + (PL * BN * CK * 2 >> 4);
-                        umma_warp_f8(dbuf + (uint32_t)(PL * BN), a0, bm, idesc_mag(), 0u);
-                        if (steps > 2) umma_warp_f8(dbuf + (uint32_t)(PL * BN), a0 + 2, bm + 2, idesc_mag(), 1u);
-                    } else if (steps == 4) {
+                    if (steps == 4) {
                         umma_warp_x4(dbuf + (uint32_t)(p * BN), a0, b0, idesc((PL - p) * BN), p == 0 ? 0u : 1u);
                     } else {
                         for (int kk = 0; kk < steps; ++kk)   // 32 bytes per K = 16 step
@@ -449,6 +460,10 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                 }
                 if (stop) break;
+                // the magnitudes: 32 bytes per K = 32 step
+                const uint32_t bm = b0 + (PL * BN * CK * 2 >> 4), am = bm + (BN * CK >> 4);
+                umma_warp_f8(dbuf + (uint32_t)(PL * BN), am, bm, idesc_mag(), 0u);
+                if (steps > 2) umma_warp_f8(dbuf + (uint32_t)(PL * BN), am + 2, bm + 2, idesc_mag(), 1u);
                 umma_commit_warp(&bempty[b]);
                 umma_commit_warp(&cfull[b]);
             }
@@ -468,7 +483,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         // left waiting at a barrier.
         const int quarter = warp & 3, eighth = (warp - 2) >> 2, half = eighth >> 1, sub = (eighth & 1) * HB;
         const int dt = (threadIdx.x - 64) & 255;   // within the half: warps 2-9 are half 0, 10-17 half 1
-        unsigned gc = 0, ni = 0;
+        unsigned gc = 0, ni = 0, nd = 0;   // chunks, items opened and drained
         int set = 0;
         bool bad = false;
         Tables *const mine = tabs + 3 * half;
@@ -509,7 +524,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         if ((int)blockIdx.x < nitems) I = open(0);
         vote_any(half, false);
         const int row = quarter * 32 + lane;
-        for (int w = blockIdx.x; w < nitems; w += gridDim.x) {
+        for (int w = blockIdx.x; w < nitems; w += gridDim.x, ++nd) {
             const Tables &T = mine[set];
             const E64Out &g = GROUPED ? T.g : static_cast<const E64Out &>(g0);
             long long hi[HB], lo[HB];
@@ -566,6 +581,16 @@ __global__ void __launch_bounds__(THREADS, 1)
                         add_sum<9>(lo[j], r2[j]);
                         add_sum<0>(lo[j], r3[j]);
                     }
+                }
+                if (!GROUPED && c == 1 && I.z > MAG_CHUNKS) {
+                    // does an element still lack magnitude?  Rows and columns of zeros or past the edge need none (K
+                    // parts have no tables: all do)
+                    const bool tables = g0.ksplit == 1;
+                    bool lacks = false;
+#pragma unroll
+                    for (int j = 0; j < HB; ++j) lacks |= mag[j] < MAG_MIN && (!tables || T.colE[sub + j] != 0);
+                    lacks = lacks && (!tables || T.rowE[row] != 0);
+                    if (!__any_sync(0xffffffffu, lacks) && lane == 0) atomicAdd(&judged[nd % ITEMS], 1);
                 }
             }
             const int m0 = I.x, n0 = I.y + half * VN, at = I.w;
