@@ -37,7 +37,7 @@
 //
 // The tile is 128 x 32: TMEM holds two buffers of 8 x 32 FP32 columns (seven digit sums and the magnitudes), so
 // the drain of one chunk overlaps the MMAs of the next; a wider tile would need TMEM that is not there.  At long K
-// moving the operands paces: 140 KB a chunk from L2 (13.8 TB/s over all SMs), and shared memory, of which the chunk's
+// moving the operands paces: 140 KB a chunk from L2 (13.7 TB/s over all SMs), and shared memory, of which the chunk's
 // MMAs read 240 KB (with N = 32 per plane an instruction takes 4 KB of A and 1 to 7 KB of B for 16 to 112 clocks)
 // while TMA writes those 140, 2990 clocks at 128 bytes a clock against 1820 of MMA at the dense rate.  A's planes
 // arrive one by one (64 K values x 128 rows, 16 KB, 128-byte swizzle) in a ring of eight, B's together with the
